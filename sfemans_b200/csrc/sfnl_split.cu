@@ -36,12 +36,13 @@
 // rows of one point meet in shared memory, 16 quarter-angles at a time; each
 // output of the pointwise program is a sum of at most four signed products of
 // two fields (a constant term table per program), evaluated by one thread per
-// (output, point, half-chunk).  The folded products, sliced, are the A operand
+// (output, point, group of 2 or 4 angles).  The folded products, sliced, are the A operand
 // of the analysis, whose rows are (output, point) pairs; each 16-angle chunk is
 // analysed into a fresh accumulator and added in FP64 to the output, which the
 // same thread updates chunk after chunk (the lines stay in L2).
 //
-// One CTA of 8 warps, persistent over tiles; two threads per row.  Thread 0
+// CTAs of 16 warps, persistent over tiles; four threads per row, one per class (slicing, output) or
+// quarter of a chunk (recombination).  Thread 0
 // issues the MMAs; completion is signalled through an mbarrier whose waits
 // are bounded (a timeout sets a status word and abandons the tile instead of
 // spinning forever).
@@ -71,6 +72,15 @@ std::mutex g_status_mu;
 int *g_status_host = nullptr;  // pinned, mapped
 int *g_status_dev = nullptr;   // its device address
 
+// One tensor-core instruction of a tile: operand descriptors, accumulator column, instruction descriptor (its free
+// bit 31 set when it accumulates).  A CTA writes its list once (up to 48 of the synthesis, then 24 of a chunk's
+// analysis), so that the issuing thread spends two shared loads on each instead of rebuilding it.
+struct __align__(16) MmaOp {
+  uint64_t a, b;
+  uint32_t d, idesc, pad0, pad1;
+};
+constexpr int kSynMma = 48, kMaxMma = kSynMma + 24;
+
 // ---------------------------------------------------------------------------
 // geometry
 // ---------------------------------------------------------------------------
@@ -80,9 +90,15 @@ struct SGeo {
   int Ks_tot, No_tot;
   int tmem_cols, tmem_alloc;
   // shared-memory byte offsets (relative to the dynamic smem base)
-  int off_asyn[4][3], off_bsyn[4][3], off_bana[4][3], off_x, off_aana[4][3], off_bar, smem_bytes;
+  int off_asyn[4][3], off_bsyn[4][3], off_bana[4][3], off_x, off_aana[4][3], off_bar, off_list, smem_bytes;
   int ana_col[4];
 };
+
+// Exchange buffer X[field][quadrant * 16 + angle][point], in doubles.  The point rows are padded by two: the
+// product phase reads 4 (8) points at 4 (2) angle groups per half-warp, 2 (4) angles apart, which then fall into
+// different banks; the fields by 8, so that the two fields that a half-warp of 8-point rows writes do as well.
+__host__ __device__ constexpr int x_row_stride(int pts) { return pts + 2; }
+__host__ __device__ constexpr int x_field_stride(int pts) { return 64 * x_row_stride(pts) + 8; }
 
 int pow2_at_least(int v) {
   int p = 32;
@@ -90,7 +106,7 @@ int pow2_at_least(int v) {
   return p;
 }
 
-bool make_sgeo(int m, int pts, int nin, SGeo *out) {
+bool make_sgeo(int m, int pts, int nin, int nout, SGeo *out) {
   SGeo g;
   std::memset(&g, 0, sizeof(g));
   g.m = m;
@@ -119,22 +135,26 @@ bool make_sgeo(int m, int pts, int nin, SGeo *out) {
     g.ana_col[c] = 8 * g.Q + acc;
     acc += g.No[c];
   }
-  // Region 1: synthesis A operands, later overlaid by the exchange buffer and the analysis A operands.
+  // Region 1: synthesis A operands overlaid by the exchange buffer, then the analysis A operands: the next tile's
+  // synthesis operands are written while the last chunk of this one is analysed.
   int asyn = 0;
   for (int c = 0; c < 4; ++c)
     for (int i = 0; i < 3; ++i) {
       g.off_asyn[c][i] = asyn;
       asyn += 128 * g.Ks[c] * 2;
     }
-  const int xbytes = nin * 64 * pts * 8;
-  int r1b = xbytes;
+  const int xbytes = nin * x_field_stride(pts) * 8;
+  int r1b = asyn > xbytes ? asyn : xbytes;
+  // the analysis A operands keep the nout * pts live rows; the MMA's 128 rows run on into what follows them
+  // (other operands, the tables: 4 KB at most), and the accumulator rows beyond the live ones are never read
   for (int c = 0; c < 4; ++c)
     for (int i = 0; i < 3; ++i) {
       g.off_aana[c][i] = r1b;
-      r1b += 128 * 16 * 2;
+      r1b += nout * pts * 16 * 2;
     }
+  const int r1_read = g.off_aana[3][2] + 128 * 16 * 2;  // end of the last operand's 128 rows
   g.off_x = 0;
-  int r1 = asyn > r1b ? asyn : r1b;
+  int r1 = r1b;
   r1 = (r1 + 127) & ~127;
   int off = r1;
   for (int c = 0; c < 4; ++c)
@@ -150,7 +170,10 @@ bool make_sgeo(int m, int pts, int nin, SGeo *out) {
   off = (off + 15) & ~15;
   g.off_bar = off;
   off += 16;
+  g.off_list = off;
+  off += kMaxMma * (int)sizeof(MmaOp);
   g.smem_bytes = off;
+  if (g.smem_bytes < r1_read) g.smem_bytes = r1_read;
   if (g.smem_bytes > 227 * 1024) return false;
   *out = g;
   return true;
@@ -315,6 +338,14 @@ __device__ __forceinline__ void report_timeout(int *status) {
   }
 }
 
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
   uint32_t r[8];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -331,11 +362,9 @@ __device__ __forceinline__ double pow2(int e) {
   return __longlong_as_double((long long)(e + 1023) << 52);
 }
 
-__device__ __forceinline__ int row_exponent(double mx) {
-  int e = 0;
-  frexp(mx, &e);  // mx = f 2^e, f in [0.5, 1) -> mx < 2^e
-  return e;
-}
+// e with mx < 2^e, mx >= 2^(e-1), from the exponent bits (0, subnormals and infinity: below or above the range that
+// slice_scale keeps).
+__device__ __forceinline__ int row_exponent(double mx) { return (int)((__double2hiint(mx) >> 20) & 0x7ff) - 1022; }
 
 // 2^e as a float (e in the normal range).
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
@@ -360,10 +389,14 @@ __device__ __forceinline__ SliceScale slice_scale(int E) {
   return s;
 }
 __device__ __forceinline__ void slice3f(double x, const SliceScale &s, float &h, float &m, float &l) {
-  const double hd = rint(x * s.i0) * s.u0;
+  // round to nearest even by adding and subtracting 1.5 * 2^52 (2^23): the scaled values stay below 2^51 (2^22),
+  // and the conversion instructions behind rint() run at a fraction of the adders' rate
+  const double big = 6755399441055744.0;
+  const float bigf = 12582912.0f;
+  const double hd = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, s.i0), big), -big), s.u0);
   const float r = (float)(x - hd);
-  m = rintf(r * s.i1) * s.u1;
-  l = rintf((r - m) * s.i2) * s.u2;
+  m = __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(r, s.i1), bigf), -bigf), s.u1);
+  l = __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(r - m, s.i2), bigf), -bigf), s.u2);
   h = (float)hd;
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -435,35 +468,31 @@ struct SplitArgs {
   int *status;  // the mapped status word
 };
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;
+constexpr int kIssuer = kThreads - 32;  // issues the MMAs: its warp has the fewest live rows and no product in most programs
 
-// Compile-time geometry of make_sgeo for a given m (0: read it from the arguments).
-__host__ __device__ constexpr int sg_qmin(int m) { return (3 * m - 2 + 3) / 4; }
-__host__ __device__ constexpr int sg_Q(int m) { return ((sg_qmin(m) + 15) / 16) * 16 < 16 ? 16 : ((sg_qmin(m) + 15) / 16) * 16; }
-__host__ __device__ constexpr int sg_ke(int m, int c) { return (c & 1) ? m / 2 : (m + 1) / 2; }
-__host__ __device__ constexpr int sg_Ks(int m, int c) { return ((sg_ke(m, c) + 15) / 16) * 16 < 16 ? 16 : ((sg_ke(m, c) + 15) / 16) * 16; }
-__host__ __device__ constexpr int sg_anacol(int m, int c) { return c == 0 ? 8 * sg_Q(m) : sg_anacol(m, c - 1) + sg_Ks(m, c - 1); }
+// Lanes that share a point's 16 angles in the product phase: as many as keep an output's lanes within the CTA's
+// warps, so that a lane's chain of products, bounds and slices stays short.
+__host__ __device__ constexpr int pr_jg(int pr) { return pr_nout(pr) * pr_pts(pr) * 8 <= kThreads ? 8 : 4; }
 
-// Product phase for one output O of program PR (warp-uniform): lane = point p + PTS*jg, each lane owns
-// J consecutive quarter-angles of the 16-angle chunk.  Evaluates the output at the 4 quadrant angles,
-// folds the products into the analysis classes, finds each class row's bound over the chunk (shuffles
-// across the lanes of the same point), slices and writes the analysis A operand row O*PTS + p.
-// Product phase for one output o (warp-uniform): lane = point p + PTS*jg, each lane owns J consecutive
-// quarter-angles of the 16-angle chunk.  The output's (at most 4) terms s*x[a]*x[b] are read once from
-// constant memory into registers as shared-memory offsets.  Evaluates the output at the 4 quadrant
-// angles, folds the products into the analysis classes, finds each class row's bound over the chunk
-// (shuffles across the lanes of the same point), slices and writes the analysis A operand row o*PTS + p.
+// Product phase for one output o and one group of 32/JG points (warp-uniform): lane = point p, angle group jg of
+// J = 16/JG consecutive quarter-angles of the 16-angle chunk.  The output's (at most 4) terms s*x[a]*x[b] are read
+// once from constant memory into registers as shared-memory offsets.  Evaluates the output at the 4 quadrant
+// angles, folds the products into the analysis classes, finds each class row's bound over the chunk (shuffles
+// across the lanes of the same point), slices and writes the analysis A operand row o*PTS + p.
 template <int PR>
-__device__ __forceinline__ void product_rows(int o, const double *X, unsigned char *sm, const SGeo &g, int lane) {
-  constexpr int PTS = pr_pts(PR), JG = 32 / PTS, J = 16 / JG;
-  const int p = lane % PTS, jg = lane / PTS;
+__device__ __forceinline__ void product_rows(int o, int pgrp, const double *X, unsigned char *sm, const SGeo &g,
+                                             int lane) {
+  constexpr int PTS = pr_pts(PR), JG = pr_jg(PR), J = 16 / JG, PW = 32 / JG;  // PW: points of a warp
+  constexpr int RS = x_row_stride(PTS), FS = x_field_stride(PTS);
+  const int p = pgrp * PW + lane % PW, jg = lane / PW;
   const double *xa[4], *xb[4];
   double sg[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const STerm tm = c_terms[PR][o][u];
-    xa[u] = X + (size_t)tm.a * 64 * PTS + (size_t)jg * J * PTS + p;
-    xb[u] = X + (size_t)tm.b * 64 * PTS + (size_t)jg * J * PTS + p;
+    xa[u] = X + (size_t)tm.a * FS + jg * J * RS + p;
+    xb[u] = X + (size_t)tm.b * FS + jg * J * RS + p;
     sg[u] = (double)tm.s;  // 0 for an unused term
   }
   double P[4][J];
@@ -473,7 +502,7 @@ __device__ __forceinline__ void product_rows(int o, const double *X, unsigned ch
     double gq[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const int off = (r * 16 + jj) * PTS;
+      const int off = (r * 16 + jj) * RS;
       double acc = 0.0;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
@@ -491,7 +520,7 @@ __device__ __forceinline__ void product_rows(int o, const double *X, unsigned ch
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int sh = PTS; sh < 32; sh <<= 1) mx[c] = fmax(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], sh));
+    for (int sh = PW; sh < 32; sh <<= 1) mx[c] = fmax(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], sh));
   const int ro = o * PTS + p, k0 = jg * J;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
@@ -508,40 +537,40 @@ __device__ __forceinline__ void product_rows(int o, const double *X, unsigned ch
     }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-      unsigned char *rowp = sm + g.off_aana[c][i] + (size_t)(ro / 8) * 256 + (size_t)(ro % 8) * 16;
-#pragma unroll
-      for (int q0 = 0; q0 < J / 2; q0 += 4) {
-        const int k = k0 + 2 * q0;  // first of the (up to) 8 k-values of this store
-        unsigned char *dst = rowp + (size_t)(k / 8) * 128 + (size_t)(k % 8) * 2;
-        if constexpr (J / 2 >= 4)
-          *reinterpret_cast<uint4 *>(dst) = make_uint4(w[i][q0], w[i][q0 + 1], w[i][q0 + 2], w[i][q0 + 3]);
-        else
-          *reinterpret_cast<uint2 *>(dst) = make_uint2(w[i][0], w[i][1]);
-      }
+      unsigned char *dst = sm + g.off_aana[c][i] + (size_t)(ro / 8) * 256 + (size_t)(ro % 8) * 16 +
+                           (size_t)(k0 / 8) * 128 + (size_t)(k0 % 8) * 2;
+      if constexpr (J == 4)
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(w[i][0], w[i][1]);
+      else
+        *reinterpret_cast<uint32_t *>(dst) = w[i][0];
     }
   }
 }
 
-template <int PR, int M>
-__global__ void __launch_bounds__(kThreads, 1) split_kernel(const SplitArgs a) {
+// KEB: bound on the modes per class (8, 16, 32: m <= 16, 32, 64), which sizes the registers; the geometry is read
+// at run time.  Up to m = 16 two CTAs share an SM (256 of the 512 TMEM columns and 64 registers a thread each).
+// Each output coefficient is the FP64 sum of its chunks: kept in registers where they hold a class (KEB <= 16),
+// else added to the output in L2 by its one thread (red.add, the same sums in the same order).
+// Measured on a B200 against two threads per row in CTAs of 8 warps (12.5 % occupancy, issue slots 17 % busy; the
+// issuing thread rebuilt every descriptor), bit for bit the same outputs: the cross product of 28,000 points at
+// m = 16 152 -> 72 us, at m = 64 0.62 -> 0.28 ms, the MHD bundle of 100,000 points at m = 64 6.0 -> 2.7 ms.  What is
+// left is the chain of a tile's phases, 40 % of it the tensor cores reading the A operands.
+template <int PR, int KEB>
+__global__ void __launch_bounds__(kThreads, KEB == 8 ? 2 : 1) split_kernel(const SplitArgs a) {
   constexpr int NI = pr_nin(PR), NO = pr_nout(PR), PTS = pr_pts(PR);
   constexpr unsigned ADJ = pr_adj_in(PR);
-  constexpr bool CT = M > 0;
-  constexpr int KE_MAX = CT ? (M + 1) / 2 : kKeMax;
+  constexpr bool REG_OUT = KEB <= 16;
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ uint32_t s_tmem;
   const SGeo &g = a.g;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int row = t & 127, half = t >> 7;  // TMEM lane = row (warp w reads lanes 32*(w%4)..)
+  const int row = t & 127, quarter = t >> 7;  // TMEM lane = row (warp w reads lanes 32*(w%4)..)
   const uint32_t mbar = smem_u32(sm + g.off_bar);
-  const int Q = CT ? sg_Q(M) : g.Q, NC = Q / 16;
-  int KE[4], KS[4], ACOL[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    KE[c] = CT ? sg_ke(M, c) : g.ke[c];
-    KS[c] = CT ? sg_Ks(M, c) : g.Ks[c];
-    ACOL[c] = CT ? sg_anacol(M, c) : g.ana_col[c];
-  }
+  // up to m = 16 one chunk of 16 angles, up to m = 32 one k-step per class
+  const int Q = KEB == 8 ? 16 : g.Q, NC = KEB == 8 ? 1 : g.NC;
+  // this thread's class in the slicing and output phases: 0, 1 cosine even / odd, 2, 3 sine
+  const int kec = g.ke[quarter], ksc = KEB <= 16 ? 16 : g.Ks[quarter], par = quarter & 1;
+  const bool sine = quarter >= 2;
 
   // ---- setup: TMEM, mbarrier, DFT tables ----
   if (warp == 0) {
@@ -571,118 +600,168 @@ __global__ void __launch_bounds__(kThreads, 1) split_kernel(const SplitArgs a) {
   const int64_t ntiles = (a.np + PTS - 1) / PTS;
   const double invN = 1.0 / (4.0 * Q), twoN = 2.0 * invN;
   const int npairs = a.nsl == 3 ? 6 : 3;
-  double *X = reinterpret_cast<double *>(sm + g.off_x);  // [f][quadrant][16][PTS], point fastest
+  double *X = reinterpret_cast<double *>(sm + g.off_x);
+  MmaOp *mma = reinterpret_cast<MmaOp *>(sm + g.off_list);
+  // Instructions of one class and k-step of the synthesis: hi x [hi, mid], two table slices stacked along N into the
+  // neighbouring accumulators D0 and D1, then mid.hi, hi.lo, mid.mid and lo.hi into D1.  An instruction costs about 40
+  // cycles for its A operand and 0.7 per column of N, so fewer and wider ones are cheaper.
+  const int per = a.nsl == 3 ? 5 : 2;
+  int nsyn = 0;
+  for (int c = 0; c < 4; ++c) nsyn += g.Ks[c] / 16 * per;
+  if (t < nsyn + 4 * npairs) {
+    // Synthesis: k-step, instruction, class; analysis: slice pair (corrections before hi x hi, one accumulator),
+    // class.  A second k-step exists for the classes of more than 16 modes: all four, or (m = 33) the even ones.
+    const bool syn = t < nsyn;
+    int u = syn ? t : t - nsyn, s = 0, ncl = 4;
+    if (syn && u >= 4 * per) {
+      u -= 4 * per;
+      s = 1;
+      ncl = (g.Ks[0] + g.Ks[1] + g.Ks[2] + g.Ks[3]) / 16 - 4;
+    }
+    const int pr = u / ncl, c = (u - pr * ncl) * (4 / ncl);
+    MmaOp m;
+    int i, j;
+    if (syn) {
+      i = pr == 1 || pr == 3 ? 1 : pr == 4 ? 2 : 0;
+      j = pr == 2 ? 2 : pr == 3 ? 1 : 0;
+      m.a = make_sdesc(smem_u32(sm + g.off_asyn[c][i]) + 256 * s, 128, 16 * g.Ks[c]);
+      m.b = make_sdesc(smem_u32(sm + g.off_bsyn[c][j]) + 256 * s, 128, 16 * g.Ks[c]);
+      m.d = tmem + (uint32_t)((c * 2 + (pr > 0)) * Q);
+      m.idesc = make_idesc(pr == 0 ? 2 * Q : Q) | (s > 0 || pr > 0 ? 0x80000000u : 0u);
+    } else {
+      if (a.nsl == 3) {
+        i = pr == 1 || pr == 3 ? 1 : pr == 4 ? 2 : 0;
+        j = pr == 0 || pr == 3 ? 1 : pr == 2 ? 2 : 0;
+      } else {
+        i = pr == 1 ? 1 : 0;
+        j = pr == 0 ? 1 : 0;
+      }
+      m.a = make_sdesc(smem_u32(sm + g.off_aana[c][i]), 128, 256);
+      m.b = make_sdesc(smem_u32(sm + g.off_bana[c][j]), 128, 16 * Q);  // chunk ch starts 256 ch bytes further
+      m.d = tmem + (uint32_t)g.ana_col[c];
+      m.idesc = make_idesc(g.Ks[c]) | (pr > 0 ? 0x80000000u : 0u);
+    }
+    m.pad0 = m.pad1 = 0;
+    mma[syn ? t : kSynMma + t - nsyn] = m;
+  }
+  auto issue = [&](const MmaOp *l, int n, int chunk) {
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) {
+      const MmaOp m = l[i];
+      umma_bf16(m.d, m.a, m.b + (uint64_t)(16 * chunk), m.idesc & 0x7FFFFFFFu, m.idesc >> 31);
+    }
+    umma_commit(mbar);
+  };
+  // One warp waits (bounded) for the tensor cores, the others sleep on the barrier (16 polling warps took issue
+  // slots from the SM's other CTA); the CTA agrees on the outcome before any barrier or loop condition depends on it.
+  auto wait_all = [&]() -> bool { return __syncthreads_and(warp != 0 || mbar_wait(mbar, phase)); };
+  double yo[REG_OUT ? KEB : 1];  // the thread's outputs: row (o, p), modes of its class
 
-  // Reads the analysis of one chunk and adds it (weighted) to the outputs: row = (o, p), half = class pair.
+  // Reads the analysis of one chunk and adds it (weighted) to the outputs: row = (o, p), the thread's class.
   auto flush_chunk = [&](int64_t tile, int chk) {
     const int o = row / PTS, p = row % PTS;
     const int64_t gp = tile * PTS + p;
     const bool live = row < NO * PTS && gp < a.np;
+    if ((row & ~31) >= NO * PTS) return;  // warp-uniform: no live row
+    double *dst = live ? a.out[o] + gp * a.out_ps + (sine ? a.np * a.out_ps : 0) : nullptr;
+    const int64_t ldm = live ? a.out_ldm[o] : 0;
 #pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-      const int c = 2 * half + cc;  // classes 0,1 (cos) or 2,3 (sin)
-      const int kec = half ? KE[2 + cc] : KE[cc], ksc = half ? KS[2 + cc] : KS[cc];
-      const int acol = half ? ACOL[2 + cc] : ACOL[cc];
-      for (int k0 = 0; k0 < ksc; k0 += 8) {
-        float v[8];
-        tmem_ld8(tmem + lane_base + (uint32_t)(acol + k0), v);
-        tmem_wait_ld();
-        if (!live) continue;
-        double *dst = a.out[o] + gp * a.out_ps + (half ? a.np * a.out_ps : 0);
-        const int64_t ldm = a.out_ldm[o];
+    for (int k0 = 0; k0 < KEB; k0 += 8) {
+      if (k0 >= ksc) break;
+      float v[8];
+      tmem_ld8(tmem + lane_base + (uint32_t)(g.ana_col[quarter] + k0), v);
+      tmem_wait_ld();
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int kk = k0 + e;
-          if (kk >= kec) break;
-          const int n = 2 * kk + cc;
-          const double sc = pr_adj_out(PR) ? 1.0 : (n == 0 ? invN : twoN);
-          const double val = (half && n == 0) ? 0.0 : (double)v[e] * sc;
+      for (int e = 0; e < 8; ++e) {
+        const int kk = k0 + e;
+        const int n = 2 * kk + par;
+        const double sc = pr_adj_out(PR) ? 1.0 : (n == 0 ? invN : twoN);
+        const double val = (sine && n == 0) ? 0.0 : (double)v[e] * sc;
+        if constexpr (REG_OUT) {
+          yo[kk] = (chk == 0 ? 0.0 : yo[kk]) + val;
+          if (live && chk == NC - 1 && kk < kec) dst[(int64_t)n * ldm] = yo[kk];
+        } else if (live && kk < kec) {
           double *q = dst + (int64_t)n * ldm;
-          *q = (chk == 0 ? 0.0 : *q) + val;
+          if (chk == 0)
+            *q = 0.0 + val;
+          else
+            atomicAdd(q, val);
         }
       }
-      (void)c;
     }
   };
 
-  for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    // ---- 1. load + slice the input rows: row = field slot f, point p; half = class pair ----
-    {
-      const int f = row / PTS, p = row % PTS;
-      const int64_t gp = tile * PTS + p;
-      const bool valid = f < NI && gp < a.np;
-      const double *src = valid ? a.in[f] + gp : nullptr;
-      const int64_t ldm = valid ? a.in_ldm[f] : 0;
-      const bool cot = f < NI && ((ADJ >> f) & 1u);
+  // Slices the tile's input rows into the synthesis A operands: row = field slot f, point p; the thread's class.
+  auto load_tile = [&](int64_t tile) {
+    const int f = row / PTS, p = row % PTS;
+    const int64_t gp = tile * PTS + p;
+    const bool valid = f < NI && gp < a.np;
+    // a warp without a live row leaves its rows as they are: their accumulator lanes are never read
+    if ((row & ~31) < NI * PTS) {
+    const double *src = valid ? a.in[f] + gp + (sine ? a.np : 0) : nullptr;
+    const int64_t ldm = valid ? a.in_ldm[f] : 0;
+    const bool cot = f < NI && ((ADJ >> f) & 1u);
+    double x[KEB];
+    double mx = 0.0;
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = 2 * half + cc;
-        const int kec = half ? KE[2 + cc] : KE[cc], ksc = half ? KS[2 + cc] : KS[cc];
-        double x[KE_MAX];
-        double mx = 0.0;
-#pragma unroll
-        for (int k = 0; k < KE_MAX; ++k) {
-          const int n = 2 * k + cc;
-          double v = 0.0;
-          if (valid && k < kec && !(half && n == 0)) {
-            v = __ldg(src + (int64_t)n * ldm + (half ? a.np : 0));
-            if (cot) v *= (n == 0 ? invN : twoN);
-          }
-          x[k] = v;
-          mx = fmax(mx, fabs(v));
-        }
-        const SliceScale sc = slice_scale(row_exponent(mx));
-#pragma unroll
-        for (int kg = 0; kg < (KE_MAX + 7) / 8 + 1; ++kg) {
-          if (kg * 8 >= ksc) break;
-          uint32_t w[3][4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            float hv[2], mv[2], lv[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int k = kg * 8 + 2 * q + e;
-              slice3f(k < KE_MAX ? x[k < KE_MAX ? k : 0] : 0.0, sc, hv[e], mv[e], lv[e]);
-            }
-            w[0][q] = pack_bf16(hv[0], hv[1]);
-            w[1][q] = pack_bf16(mv[0], mv[1]);
-            w[2][q] = pack_bf16(lv[0], lv[1]);
-          }
-          const size_t off = (size_t)(row / 8) * (16 * ksc) + (size_t)kg * 128 + (size_t)(row % 8) * 16;
-#pragma unroll
-          for (int i = 0; i < 3; ++i)
-            *reinterpret_cast<uint4 *>(sm + g.off_asyn[c][i] + off) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
-        }
-      }
+    for (int k = 0; k < KEB; ++k) {
+      const int n = 2 * k + par;
+      double v = 0.0;
+      if (valid && k < kec && !(sine && n == 0)) v = __ldg(src + (int64_t)n * ldm);
+      x[k] = v;
     }
+    if (valid && gp + (int64_t)gridDim.x * PTS < a.np && (p & 3) == 0) {
+      // the next tile's rows into L2 while this one is computed (one lane per 32-byte sector)
+      const double *nx = src + (int64_t)gridDim.x * PTS;
+#pragma unroll
+      for (int k = 0; k < KEB; ++k)
+        if (k < kec) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + (int64_t)(2 * k + par) * ldm));
+    }
+#pragma unroll
+    for (int k = 0; k < KEB; ++k) {
+      if (cot) x[k] *= (2 * k + par == 0 ? invN : twoN);
+      mx = fmax(mx, fabs(x[k]));
+    }
+    const SliceScale sc = slice_scale(row_exponent(mx));
+#pragma unroll
+    for (int kg = 0; kg < (KEB < 16 ? 2 : KEB / 8); ++kg) {
+      if (kg * 8 >= ksc) break;
+      uint32_t w[3][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float hv[2], mv[2], lv[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int k = kg * 8 + 2 * q + e;
+          slice3f(k < KEB ? x[k < KEB ? k : 0] : 0.0, sc, hv[e], mv[e], lv[e]);
+        }
+        w[0][q] = pack_bf16(hv[0], hv[1]);
+        w[1][q] = pack_bf16(mv[0], mv[1]);
+        w[2][q] = pack_bf16(lv[0], lv[1]);
+      }
+      const size_t off = (size_t)(row / 8) * (16 * ksc) + (size_t)kg * 128 + (size_t)(row % 8) * 16;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        *reinterpret_cast<uint4 *>(sm + g.off_asyn[quarter][i] + off) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+    }
+    }
+  };
+
+  load_tile(blockIdx.x);
+  for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    // ---- 1. the tile's operands are in place ----
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
 
     // ---- 2. synthesis MMAs: D0 (hi x hi) and D1 (corrections) per class ----
-    if (t == 0) {
+    if (t == kIssuer) {
       tc_fence_after();
-      const uint32_t idesc = make_idesc(Q);
-      for (int c = 0; c < 4; ++c) {
-        const uint32_t sbo = 16 * KS[c];
-        for (int s = 0; s < KS[c] / 16; ++s)
-          for (int pr = 0; pr < npairs; ++pr) {
-            const int i = pr == 0 ? 0 : pr == 1 ? 0 : pr == 2 ? 1 : pr == 3 ? 0 : pr == 4 ? 1 : 2;
-            const int j = pr == 0 ? 0 : pr == 1 ? 1 : pr == 2 ? 0 : pr == 3 ? 2 : pr == 4 ? 1 : 0;
-            const int accn = (i + j == 0) ? 0 : 1;
-            const uint32_t dcol = tmem + (uint32_t)((c * 2 + accn) * Q);
-            const uint64_t ad = make_sdesc(smem_u32(sm + g.off_asyn[c][i]) + 256 * s, 128, sbo);
-            const uint64_t bd = make_sdesc(smem_u32(sm + g.off_bsyn[c][j]) + 256 * s, 128, sbo);
-            const uint32_t en = (s > 0 || (accn == 1 && pr > 1)) ? 1u : 0u;
-            umma_bf16(dcol, ad, bd, idesc, en);
-          }
-      }
-      umma_commit(mbar);
+      issue(mma, nsyn, 0);
     }
     __syncwarp();
-    // Every thread waits (bounded) and the CTA agrees on the outcome before any barrier or loop
-    // condition depends on it; on a timeout the phase stays, so the final drain waits for it again.
-    if (!__syncthreads_and(mbar_wait(mbar, phase))) {
+    // On a timeout the phase stays, so the final drain waits for it again.
+    if (!wait_all()) {
       ok = false;
       if (t == 0) report_timeout(a.status);
     } else {
@@ -691,37 +770,40 @@ __global__ void __launch_bounds__(kThreads, 1) split_kernel(const SplitArgs a) {
     tc_fence_after();
 
     for (int ch = 0; ch < NC && ok; ++ch) {
-      // ---- 3a. read out, recombine in FP64, fold to the 4 quadrant angles (half = 8 quarter-angles) ----
+      // ---- 3a. read out, recombine in FP64, fold to the 4 quadrant angles (quarter = 4 quarter-angles) ----
       {
         const int f = row / PTS, p = row % PTS;
-        float d[4][2][8];
+        if ((row & ~31) < NI * PTS) {  // warp-uniform: a live row
+          double y[4][4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 4; ++c) {
+            float d[2][4];
 #pragma unroll
-          for (int ac = 0; ac < 2; ++ac)
-            tmem_ld8(tmem + lane_base + (uint32_t)((c * 2 + ac) * Q + ch * 16 + half * 8), d[c][ac]);
-        tmem_wait_ld();
-        if (f < NI) {
-          double *xr = X + (size_t)f * 64 * PTS + (size_t)half * 8 * PTS + p;
+            for (int ac = 0; ac < 2; ++ac)
+              tmem_ld4(tmem + lane_base + (uint32_t)((c * 2 + ac) * Q + ch * 16 + quarter * 4), d[ac]);
+            tmem_wait_ld();
 #pragma unroll
-          for (int jj = 0; jj < 8; ++jj) {
-            const double CE = (double)d[0][0][jj] + (double)d[0][1][jj];
-            const double CO = (double)d[1][0][jj] + (double)d[1][1][jj];
-            const double SE = (double)d[2][0][jj] + (double)d[2][1][jj];
-            const double SO = (double)d[3][0][jj] + (double)d[3][1][jj];
-            const double A = CE + CO, B = CE - CO, C = SE + SO, D = SO - SE;
-            xr[(0 * 16 + jj) * PTS] = A + C;  // theta
-            xr[(1 * 16 + jj) * PTS] = B + D;  // pi - theta
-            xr[(2 * 16 + jj) * PTS] = B - D;  // pi + theta
-            xr[(3 * 16 + jj) * PTS] = A - C;  // 2 pi - theta
+            for (int jj = 0; jj < 4; ++jj) y[c][jj] = (double)d[0][jj] + (double)d[1][jj];
+          }
+          if (f < NI) {
+            double *xr = X + (size_t)f * x_field_stride(PTS) + (size_t)quarter * 4 * x_row_stride(PTS) + p;
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj) {
+              const double CE = y[0][jj], CO = y[1][jj], SE = y[2][jj], SO = y[3][jj];
+              const double A = CE + CO, B = CE - CO, C = SE + SO, D = SO - SE;
+              xr[(0 * 16 + jj) * x_row_stride(PTS)] = A + C;  // theta
+              xr[(1 * 16 + jj) * x_row_stride(PTS)] = B + D;  // pi - theta
+              xr[(2 * 16 + jj) * x_row_stride(PTS)] = B - D;  // pi + theta
+              xr[(3 * 16 + jj) * x_row_stride(PTS)] = A - C;  // 2 pi - theta
+            }
           }
         }
       }
       tc_fence_before();
-      __syncthreads();
-      // The previous chunk's analysis must be complete before its A operand is rewritten.
+      // The exchange buffer is complete, and the previous chunk's analysis must be before its A operand is
+      // rewritten.
       if (ch > 0) {
-        if (!__syncthreads_and(mbar_wait(mbar, phase))) {
+        if (!wait_all()) {
           ok = false;
           if (t == 0) report_timeout(a.status);
           break;
@@ -729,39 +811,29 @@ __global__ void __launch_bounds__(kThreads, 1) split_kernel(const SplitArgs a) {
         phase ^= 1;
         tc_fence_after();
         flush_chunk(tile, ch - 1);
+      } else {
+        __syncthreads();
       }
-      // ---- 3b. program, analysis pre-fold, slicing: one output per warp ----
-      for (int o = warp; o < NO; o += kThreads / 32) product_rows<PR>(o, X, sm, g, lane);
+      // ---- 3b. program, analysis pre-fold, slicing ----
+      {
+        constexpr int GRP = PTS * pr_jg(PR) / 32;  // warps of one output
+        for (int w = warp; w < NO * GRP; w += kThreads / 32) product_rows<PR>(w / GRP, w % GRP, X, sm, g, lane);
+      }
       fence_async_smem();
       tc_fence_before();
       __syncthreads();
       // ---- 3c. analysis MMAs for this chunk, fresh accumulator (corrections first, then hi x hi) ----
-      if (t == 0 && ok) {
+      if (t == kIssuer && ok) {
         tc_fence_after();
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t idesc = make_idesc(KS[c]);
-          const uint32_t dcol = tmem + (uint32_t)ACOL[c];
-          for (int pr = 0; pr < npairs; ++pr) {
-            int i, j;
-            if (a.nsl == 3) {
-              i = pr == 0 ? 0 : pr == 1 ? 1 : pr == 2 ? 0 : pr == 3 ? 1 : pr == 4 ? 2 : 0;
-              j = pr == 0 ? 1 : pr == 1 ? 0 : pr == 2 ? 2 : pr == 3 ? 1 : pr == 4 ? 0 : 0;
-            } else {
-              i = pr == 1 ? 1 : 0;
-              j = pr == 0 ? 1 : 0;
-            }
-            const uint64_t ad = make_sdesc(smem_u32(sm + g.off_aana[c][i]), 128, 256);
-            const uint64_t bd = make_sdesc(smem_u32(sm + g.off_bana[c][j]) + 256 * ch, 128, 16 * Q);
-            umma_bf16(dcol, ad, bd, idesc, pr > 0 ? 1u : 0u);
-          }
-        }
-        umma_commit(mbar);
+        issue(mma + kSynMma, 4 * npairs, ch);
       }
       __syncwarp();
+      // the exchange buffer is free after the last chunk's products: the next tile's operands meanwhile
+      if (ch == NC - 1 && tile + gridDim.x < ntiles) load_tile(tile + gridDim.x);
     }
     // ---- 4. the last chunk into the outputs ----
     if (ok) {
-      if (!__syncthreads_and(mbar_wait(mbar, phase))) {
+      if (!wait_all()) {
         ok = false;
         if (t == 0) report_timeout(a.status);
       } else {
@@ -770,9 +842,8 @@ __global__ void __launch_bounds__(kThreads, 1) split_kernel(const SplitArgs a) {
     }
     tc_fence_after();
     if (ok) flush_chunk(tile, NC - 1);
-    tc_fence_before();
-    __syncthreads();
   }
+  tc_fence_before();
   __syncthreads();
   // After a timeout the last commit's phase is still pending: wait for it once more (bounded) so that
   // no tensor-core operation still writes the columns being freed; the status word already reports
@@ -788,18 +859,19 @@ __global__ void __launch_bounds__(kThreads, 1) split_kernel(const SplitArgs a) {
   }
 }
 
-template <int PR, int M>
+template <int PR, int KEB>
 int launch_split_pr(SplitArgs &sa, int batch, const ProgArgs &pa, const int *in_map, const int *out_map,
                     cudaStream_t st) {
   constexpr int NI = pr_nin(PR), NO = pr_nout(PR), PTS = pr_pts(PR);
-  auto kern = split_kernel<PR, M>;
+  auto kern = split_kernel<PR, KEB>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sa.g.smem_bytes) != cudaSuccess)
     return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (split form)");
   const int64_t ntiles = (sa.np + PTS - 1) / PTS;
-  int per_sm_tmem = 512 / sa.g.tmem_alloc;
-  int per_sm_smem = (int)((228 * 1024) / (sa.g.smem_bytes + 1024));
-  int per_sm = per_sm_tmem < per_sm_smem ? per_sm_tmem : per_sm_smem;
-  if (per_sm < 1) per_sm = 1;
+  // resident CTAs: by TMEM columns, shared memory and the kernel's launch bounds (the occupancy query answers 1 for
+  // kernels that allocate TMEM)
+  int per_sm = (int)((227 * 1024) / (sa.g.smem_bytes + 1024 + 128));
+  per_sm = per_sm < 512 / sa.g.tmem_alloc ? per_sm : 512 / sa.g.tmem_alloc;
+  per_sm = per_sm < 1 ? 1 : per_sm > (KEB == 8 ? 2 : 1) ? (KEB == 8 ? 2 : 1) : per_sm;
   int64_t grid = (int64_t)num_sms() * per_sm;
   if (grid > ntiles) grid = ntiles;
   if (grid < 1) grid = 1;
@@ -864,7 +936,7 @@ int run_split_program(const ProgArgs &pa, int split, const int *in_map, const in
   SplitArgs sa;
   std::memset(&sa, 0, sizeof(sa));
   if (int rc = status_word(&sa.status)) return rc;
-  if (!make_sgeo(pa.m, pr_pts(PR), pr_nin(PR), &sa.g)) return set_error(SFNL_ERR_UNSUPPORTED, "split form: m too large");
+  if (!make_sgeo(pa.m, pr_pts(PR), pr_nin(PR), pr_nout(PR), &sa.g)) return set_error(SFNL_ERR_UNSUPPORTED, "split form: m too large");
   STables T;
   int rc = get_stables(sa.g, &T);
   if (rc) return rc;
@@ -877,12 +949,10 @@ int run_split_program(const ProgArgs &pa, int split, const int *in_map, const in
   sa.bana_bytes = (int)T.bana_bytes;
   if (sa.g.off_bsyn[0][0] + sa.bsyn_bytes != sa.g.off_bana[0][0] || sa.g.off_bana[0][0] + sa.bana_bytes > sa.g.off_bar)
     return set_error(SFNL_ERR_UNSUPPORTED, "split form: table layout mismatch");
-  switch (pa.m) {
-    case 16: return launch_split_pr<PR, 16>(sa, pa.batch, pa, in_map, out_map, st);
-    case 32: return launch_split_pr<PR, 32>(sa, pa.batch, pa, in_map, out_map, st);
-    case 64: return launch_split_pr<PR, 64>(sa, pa.batch, pa, in_map, out_map, st);
-    default: return launch_split_pr<PR, 0>(sa, pa.batch, pa, in_map, out_map, st);
-  }
+  // by the modes of the largest class, (m + 1) / 2
+  if (pa.m <= 16) return launch_split_pr<PR, 8>(sa, pa.batch, pa, in_map, out_map, st);
+  if (pa.m <= 32) return launch_split_pr<PR, 16>(sa, pa.batch, pa, in_map, out_map, st);
+  return launch_split_pr<PR, 32>(sa, pa.batch, pa, in_map, out_map, st);
 }
 
 }  // namespace
@@ -890,7 +960,7 @@ int run_split_program(const ProgArgs &pa, int split, const int *in_map, const in
 bool split_supported(int op, int m) {
   if (m < 1 || m > 64 || !op_bilinear(op) || op == OP_ADVECT) return false;
   SGeo g;
-  return make_sgeo(m, 8, 16, &g) && make_sgeo(m, 16, 8, &g) && make_sgeo(m, 32, 4, &g);
+  return make_sgeo(m, 8, 16, 10, &g) && make_sgeo(m, 16, 8, 3, &g) && make_sgeo(m, 32, 4, 3, &g);
 }
 
 int launch_split(const ProgArgs &a, int split, cudaStream_t st) {
