@@ -281,9 +281,9 @@ __host__ __device__ constexpr int ek_nout(int ek) {
 // With NT <= 8 angle tiles every warp (pair, with the class split) owns one tile and the products
 // (and the exchange) overlay the coefficients.
 // The class split (two warps per angle tile, one per class pair) halves the accumulators of a warp
-// and doubles the warps per SM; it pays for the six-field programs at m >= 64, where the accumulator
+// and doubles the warps per SM; it pays for the six-field programs from m = 33, where the accumulator
 // registers limit residency, and costs shared memory and a barrier elsewhere (measured on B200).
-constexpr bool class_split(int ek, int M) { return (ek == EK_CROSS || ek == EK_DOT) && (M == 64 || M == 0); }
+constexpr bool class_split(int ek, int KSC) { return (ek == EK_CROSS || ek == EK_DOT) && (KSC >= 5 || KSC == 0); }
 // With several passes the products (written after a barrier that ends pass 0's synthesis, added to in the
 // later passes) may overlay only pass 0's coefficients.
 __host__ __device__ constexpr bool fast_overlay(int ek, int NT, int KT) {
@@ -298,31 +298,25 @@ inline size_t fast_smem_bytes(int ek, int NT, int KT, bool cs) {
 }
 
 
-// Geometry of make_geo as constant expressions (the kernels specialise on m).
-__host__ __device__ constexpr int cg_qmin(int m) { return (3 * m - 2 + 3) / 4 < 1 ? 1 : (3 * m - 2 + 3) / 4; }
-__host__ __device__ constexpr int cg_NT(int m) { return (cg_qmin(m) + 7) / 8; }
-__host__ __device__ constexpr int cg_ke(int m, int c) { return (c & 1) ? m / 2 : (m + 1) / 2; }
-__host__ __device__ constexpr int cg_KS(int m, int c) { return (cg_ke(m, c) + 3) / 4; }
-__host__ __device__ constexpr int cg_NU(int m, int c) { return (cg_ke(m, c) + 7) / 8; }
-__host__ __device__ constexpr int cg_ksoff(int m, int c) { return c == 0 ? 0 : cg_ksoff(m, c - 1) + cg_KS(m, c - 1); }
-__host__ __device__ constexpr int cg_nuoff(int m, int c) { return c == 0 ? 0 : cg_nuoff(m, c - 1) + cg_NU(m, c - 1); }
-
-
-// EK: elementary program; M: modes when specialised (0: any m, geometry at run time);
+// EK: elementary program; KSC, NTC: k-steps per class and quarter-angle tiles (make_geo, every m <= 64), which fix
+// all loops at compile time; 0, 0: any m, geometry at run time;
 // ADJ: 0 plain, 1 first operand (fields 0-2) a cotangent, 2 second operand (fields 3-5) a cotangent.
-// Launch bounds (measured on B200): the class-split cross product at m = 64 runs best at 3 CTAs of 12
-// warps per SM (56 registers); the tensor program wants registers (no residency target); the others
-// keep the compiler's default register target.
-constexpr int fast_max_threads(int M, bool cs) { return cs ? (M == 64 ? 384 : 512) : 256; }
-constexpr int fast_min_blocks(int ek, int M, bool cs) { return (cs && M == 64 && ek == EK_CROSS) ? 3 : ek == EK_TENSOR ? 1 : 0; }
+// Launch bounds (measured on B200): the class-split cross product runs best with as many CTAs of 2 NT warps per SM as
+// 1152 threads hold (3 of 12 at m = 64: 56 registers); the tensor program wants registers (no residency target); the
+// others keep the compiler's default register target.
+constexpr int fast_max_threads(int NTC, bool cs) { return cs ? (NTC > 0 ? 64 * NTC : 512) : 256; }
+constexpr int fast_min_blocks(int ek, int NTC, bool cs) {
+  return cs && NTC > 0 && ek == EK_CROSS ? 1152 / (64 * NTC) : ek == EK_TENSOR ? 1 : 0;
+}
 
 // GK >= 0 (a Gauss-point caller, GK_*): the operands are built in the staging from the node-major nodal
 // fields of a.ga instead of read from a.in (one batch entry).
-template <int EK, int M, int ADJ, bool CS, int GK = -1>
-__global__ void __launch_bounds__(fast_max_threads(M, CS),
-                                  GK >= 0 && fast_min_blocks(EK, M, CS) > 2 ? 2 : fast_min_blocks(EK, M, CS))
+template <int EK, int KSC, int NTC, int ADJ, bool CS, int GK = -1>
+__global__ void __launch_bounds__(fast_max_threads(NTC, CS),
+                                  GK >= 0 && fast_min_blocks(EK, NTC, CS) > 2 ? 2 : fast_min_blocks(EK, NTC, CS))
     fast_kernel(const FastArgs a) {
-  constexpr bool CT = M > 0;
+  constexpr bool CT = KSC > 0;
+  constexpr int NUC = (KSC + 1) / 2;
   constexpr int NI = EKDef<EK>::NI, NO = EKDef<EK>::NO;
   // Shared memory: folded products ps [NO][4][NT][2][32], with the class split (CS) the exchange
   // between the two warps of an angle tile xc [NW/2][2][NI][2][32], and the staged coefficients
@@ -334,15 +328,15 @@ __global__ void __launch_bounds__(fast_max_threads(M, CS),
   const int64_t p0 = (int64_t)blockIdx.x * 8, p = p0 + g;
   const bool valid = p < a.np;
   const int b = blockIdx.y;
-  const int NT = CT ? cg_NT(M) : a.NT;
+  const int NT = CT ? NTC : a.NT;
   int KS[4], KOFF[4], KE[4], NU[4], NOFF[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    KS[c] = CT ? cg_KS(M, c) : a.KS[c];
-    KOFF[c] = CT ? cg_ksoff(M, c) : a.ks_off[c];
-    KE[c] = CT ? cg_ke(M, c) : a.ke[c];
-    NU[c] = CT ? cg_NU(M, c) : a.NU[c];
-    NOFF[c] = CT ? cg_nuoff(M, c) : a.nu_off[c];
+    KS[c] = CT ? KSC : a.KS[c];
+    KOFF[c] = CT ? c * KSC : a.ks_off[c];
+    KE[c] = a.ke[c];
+    NU[c] = CT ? NUC : a.NU[c];
+    NOFF[c] = CT ? c * NUC : a.nu_off[c];
   }
   const int KS_tot = KS[0] + KS[1] + KS[2] + KS[3], KT = 4 * KS_tot;
   const int NU_tot = NU[0] + NU[1] + NU[2] + NU[3];
@@ -369,7 +363,7 @@ __global__ void __launch_bounds__(fast_max_threads(M, CS),
     // row is 4*KOFF[i & 1] + (i >> 1), its sine row 4*KOFF[2 + (i & 1)] + (i >> 1); other rows stay 0
     for (int t = threadIdx.x; t < NI * KS_tot * 32; t += blockDim.x) xs[t] = 0.0;
     __syncthreads();
-    const int m = CT ? M : a.m;
+    const int m = a.m;
     for (int it = threadIdx.x; it < 8 * m; it += blockDim.x) {
       const int i = it % m, gp = it / m;  // a warp takes consecutive modes of one point
       if (p0 + gp >= a.np) continue;
@@ -388,7 +382,7 @@ __global__ void __launch_bounds__(fast_max_threads(M, CS),
     const int pc = 2 * (threadIdx.x & 3), rstep = blockDim.x >> 2;
     const bool v16 = a.vec16 && p0 + 8 <= a.np;
     const bool pv0 = p0 + pc < a.np, pv1 = p0 + pc + 1 < a.np;
-    if constexpr (M != 0) {
+    if constexpr (CT) {
       // rows outermost: the row's class, mode and sine offset are decoded once for the NI fields
       for (int r = threadIdx.x >> 2; r < KT; r += rstep) {
         const int c = (r >= 4 * KOFF[1]) + (r >= 4 * KOFF[2]) + (r >= 4 * KOFF[3]);
@@ -662,6 +656,176 @@ __global__ void __launch_bounds__(fast_max_threads(M, CS),
 }
 
 // ---------------------------------------------------------------------------
+// one warp per 8-point tile (small m)
+// ---------------------------------------------------------------------------
+// Up to m = 16 (one output tile of 8 modes per class) a warp can keep a whole tile to itself: the analysis
+// accumulators of every class (NO * 4 * NUC pairs) fit in its registers beside the synthesis accumulators, so the
+// folded products of an angle tile go from the registers of the lane that formed them straight into the analysis
+// as A fragments and no warp waits for another.
+// The two-warp CTAs of fast_kernel ran copy, synthesis, products and analysis one after the other with barriers
+// between (DMMA pipe 31 % busy at m = 16).  Programs with one output fit up to m = 32.  Every class takes KSC k-steps
+// and NUC output tiles, also where the odd one needs fewer (zero coefficients; results not stored), so that no
+// branch keeps the loads of the table fragments from running ahead (with the branches the cross product at m = 16 took
+// 33 us).  One buffer and three CTAs of four warps per SM beat two buffers and two CTAs (22.2 against 23.7 us per call
+// with the host's share): the next tile's copies start when the last angle tile's coefficients are read.  Measured on
+// a B200 against fast_kernel: cross product, 28,000 points, m = 16 26.6 -> 24.6 us; 50,001 points, m = 10 50 -> 30 us;
+// product of scalars, 100,000 points, m = 8 32 -> 19 us; dot product, 50,001 points, m = 24 114 -> 69 us.  Three
+// outputs at m = 17..32 need 255 registers (two CTAs) and were slower than fast_kernel (m = 32: 192 against 160 us).
+constexpr int kSoloWarps = 4;
+// Largest k-steps per class (KSC; the analysis has NUC = (KSC + 1) / 2 output tiles of 8 per class).
+constexpr int solo_max_ks(int ek) { return ek_nout(ek) == 1 ? 4 : 2; }
+constexpr bool solo_ek(int ek) { return ek == EK_CROSS || ek == EK_DOT || ek == EK_PROD || ek == EK_SVECT; }
+constexpr size_t solo_smem_bytes(int ek, int KSC) { return sizeof(double) * (size_t)kSoloWarps * ek_nin(ek) * 4 * KSC * 32; }
+
+template <int EK, int KSC, int ADJ>
+__global__ void __launch_bounds__(32 * kSoloWarps, EKDef<EK>::NI <= 2 ? 4 : 3) solo_kernel(const FastArgs a) {
+  constexpr int NI = EKDef<EK>::NI, NO = EKDef<EK>::NO;
+  constexpr int NUC = (KSC + 1) / 2, KS_tot = 4 * KSC, bufd = NI * KS_tot * 32;
+  constexpr int RG = 2 * KSC;  // groups of 8 staged rows (4 KSC rows per class)
+  extern __shared__ __align__(16) double smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, q = lane & 3, b = blockIdx.y;
+  const int NT = a.NT;
+  const double invN = 1.0 / (4.0 * 8.0 * NT), twoN = 2.0 * invN;
+  double *buf = smem + (size_t)warp * bufd;
+
+  // Staging: lane l copies points 2 (l & 3), 2 (l & 3) + 1 of row 8 rg + (l >> 2) of every field (rows as in
+  // fast_kernel: class, then mode, padded to k-steps).  Rows without a mode stay zero.
+  const int pc = 2 * (lane & 3);
+  int64_t soff[RG];  // of the row in a field, minus the mode's offset: np for a sine row; -1: no mode
+  int mode[RG];
+#pragma unroll
+  for (int rg = 0; rg < RG; ++rg) {
+    const int r = 8 * rg + (lane >> 2);
+    const int c = r / (4 * KSC), k = r - 4 * KSC * c;
+    mode[rg] = class_mode(c, k);
+    soff[rg] = k < sel4(a.ke, c) && !(c == 2 && k == 0) ? (c >= 2 ? a.np : 0) : -1;
+  }
+  for (int i = lane; i < bufd; i += 32) buf[i] = 0.0;
+  __syncwarp();
+  auto stage = [&](double *dst0, int64_t tile) {
+    const int64_t p = tile * 8 + pc;
+    const bool v16 = a.vec16 && p + 1 < a.np;
+#pragma unroll
+    for (int rg = 0; rg < RG; ++rg) {
+      if (soff[rg] < 0) continue;
+      const int r = 8 * rg + (lane >> 2);
+      double *dst = dst0 + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
+#pragma unroll
+      for (int f = 0; f < NI; ++f, dst += KS_tot * 32) {
+        const double *src = a.in[f] + (int64_t)b * a.in_bs[f] + p + soff[rg] + (int64_t)mode[rg] * a.in_ldm[f];
+        if (v16) {
+          cp_async16(dst, src);
+        } else {
+          if (p < a.np) cp_async8(dst, src); else dst[0] = 0.0;
+          if (p + 1 < a.np) cp_async8(dst + 1, src + 1); else dst[1] = 0.0;
+        }
+      }
+    }
+    cp_async_commit();
+  };
+
+  const int64_t tiles = (a.np + 7) / 8, step = (int64_t)gridDim.x * kSoloWarps;
+  int64_t tile = (int64_t)blockIdx.x * kSoloWarps + warp;
+  if (tile < tiles) stage(buf, tile);
+  const double *ana0 = a.ana + (size_t)(a.adj_out ? 1 : 0) * a.NU_tot * NT * 64 + lane;
+  for (; tile < tiles; tile += step) {
+    cp_async_wait_0();
+    __syncwarp();
+    const double *xs = buf + a_frag_slot(q, g);
+    double y[4][NUC][NO][2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int u = 0; u < NUC; ++u)
+#pragma unroll
+        for (int o = 0; o < NO; ++o) y[c][u][o][0] = y[c][u][o][1] = 0.0;
+#pragma unroll 1
+    for (int t = 0; t < NT; ++t) {
+      double acc[NI][4][2];
+#pragma unroll
+      for (int f = 0; f < NI; ++f)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[f][c][0] = acc[f][c][1] = 0.0;
+      const double *syn_t = a.syn + (size_t)t * 32 + lane;
+#pragma unroll
+      for (int s = 0; s < KSC; ++s)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int ks = c * KSC + s, kt = a.ks_off[c] + (s < a.KS[c] ? s : 0);
+          const double bv = __ldg(syn_t + (size_t)kt * NT * 32);
+#pragma unroll
+          for (int f = 0; f < NI; ++f) {
+            double av = xs[(f * KS_tot + ks) * 32];
+            if ((ADJ == 1 && f < 3) || (ADJ == 2 && f >= 3)) av *= (s == 0 && q == 0 && (c & 1) == 0) ? invN : twoN;
+            dmma(acc[f][c], av, bv);
+          }
+        }
+      if (t == NT - 1 && tile + step < tiles) {  // the coefficients are read: the next tile's may arrive
+        __syncwarp();
+        stage(buf, tile + step);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        double v[4][NI], gq[4][NO];
+#pragma unroll
+        for (int f = 0; f < NI; ++f) {
+          const double A = acc[f][0][e] + acc[f][1][e], B = acc[f][0][e] - acc[f][1][e];
+          const double C = acc[f][2][e] + acc[f][3][e], D = acc[f][3][e] - acc[f][2][e];
+          v[0][f] = A + C;  // theta
+          v[1][f] = B + D;  // pi - theta
+          v[2][f] = B - D;  // pi + theta
+          v[3][f] = A - C;  // 2 pi - theta
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) EKDef<EK>::op(v[r], gq[r]);
+        double P[4][NO];
+#pragma unroll
+        for (int o = 0; o < NO; ++o) {
+          const double s14 = gq[0][o] + gq[3][o], d14 = gq[0][o] - gq[3][o];
+          const double s23 = gq[1][o] + gq[2][o], d32 = gq[2][o] - gq[1][o];
+          P[0][o] = s14 + s23;  // PE
+          P[1][o] = s14 - s23;  // PO
+          P[2][o] = d14 + d32;  // QE
+          P[3][o] = d14 - d32;  // QO
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int u = 0; u < NUC; ++u) {
+            const int ut = a.nu_off[c] + (u < a.NU[c] ? u : 0);
+            const double bv = __ldg(ana0 + ((size_t)ut * NT + t) * 64 + e * 32);
+#pragma unroll
+            for (int o = 0; o < NO; ++o) dmma(y[c][u][o], P[c][o], bv);
+          }
+      }
+    }
+    const int64_t p = tile * 8 + g;
+    if (p >= a.np) continue;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int u = 0; u < NUC; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int kk = 8 * u + 2 * q + h;
+          if (kk >= a.ke[c]) continue;
+          const int n = class_mode(c, kk);
+#pragma unroll
+          for (int o = 0; o < NO; ++o) {
+            double *dst = a.out[o] + (int64_t)b * a.out_bs[o] + p * a.out_ps + (int64_t)n * a.out_ldm[o] +
+                          (c >= 2 ? a.np * a.out_ps : 0);
+            const double r = (c == 2 && n == 0) ? 0.0 : y[c][u][o][h];
+            if (a.accumulate)
+              *dst += r;
+            else
+              *dst = r;
+          }
+        }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // third-fold building blocks (class split, one angle tile per warp pair, M with tf_NT(M) even)
 // ---------------------------------------------------------------------------
 // Warp w of a CTA: angle tile tau = w / 2, half h = w % 2 (0: cosine classes, 1: sine classes).  It
@@ -680,9 +844,10 @@ struct FieldSet {  // NG scalar fields: cos of mode n, point p at p[f][p + n*ldm
 
 // Stages the NG fields of the 8-point tile at p0 into xs [NG][KS_tot][4][8] (rows in group order:
 // CE0, CE2, CO, SE0, SE2, SO) with cp.async and commits one group.  Four consecutive threads copy one
-// row (two points each, one 16-byte copy when the row is 16-byte aligned).
+// row (two points each, one 16-byte copy when the row is 16-byte aligned).  The modes from m on are zero.
 template <int M, int NG>
-__device__ __forceinline__ void tf_stage(double *xs, const FieldSet<NG> &fs, int64_t p0, int64_t np, bool vec16) {
+__device__ __forceinline__ void tf_stage(double *xs, const FieldSet<NG> &fs, int64_t p0, int64_t np, bool vec16,
+                                         int m = M) {
   constexpr int KS_tot = TfGeo<M>::KS_tot, KT = TfGeo<M>::KT;
   const int pc = 2 * (threadIdx.x & 3), rstep = blockDim.x >> 2;
   const bool v16 = vec16 && p0 + 8 <= np;
@@ -696,7 +861,7 @@ __device__ __forceinline__ void tf_stage(double *xs, const FieldSet<NG> &fs, int
     const int keg = gr % 3 == 0 ? tf_ke(M, 0) : gr % 3 == 1 ? tf_ke(M, 1) : tf_ke(M, 2);
     const int k = r - 4 * kg, n = tf_mode(gr, k);
     double *dst0 = xs + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
-    const bool live = k < keg && !(gr == 3 && k == 0);  // the sine of mode 0 is ignored
+    const bool live = k < keg && n < m && !(gr == 3 && k == 0);  // the sine of mode 0 is ignored
     const int64_t off = p0 + pc + (gr >= 3 ? np : 0);
 #pragma unroll
     for (int f = 0; f < NG; ++f) {
@@ -799,7 +964,7 @@ struct OutSet {  // NO output fields: cos of mode n, point p at p[o][p*ps + n*ld
 // variant (weights or not); accumulate: add to the outputs.
 template <int M, int NO>
 __device__ __forceinline__ void tf_analysis(const double *ps, const double *ana, const OutSet<NO> &os, int64_t p0,
-                                            int64_t np, int64_t out_ps, bool accumulate) {
+                                            int64_t np, int64_t out_ps, bool accumulate, int m = M) {
   constexpr int NT = TfGeo<M>::NT, NU_tot = TfGeo<M>::NU_tot;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
   const int q = lane & 3;
@@ -879,6 +1044,7 @@ __device__ __forceinline__ void tf_analysis(const double *ps, const double *ana,
       const int kk = 8 * u + 2 * q + h;
       if (kk >= keg) continue;
       const int n = tf_mode(gr, kk);
+      if (n >= m) continue;
 #pragma unroll
       for (int o = 0; o < NO; ++o) {
         double *dst = os.p[o] + p * out_ps + (int64_t)n * os.ldm[o] + (gr >= 3 ? np * out_ps : 0);
@@ -892,7 +1058,7 @@ __device__ __forceinline__ void tf_analysis(const double *ps, const double *ana,
   }
 }
 
-// The FAST kernel with the third fold (one elementary program, class split, NT even: M = 64).
+// The FAST kernel with the third fold (one elementary program, class split, NT even: M = 64, a.m <= M modes).
 template <int EK, int M, int ADJ>
 __global__ void __launch_bounds__(384, EK == EK_CROSS ? 3 : 0) fast_tf_kernel(const FastArgs a) {
   static_assert(third_fold(M), "third fold needs the specialised geometry");
@@ -909,7 +1075,7 @@ __global__ void __launch_bounds__(384, EK == EK_CROSS ? 3 : 0) fast_tf_kernel(co
     fs.p[f] = a.in[f] + (int64_t)b * a.in_bs[f];
     fs.ldm[f] = a.in_ldm[f];
   }
-  tf_stage<M, NI>(xs, fs, p0, a.np, a.vec16);
+  tf_stage<M, NI>(xs, fs, p0, a.np, a.vec16, a.m);
   cp_async_wait_0();
   __syncthreads();
   double acc_e[NI][2], acc_o[NI][2];
@@ -929,7 +1095,7 @@ __global__ void __launch_bounds__(384, EK == EK_CROSS ? 3 : 0) fast_tf_kernel(co
     os.ldm[o] = a.out_ldm[o];
   }
   tf_analysis<M, NO>(ps, a.ana + (size_t)(a.adj_out ? 1 : 0) * TfGeo<M>::ASTEPS * 32, os, p0, a.np, a.out_ps,
-                     a.accumulate != 0);
+                     a.accumulate != 0, a.m);
 }
 
 // The Gauss-point cross products with their operands built in the staging (third fold, M = 64):
@@ -1229,24 +1395,27 @@ __global__ void __launch_bounds__(384, 2) fast_bundle_tf_kernel(const BundleArgs
   tf_analysis<M, 3>(ps, a.ana, outs3(6), p0, a.np, 1, false);  // j x b
 }
 
-template <int EK, int M, int ADJ>
+template <int EK, int KSC, int NTC, int ADJ>
 int launch_ek_m(FastArgs &fa, int batch, cudaStream_t st) {
   constexpr int NI = EKDef<EK>::NI, NO = EKDef<EK>::NO;
   static_assert(ek_nin(EK) == NI && ek_nout(EK) == NO, "elementary program table");
-  constexpr bool CS = class_split(EK, M);
+  constexpr bool CS = class_split(EK, KSC);
   fa.KT = 4 * (fa.KS[0] + fa.KS[1] + fa.KS[2] + fa.KS[3]);
-  const size_t smem = fast_smem_bytes(EK, fa.NT, fa.KT, CS);
+  size_t smem = fast_smem_bytes(EK, fa.NT, fa.KT, CS);
   if (smem > 200 * 1024) return set_error(SFNL_ERR_UNSUPPORTED, "FAST form: m too large for shared memory");
   const int tiles_per_pass = fa.NT < 8 ? fa.NT : 8;
   const int nw = CS ? 2 * tiles_per_pass : (tiles_per_pass < 2 ? 2 : tiles_per_pass);
-  auto kern = fast_kernel<EK, M, ADJ, CS>;
-  if constexpr (CS && third_fold(M)) {
-    if (fa.allow_tf) {  // the third-fold kernel (same shared memory and warps, its own tables)
+  auto kern = fast_kernel<EK, KSC, NTC, ADJ, CS>;
+  if constexpr (CS && NTC == 6) {
+    // the third-fold kernel of 64 modes (same warps, its own tables), the modes from m on zero: from m = 55, where
+    // the class-split kernel needs its six angle tiles too (50,001 points: m = 60 0.38 -> 0.24 ms)
+    if (fa.allow_tf) {
       Tables T;
-      if (int rc = get_tf_tables(make_geo(fa.m), &T)) return rc;
+      if (int rc = get_tf_tables(make_geo(64), &T)) return rc;
       fa.syn = T.syn;
       fa.ana = T.ana;
-      kern = fast_tf_kernel<EK, M, ADJ>;
+      kern = fast_tf_kernel<EK, 64, ADJ>;
+      smem = fast_smem_bytes(EK, NTC, 4 * TfGeo<64>::KS_tot, CS);
     }
   }
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -1258,13 +1427,47 @@ int launch_ek_m(FastArgs &fa, int batch, cudaStream_t st) {
   return check_launch("fast form");
 }
 
+// The solo kernel where every class has at most solo_max_ks(EK) k-steps.
+template <int EK, int KSC, int ADJ>
+int launch_solo(FastArgs &fa, int batch, cudaStream_t st) {
+  constexpr size_t smem = solo_smem_bytes(EK, KSC);
+  auto kern = solo_kernel<EK, KSC, ADJ>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (fast form)");
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kSoloWarps, smem) != cudaSuccess || per_sm < 1)
+    return set_error(SFNL_ERR_CUDA, "fast form: no resident CTA");
+  const int64_t ctas = ((fa.np + 7) / 8 + kSoloWarps - 1) / kSoloWarps, cap = (int64_t)num_sms() * per_sm;
+  kern<<<dim3((unsigned)(ctas < cap ? ctas : cap), (unsigned)batch), 32 * kSoloWarps, smem, st>>>(fa);
+  return check_launch("fast form");
+}
+
 template <int EK, int ADJ>
 int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
-  switch (fa.m) {
-    case 16: return launch_ek_m<EK, 16, ADJ>(fa, batch, st);
-    case 32: return launch_ek_m<EK, 32, ADJ>(fa, batch, st);
-    case 64: return launch_ek_m<EK, 64, ADJ>(fa, batch, st);
-    default: return launch_ek_m<EK, 0, ADJ>(fa, batch, st);
+  if constexpr (solo_ek(EK)) {
+    if (fa.KS[0] == 1) return launch_solo<EK, 1, ADJ>(fa, batch, st);
+    if (fa.KS[0] == 2) return launch_solo<EK, 2, ADJ>(fa, batch, st);
+    if constexpr (solo_max_ks(EK) == 4) {
+      if (fa.KS[0] == 3) return launch_solo<EK, 3, ADJ>(fa, batch, st);
+      if (fa.KS[0] == 4) return launch_solo<EK, 4, ADJ>(fa, batch, st);
+    }
+  }
+  // every (KS, NT) of make_geo up to m = 64; run-time loops cost the sizes between 16, 32 and 64 a third of their time
+  // (cross product, 50,001 points: m = 20 99 -> 62 us, m = 40 207 -> 148, m = 48 337 -> 202, m = 52 384 -> 229)
+  switch (10 * fa.KS[0] + fa.NT) {
+    case 11: return launch_ek_m<EK, 1, 1, ADJ>(fa, batch, st);
+    case 21: return launch_ek_m<EK, 2, 1, ADJ>(fa, batch, st);
+    case 22: return launch_ek_m<EK, 2, 2, ADJ>(fa, batch, st);
+    case 32: return launch_ek_m<EK, 3, 2, ADJ>(fa, batch, st);
+    case 33: return launch_ek_m<EK, 3, 3, ADJ>(fa, batch, st);
+    case 43: return launch_ek_m<EK, 4, 3, ADJ>(fa, batch, st);
+    case 54: return launch_ek_m<EK, 5, 4, ADJ>(fa, batch, st);
+    case 64: return launch_ek_m<EK, 6, 4, ADJ>(fa, batch, st);
+    case 65: return launch_ek_m<EK, 6, 5, ADJ>(fa, batch, st);
+    case 75: return launch_ek_m<EK, 7, 5, ADJ>(fa, batch, st);
+    case 76: return launch_ek_m<EK, 7, 6, ADJ>(fa, batch, st);
+    case 86: return launch_ek_m<EK, 8, 6, ADJ>(fa, batch, st);
+    default: return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);
   }
 }
 
@@ -1375,15 +1578,15 @@ int fast_grid_length(int m) { return make_geo(m).N; }
 bool gauss_cross_fused_supported(int m, int n_w) { return third_fold(64) && m == 64 && n_w == 6; }
 
 namespace {
-template <int EK, int GK, int M>
+template <int EK, int GK, int KSC, int NTC>
 int launch_gauss_general_m(FastArgs &fa, int64_t ng, cudaStream_t st) {
-  constexpr bool CS = class_split(EK, M);
+  constexpr bool CS = class_split(EK, KSC);
   fa.KT = 4 * (fa.KS[0] + fa.KS[1] + fa.KS[2] + fa.KS[3]);
   const size_t smem = fast_smem_bytes(EK, fa.NT, fa.KT, CS);
   if (smem > 200 * 1024) return set_error(SFNL_ERR_UNSUPPORTED, "fused Gauss-point product: m too large");
   const int tiles_per_pass = fa.NT < 8 ? fa.NT : 8;
   const int nw = CS ? 2 * tiles_per_pass : (tiles_per_pass < 2 ? 2 : tiles_per_pass);
-  auto kern = fast_kernel<EK, M, 0, CS, GK>;
+  auto kern = fast_kernel<EK, KSC, NTC, 0, CS, GK>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (fused Gauss-point product)");
   const int64_t tiles = (ng + 7) / 8;
@@ -1391,14 +1594,22 @@ int launch_gauss_general_m(FastArgs &fa, int64_t ng, cudaStream_t st) {
   kern<<<(unsigned)tiles, nw * 32, smem, st>>>(fa);
   return check_launch("fused Gauss-point product");
 }
-// the geometries the plain products specialise (m = 16, 32, 64), else run-time geometry
 template <int EK, int GK>
 int launch_gauss_general(FastArgs &fa, int64_t ng, cudaStream_t st) {
-  switch (fa.m) {
-    case 16: return launch_gauss_general_m<EK, GK, 16>(fa, ng, st);
-    case 32: return launch_gauss_general_m<EK, GK, 32>(fa, ng, st);
-    case 64: return launch_gauss_general_m<EK, GK, 64>(fa, ng, st);
-    default: return launch_gauss_general_m<EK, GK, 0>(fa, ng, st);
+  switch (10 * fa.KS[0] + fa.NT) {
+    case 11: return launch_gauss_general_m<EK, GK, 1, 1>(fa, ng, st);
+    case 21: return launch_gauss_general_m<EK, GK, 2, 1>(fa, ng, st);
+    case 22: return launch_gauss_general_m<EK, GK, 2, 2>(fa, ng, st);
+    case 32: return launch_gauss_general_m<EK, GK, 3, 2>(fa, ng, st);
+    case 33: return launch_gauss_general_m<EK, GK, 3, 3>(fa, ng, st);
+    case 43: return launch_gauss_general_m<EK, GK, 4, 3>(fa, ng, st);
+    case 54: return launch_gauss_general_m<EK, GK, 5, 4>(fa, ng, st);
+    case 64: return launch_gauss_general_m<EK, GK, 6, 4>(fa, ng, st);
+    case 65: return launch_gauss_general_m<EK, GK, 6, 5>(fa, ng, st);
+    case 75: return launch_gauss_general_m<EK, GK, 7, 5>(fa, ng, st);
+    case 76: return launch_gauss_general_m<EK, GK, 7, 6>(fa, ng, st);
+    case 86: return launch_gauss_general_m<EK, GK, 8, 6>(fa, ng, st);
+    default: return launch_gauss_general_m<EK, GK, 0, 0>(fa, ng, st);
   }
 }
 constexpr int gauss_ek(int kind, bool conservative) {

@@ -40,8 +40,11 @@ inline Geo make_geo(int m) {
   g.KS_tot = g.NU_tot = 0;
   for (int c = 0; c < 4; ++c) {
     g.ke[c] = cnt[c];
-    g.KS[c] = (cnt[c] + 3) / 4;
-    g.NU[c] = (cnt[c] + 7) / 8;
+    // up to m = 64 every class has the k-steps and output tiles of the largest one (zero table entries where it has
+    // fewer modes), so that the fused kernels' geometry is two compile-time numbers, KS and NT
+    const int k = m <= 64 ? ev : cnt[c];
+    g.KS[c] = (k + 3) / 4;
+    g.NU[c] = (k + 7) / 8;
     g.ks_off[c] = g.KS_tot;
     g.nu_off[c] = g.NU_tot;
     g.KS_tot += g.KS[c];
