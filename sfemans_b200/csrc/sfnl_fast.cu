@@ -360,22 +360,72 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
   double *xs = overlay ? smem : smem + prod_d + xch_d;
   if constexpr (GK >= 0) {
     // the operands of the tile's 8 Gauss points and every mode, from the nodal fields: mode i's cosine
-    // row is 4*KOFF[i & 1] + (i >> 1), its sine row 4*KOFF[2 + (i & 1)] + (i >> 1); other rows stay 0
-    for (int t = threadIdx.x; t < NI * KS_tot * 32; t += blockDim.x) xs[t] = 0.0;
+    // row is 4*KOFF[i & 1] + (i >> 1), its sine row 4*KOFF[2 + (i & 1)] + (i >> 1); other rows are 0
+    // Each point's nodes, basis values and derivatives are gathered once (not once per mode).
+    constexpr int NWMAX = 6;  // up to P2 triangles; larger elements read the mesh arrays for every mode
+    __shared__ int s_node[8 * NWMAX];
+    __shared__ double s_wt[8 * NWMAX], s_g1[8 * NWMAX], s_g2[8 * NWMAX], s_ray[8];
+    const int n_w = a.ga.n_w;
+    if (n_w <= NWMAX)
+      for (int it = threadIdx.x; it < 8 * n_w; it += blockDim.x) {
+        const int gp = it / n_w, n = it - gp * n_w, at = gp * NWMAX + n;
+        if (p0 + gp < a.np) gauss_node(a.ga, p0 + gp, n, s_node[at], s_wt[at], s_g1[at], s_g2[at]);
+      }
     __syncthreads();
+    if (threadIdx.x < 8 && p0 + threadIdx.x < a.np) {
+      double ray = 0.0;
+      for (int n = 0; n < n_w; ++n) {
+        int node = 0;
+        double wt = 0.0, g1, g2;
+        if (n_w <= NWMAX) {
+          node = s_node[threadIdx.x * NWMAX + n];
+          wt = s_wt[threadIdx.x * NWMAX + n];
+        } else {
+          gauss_node(a.ga, p0 + threadIdx.x, n, node, wt, g1, g2);
+        }
+        ray = fma(a.ga.rr[2 * (size_t)node], wt, ray);
+      }
+      s_ray[threadIdx.x] = ray;
+    }
+    __syncthreads();
+    // A warp takes one k-step of a parity, 4 modes of the 8 points: its lanes fill whole A-fragment blocks (a warp on
+    // 32 modes of one point stored to two banks, 8 lanes each), and the points, most of them of one element, read
+    // the same nodal values.  Navier-Stokes caller, 101,150 Gauss points of P2 triangles: m = 32 0.311 -> 0.284 ms, m = 20
+    // 0.204 -> 0.185 ms (the third-fold kernels at m = 64 0.750 -> 0.701 ms); one more warp for the analysis' eight output
+    // tiles changed nothing at m = 32 and cost a quarter at m = 20.
     const int m = a.m;
-    for (int it = threadIdx.x; it < 8 * m; it += blockDim.x) {
-      const int i = it % m, gp = it / m;  // a warp takes consecutive modes of one point
-      if (p0 + gp >= a.np) continue;
+    for (int it = warp; it < KS[0] + KS[1]; it += NW) {
+      const int c = it >= KS[0], s = it - (c ? KS[0] : 0), kq = lane >> 3, gp = lane & 7;
+      const int i = class_mode(c, 4 * s + kq);
+      const bool live = i < m && p0 + gp < a.np;
+      const int me = live ? (int)((p0 + gp) / a.ga.l_G) : 0;
       double f[8][2];
-      gauss_operands_nm<GK>(a.ga, p0 + gp, i, m, f);
-      const int c = i & 1, k = i >> 1;
-      const int rc = 4 * sel4(KOFF, c) + k, rs = 4 * sel4(KOFF, 2 + c) + k;
-      const int oc = (rc >> 2) * 32 + a_frag_slot(rc & 3, gp), os = (rs >> 2) * 32 + a_frag_slot(rs & 3, gp);
+      if (!live)
+#pragma unroll
+        for (int fi = 0; fi < 8; ++fi) f[fi][0] = f[fi][1] = 0.0;
+      else if (n_w <= NWMAX)
+        gauss_operands_geo<GK, NWMAX>(
+            a.ga,
+            [&](int n, int &node, double &wt, double &g1, double &g2) {
+              const int at = gp * NWMAX + n;
+              node = s_node[at];
+              wt = s_wt[at];
+              g1 = s_g1[at];
+              g2 = s_g2[at];
+            },
+            s_ray[gp], me, i, m, f);
+      else
+        gauss_operands_geo<GK, 0>(
+            a.ga,
+            [&](int n, int &node, double &wt, double &g1, double &g2) {
+              gauss_node(a.ga, p0 + gp, n, node, wt, g1, g2);
+            },
+            s_ray[gp], me, i, m, f);
+      const int oc = (sel4(KOFF, c) + s) * 32 + a_frag_slot(kq, gp), os = (sel4(KOFF, 2 + c) + s) * 32 + a_frag_slot(kq, gp);
 #pragma unroll
       for (int fi = 0; fi < NI; ++fi) {
         xs[(size_t)fi * KS_tot * 32 + oc] = f[fi][0];
-        if (i != 0) xs[(size_t)fi * KS_tot * 32 + os] = f[fi][1];  // the sine of mode 0 is ignored
+        xs[(size_t)fi * KS_tot * 32 + os] = i == 0 ? 0.0 : f[fi][1];  // the sine of mode 0 is ignored
       }
     }
   } else {
@@ -1101,11 +1151,10 @@ __global__ void __launch_bounds__(384, EK == EK_CROSS ? 3 : 0) fast_tf_kernel(co
 // The Gauss-point cross products with their operands built in the staging (third fold, M = 64):
 // Navier-Stokes (curl u + 2 Om) x u (GK_NS) and Lorentz force (curl H) x B (GK_LORENTZ).  The tile's
 // 8 Gauss points get the curl and values of every mode straight from the nodal fields (node-major
-// copies: the element's nodes gathered through jj, the lanes of a warp reading 32 consecutive modes of
-// one node) into the coefficient layout, so the (l_G*me, 6, m) operand arrays never go through HBM.
+// copies: the element's nodes gathered through jj) into the coefficient layout, so the (l_G*me, 6, m) operand arrays never go through HBM.
 template <int M, int KIND>
 __global__ void __launch_bounds__(384, 2) gauss_tf_cross_kernel(const FastArgs a, const GaussArgs ga) {
-  static_assert(third_fold(M), "third fold needs the specialised geometry");
+  static_assert(third_fold(M) && tf_KS(M, 0) * 16 == M && tf_KS(M, 1) * 16 == M, "every staged row holds a mode");
   constexpr int NI = 6, NO = 3, NT = TfGeo<M>::NT, KS_tot = TfGeo<M>::KS_tot;
   constexpr size_t fstride = (size_t)KS_tot * 32;
   extern __shared__ double smem[];
@@ -1115,7 +1164,6 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_cross_kernel(const FastArgs a
   constexpr int NW = 6;  // P2 elements
   __shared__ int s_node[8][NW];
   __shared__ double s_wt[8][NW], s_g1[8][NW], s_g2[8][NW], s_ray[8];
-  for (int t = threadIdx.x; t < NI * (int)fstride; t += blockDim.x) xs[t] = 0.0;  // padding rows, sine of mode 0
   if (threadIdx.x < 8 * NW) {  // the points' nodes, basis values and derivatives (mesh%jj, ww, dw)
     const int g = threadIdx.x / NW, n = threadIdx.x % NW;
     const int64_t p = p0 + g < a.np ? p0 + g : a.np - 1;
@@ -1136,23 +1184,24 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_cross_kernel(const FastArgs a
     s_ray[threadIdx.x] = ray;
   }
   __syncthreads();
-  for (int it = threadIdx.x; it < 8 * M; it += blockDim.x) {
-    const int i = it % M, g = it / M;  // mode index, point of the tile: a warp reads 32 modes of a node
-    if (p0 + g >= a.np) continue;
+  // a warp takes one k-step of a group of modes (CE0, CE2, CO), 4 modes of the 8 points, as in fast_kernel (the points
+  // past np repeat the last one and are not stored)
+  for (int it = threadIdx.x >> 5; it < KS_tot / 2; it += blockDim.x >> 5) {
+    const int gc = it < tf_koff(M, 1) ? 0 : it < tf_koff(M, 2) ? 1 : 2;
+    const int s = it - (gc == 0 ? 0 : gc == 1 ? tf_koff(M, 1) : tf_koff(M, 2));
+    const int g = threadIdx.x & 7, kq = (threadIdx.x & 31) >> 3, i = tf_mode(gc, 4 * s + kq);
     double rot[6], w[6];
     gauss_curl_gathered<KIND, M, NW>(ga, s_node[g], s_wt[g], s_g1[g], s_g2[g], s_ray[g], i, rot, w);
     // rows of mode i: cosine group CE0 (i = 0 mod 4), CE2 (i = 2 mod 4) or CO (odd), sine group 3 further
-    const int gc = (i & 1) ? 2 : (i & 3) == 0 ? 0 : 1, k = (i & 1) ? i >> 1 : i >> 2;
-    const int rc = 4 * tf_koff(M, gc) + k, rs = 4 * tf_koff(M, gc + 3) + k;
-    const int oc = (rc >> 2) * 32 + a_frag_slot(rc & 3, g), os = (rs >> 2) * 32 + a_frag_slot(rs & 3, g);
+    const int kc = gc == 0 ? 0 : gc == 1 ? tf_koff(M, 1) : tf_koff(M, 2);
+    const int ks = gc == 0 ? tf_koff(M, 3) : gc == 1 ? tf_koff(M, 4) : tf_koff(M, 5);
+    const int oc = (kc + s) * 32 + a_frag_slot(kq, g), os = (ks + s) * 32 + a_frag_slot(kq, g);
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       xs[f * fstride + oc] = rot[2 * f];
       xs[(3 + f) * fstride + oc] = w[2 * f];
-      if (i != 0) {  // the sine of mode 0 is ignored
-        xs[f * fstride + os] = rot[2 * f + 1];
-        xs[(3 + f) * fstride + os] = w[2 * f + 1];
-      }
+      xs[f * fstride + os] = i == 0 ? 0.0 : rot[2 * f + 1];  // the sine of mode 0 is ignored
+      xs[(3 + f) * fstride + os] = i == 0 ? 0.0 : w[2 * f + 1];
     }
   }
   __syncthreads();
@@ -1184,7 +1233,7 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_cross_kernel(const FastArgs a
 // capacity or null.
 template <int M, bool CONS>
 __global__ void __launch_bounds__(384, 2) gauss_tf_advect_kernel(const FastArgs a, const GaussArgs ga) {
-  static_assert(third_fold(M), "third fold needs the specialised geometry");
+  static_assert(third_fold(M) && tf_KS(M, 0) * 16 == M && tf_KS(M, 1) * 16 == M, "every staged row holds a mode");
   constexpr int NI = CONS ? 8 : 6, NT = TfGeo<M>::NT, KS_tot = TfGeo<M>::KS_tot;
   constexpr size_t fstride = (size_t)KS_tot * 32;
   extern __shared__ double smem[];
@@ -1194,7 +1243,6 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_advect_kernel(const FastArgs 
   constexpr int NW = 6;  // P2 elements
   __shared__ int s_node[8][NW];
   __shared__ double s_wt[8][NW], s_g1[8][NW], s_g2[8][NW], s_ray[8], s_heat[8];
-  for (int t = threadIdx.x; t < NI * (int)fstride; t += blockDim.x) xs[t] = 0.0;  // padding rows, sine of mode 0
   if (threadIdx.x < 8 * NW) {  // the points' nodes, basis values and derivatives (mesh%jj, ww, dw)
     const int g = threadIdx.x / NW, n = threadIdx.x % NW;
     const int64_t p = p0 + g < a.np ? p0 + g : a.np - 1;
@@ -1216,9 +1264,12 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_advect_kernel(const FastArgs 
     s_ray[threadIdx.x] = ray;
   }
   __syncthreads();
-  for (int it = threadIdx.x; it < 8 * M; it += blockDim.x) {
-    const int i = it % M, g = it / M;  // mode index, point of the tile: a warp reads 32 modes of a node
-    if (p0 + g >= a.np) continue;
+  // a warp takes one k-step of a group of modes (CE0, CE2, CO), 4 modes of the 8 points, as in fast_kernel (the points
+  // past np repeat the last one and are not stored)
+  for (int it = threadIdx.x >> 5; it < KS_tot / 2; it += blockDim.x >> 5) {
+    const int gc = it < tf_koff(M, 1) ? 0 : it < tf_koff(M, 2) ? 1 : 2;
+    const int s = it - (gc == 0 ? 0 : gc == 1 ? tf_koff(M, 1) : tf_koff(M, 2));
+    const int g = threadIdx.x & 7, kq = (threadIdx.x & 31) >> 3, i = tf_mode(gc, 4 * s + kq);
     double wv[6] = {0, 0, 0, 0, 0, 0}, d1[6] = {0, 0, 0, 0, 0, 0}, d2[6] = {0, 0, 0, 0, 0, 0};
     double cw[2] = {0, 0}, c1[2] = {0, 0}, c2[2] = {0, 0};
 #pragma unroll
@@ -1263,13 +1314,13 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_advect_kernel(const FastArgs 
       f[7][1] = hc * cw[1];
     }
     // rows of mode i: cosine group CE0 (i = 0 mod 4), CE2 (i = 2 mod 4) or CO (odd), sine group 3 further
-    const int gc = (i & 1) ? 2 : (i & 3) == 0 ? 0 : 1, k = (i & 1) ? i >> 1 : i >> 2;
-    const int rc = 4 * tf_koff(M, gc) + k, rs = 4 * tf_koff(M, gc + 3) + k;
-    const int oc = (rc >> 2) * 32 + a_frag_slot(rc & 3, g), os = (rs >> 2) * 32 + a_frag_slot(rs & 3, g);
+    const int kc = gc == 0 ? 0 : gc == 1 ? tf_koff(M, 1) : tf_koff(M, 2);
+    const int ks = gc == 0 ? tf_koff(M, 3) : gc == 1 ? tf_koff(M, 4) : tf_koff(M, 5);
+    const int oc = (kc + s) * 32 + a_frag_slot(kq, g), os = (ks + s) * 32 + a_frag_slot(kq, g);
 #pragma unroll
     for (int fi = 0; fi < NI; ++fi) {
       xs[fi * fstride + oc] = f[fi][0];
-      if (i != 0) xs[fi * fstride + os] = f[fi][1];  // the sine of mode 0 is ignored
+      xs[fi * fstride + os] = i == 0 ? 0.0 : f[fi][1];  // the sine of mode 0 is ignored
     }
   }
   __syncthreads();

@@ -108,19 +108,21 @@ __device__ __forceinline__ void gauss_curl_gathered(const GaussArgs &a, const in
 // and the Lorentz field a.v2, 2 for the advection scalar a.v2).  f[field][cos, sin]:
 //   GK_NS, GK_LORENTZ: fields 0-2 = RotV (r, theta, z), 3-5 = W;
 //   GK_ADVECT: 0-2 = heat grad c, 3-5 = u, 6 = div u, 7 = heat c (subroutine_temperature_with_T.F90:300-331).
-template <int KIND>
-__device__ __forceinline__ void gauss_operands_nm(const GaussArgs &a, int64_t p, int i, int tm, double (&f)[8][2]) {
-  const int me = (int)(p / a.l_G), l = (int)(p % a.l_G);
+//
+// The geometry of the point comes from geo(n, node, wt, g1, g2), node n's number (0-based, inside the fields), basis
+// value and derivatives, and from ray; NW > 0: at most NW nodes, the loop unrolled so that all loads of the nodal
+// values are in flight together, NW = 0: any number.
+template <int KIND, int NW, typename Geo>
+__device__ __forceinline__ void gauss_operands_geo(const GaussArgs &a, Geo geo, double ray, int me, int i, int tm,
+                                                   double (&f)[8][2]) {
   const double mode = (double)a.list_mode[i];
-  const double *dwl = a.dw + (size_t)2 * a.n_w * (l + (size_t)a.l_G * me);
-  double ray = 0.0, wv[6] = {0, 0, 0, 0, 0, 0}, d1[6] = {0, 0, 0, 0, 0, 0}, d2[6] = {0, 0, 0, 0, 0, 0};
+  double wv[6] = {0, 0, 0, 0, 0, 0}, d1[6] = {0, 0, 0, 0, 0, 0}, d2[6] = {0, 0, 0, 0, 0, 0};
   double om[6] = {0, 0, 0, 0, 0, 0}, w2[6] = {0, 0, 0, 0, 0, 0};
   double cw[2] = {0, 0}, c1[2] = {0, 0}, c2[2] = {0, 0};
-  for (int n = 0; n < a.n_w; ++n) {
-    int node = a.jj[n + (size_t)a.n_w * me] - 1;  // 1-based node numbers
-    node = node < 0 ? 0 : node >= a.np_nodes ? a.np_nodes - 1 : node;  // no access outside the fields
-    const double wt = a.ww[n + (size_t)a.n_w * l], g1 = dwl[2 * n], g2 = dwl[2 * n + 1];
-    ray = fma(a.rr[2 * (size_t)node], wt, ray);
+  auto add = [&](int n) {
+    int node;
+    double wt, g1, g2;
+    geo(n, node, wt, g1, g2);
     const double *vn = a.v + (size_t)node * 6 * tm + i;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -149,6 +151,13 @@ __device__ __forceinline__ void gauss_operands_nm(const GaussArgs &a, int64_t p,
         c2[k] = fma(cs, g2, c2[k]);
       }
     }
+  };
+  if constexpr (NW > 0) {
+#pragma unroll
+    for (int n = 0; n < NW; ++n)
+      if (n < a.n_w) add(n);
+  } else {
+    for (int n = 0; n < a.n_w; ++n) add(n);
   }
   if constexpr (KIND == GK_ADVECT) {
     const double mr = mode / ray, hc = a.heat ? a.heat[me] : 1.0;
@@ -179,6 +188,18 @@ __device__ __forceinline__ void gauss_operands_nm(const GaussArgs &a, int64_t p,
     }
     f[6][0] = f[6][1] = f[7][0] = f[7][1] = 0.0;
   }
+}
+
+// Node n (0-based, clamped to the fields) of Gauss point p with its basis value and derivatives.
+__device__ __forceinline__ void gauss_node(const GaussArgs &a, int64_t p, int n, int &node, double &wt, double &g1,
+                                           double &g2) {
+  const int me = (int)(p / a.l_G), l = (int)(p % a.l_G);
+  const double *dwl = a.dw + (size_t)2 * a.n_w * (l + (size_t)a.l_G * me);
+  node = a.jj[n + (size_t)a.n_w * me] - 1;  // 1-based node numbers
+  node = node < 0 ? 0 : node >= a.np_nodes ? a.np_nodes - 1 : node;  // no access outside the fields
+  wt = a.ww[n + (size_t)a.n_w * l];
+  g1 = dwl[2 * n];
+  g2 = dwl[2 * n + 1];
 }
 
 }  // namespace sfnl
