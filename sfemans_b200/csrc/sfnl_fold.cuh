@@ -242,4 +242,18 @@ __device__ __forceinline__ int sel4(const int (&v)[4], int c) { return c == 0 ? 
 bool fast_fused_fits(int op, int m);
 int launch_fast_large(const ProgArgs &a, const Geo &g, const Tables &T, cudaStream_t st);
 
+// Tables of a residue grid of N/R angles (sfnl_large.cu): synthesis and analysis B fragments and the twiddles
+// cos, sin of n d_r [R][m][2].  Cached per (device, m, N, R).
+struct ResTab {
+  double *base = nullptr;  // syn, ana (two equal variants, no weights), tw
+  double *syn = nullptr, *ana = nullptr;
+  const double *tw = nullptr;
+};
+int get_residue_tables(int m, int N, int R, ResTab *out);
+// The library's device workspace of (stream, use), grown to `bytes` (sfnl_large.cu).
+int large_workspace(cudaStream_t st, size_t bytes, double **out, int use = 0);
+// Residue grids of 128 angles with one program kernel (sfnl_res.cu); cap: bytes of workspace.
+bool res_supported(int op, int m);
+int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st);
+
 }  // namespace sfnl

@@ -525,7 +525,9 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32) large_prod_kernel(const 
 std::mutex g_lws_mu;
 std::map<std::tuple<int, cudaStream_t, int>, std::pair<double *, size_t>> g_lws;
 
-int large_workspace(cudaStream_t st, size_t bytes, double **out, int use = 0) {
+}  // namespace
+
+int large_workspace(cudaStream_t st, size_t bytes, double **out, int use) {
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(g_lws_mu);
@@ -546,6 +548,8 @@ int large_workspace(cudaStream_t st, size_t bytes, double **out, int use = 0) {
   *out = w.first;
   return SFNL_OK;
 }
+
+namespace {
 
 template <int OP, int O0, int CPW>
 int launch_large_prod(const LargeArgs &la, bool tf, cudaStream_t st) {
@@ -633,6 +637,7 @@ int launch_large_syn(const LargeArgs &la, int nfields, int nbz, bool tf, cudaStr
   return set_error(SFNL_ERR_UNSUPPORTED, "large-m FAST form: m too large");
 }
 
+constexpr size_t kResWorkspaceBytes = size_t(2) << 30;    // launch_res: coefficients, base values and sums of a chunk
 constexpr size_t kLargeWorkspaceBytes = size_t(1) << 30;  // grid values of one point chunk
 // Tests only (sfnl_test_large_workspace_cap): a bound on both workspaces far below the production ones, so
 // that small calls run many point chunks and batch groups; 0: none.
@@ -837,24 +842,21 @@ int large_residues(int m, int N) {
   return residues_fit(m, N, 6) ? 6 : residues_fit(m, N, 3) ? 3 : 0;
 }
 
-struct ResTab {
-  double *base = nullptr;  // syn, ana (two equal variants, no weights), tw [R][m][2]
-  double *syn = nullptr, *ana = nullptr;
-  const double *tw = nullptr;
-};
 std::mutex g_res_mu;
-std::map<std::tuple<int, int, int>, ResTab> g_res;  // (device, m, R) -> tables
+std::map<std::tuple<int, int, int, int>, ResTab> g_res;  // (device, m, N, R) -> tables
 
 __host__ __device__ constexpr int res_mode(int gr, int k, int mh) { return (gr == 3 && k == 0) ? mh : tf_mode(gr, k); }
 
 // Third-fold tables of the residue grid (M angles, quadrant tiles NT = M/32, row and output groups of M/2
 // modes with mode M/2 as the sine of group 3's k = 0), laid out like get_tf_tables', and the twiddles
 // cos, sin of n d_r for n < m, r < R.
+}  // namespace
+
 int get_residue_tables(int m, int N, int R, ResTab *out) {
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(g_res_mu);
-  auto it = g_res.find({dev, m, R});
+  auto it = g_res.find({dev, m, N, R});
   if (it != g_res.end()) {
     *out = it->second;
     return SFNL_OK;
@@ -910,10 +912,12 @@ int get_residue_tables(int m, int N, int R, ResTab *out) {
   T.syn = T.base;
   T.ana = T.base + nsyn;
   T.tw = T.base + nsyn + nana;
-  g_res[{dev, m, R}] = T;
+  g_res[{dev, m, N, R}] = T;
   *out = T;
   return SFNL_OK;
 }
+
+namespace {
 
 // The R residues of one input field (batch entry blockIdx.z) at the chunk's points: thread (point, k),
 // k < M/2, gathers Y_k and Y_{M-k} of each residue from the modes qM + k and qM + M - k (k = 0: Y_0 and
@@ -1133,6 +1137,10 @@ void large_res_release_tables() {
 // The two-kernel form: on the grid's residue classes when the grid is 3m angles and m >= 256 (R of them:
 // 3/R of the DMMAs of the whole grid, launch_large_res), else on the whole grid.
 int launch_fast_large(const ProgArgs &a, const Geo &g, const Tables &T, cudaStream_t st) {
+  if (!g_test_residues.load() && res_supported(a.op, a.m)) {
+    const size_t tc = g_test_cap.load();
+    return launch_res(a, tc ? tc : kResWorkspaceBytes, st);
+  }
   if (const int R = large_residues(a.m, g.N)) return launch_large_res(a, g, R, st);
   return run_large(a, g, T, nullptr, st);
 }
