@@ -195,12 +195,17 @@ def to_host(t):
 
 
 def _is_fortran(t) -> bool:
-    expect, s = [], 1
-    for d in t.shape:
-        expect.append(s)
+    if not (t.is_cuda and t.dtype.itemsize == 8):
+        return False
+    shape, stride = t.shape, t.stride()
+    if len(shape) == 3 and stride == (1, shape[0], shape[0] * shape[1]):
+        return True
+    s = 1
+    for d, st in zip(shape, stride):  # the stride of an extent of 1 does not matter
+        if d > 1 and st != s:
+            return t.numel() == 0
         s *= d
-    return t.is_cuda and t.dtype.itemsize == 8 and (t.numel() == 0 or list(t.stride()) == expect
-                                                   or all(st == e for st, e, d in zip(t.stride(), expect, t.shape) if d > 1))
+    return True
 
 
 def _dptr(t, what):
@@ -208,15 +213,26 @@ def _dptr(t, what):
         return None
     if not _is_fortran(t):
         raise ValueError(f"{what}: expected a float64 CUDA tensor in Fortran order (np, nslot, m[, k])")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+_raw_stream = None  # () -> handle of torch's current stream on the current device
 
 
 def _stream(stream):
+    global _raw_stream
     if stream is None:
-        import torch
+        if _raw_stream is None:
+            import torch
 
-        stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream))
+            stream = torch.cuda.current_stream()  # initialises CUDA if need be
+            # the handle alone: building torch's Stream object took 3.6 of the 12.9 us of a small call
+            device, handle = (getattr(torch._C, n, None) for n in ("_cuda_getDevice", "_cuda_getCurrentRawStream"))
+            if device is not None and handle is not None:
+                _raw_stream = lambda: handle(device())  # noqa: E731
+            return stream.cuda_stream
+        return _raw_stream()
+    return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
 # ----------------------------------------------------------------------------
@@ -230,14 +246,14 @@ def product(op: int, a, b, out=None, m_max_pad: int | None = None, n_theta: int 
         raise SfnlError(-1, f"op must be one of OP_* (0..7), got {op}")
     _, nsl_a, nsl_b, nsl_o = KINDS[OP_KIND[op]]
     npts, nsl, m = a.shape
-    if nsl != nsl_a or tuple(b.shape) != (npts, nsl_b, m):
+    if nsl != nsl_a or b.shape != (npts, nsl_b, m):
         raise SfnlError(-2, f"{OP_KIND[op]}: inputs must be (np, {nsl_a}, m) and (np, {nsl_b}, m)")
     if m_max_pad is None:
         m_max_pad = 3 * m // 2
     if out is None:
         out = out_empty(op, npts, m, device=a.device)
     want = (3, npts, 6, m) if op in TENSOR_OPS else (npts, nsl_o, m)
-    if tuple(out.shape) != want:
+    if out.shape != want:
         raise SfnlError(-2, f"{OP_KIND[op]}: output must be {want}")
     if split is None:
         _check(lib().sfnl_product_f64(op, _dptr(a, "a"), _dptr(b, "b"), _dptr(out, "out"), npts, m, m_max_pad,

@@ -78,6 +78,44 @@ int check_launch(const char *what) {
   return SFNL_OK;
 }
 
+namespace {
+std::atomic<uint32_t> g_setup_epoch{1};
+std::mutex g_setup_mu;
+}  // namespace
+
+void KernelSetup::forget_all() { g_setup_epoch.fetch_add(1); }
+
+int KernelSetup::opt_in(const void *kern, size_t smem) {
+  int d = 0;
+  if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= kDevs) return set_error(SFNL_ERR_CUDA, "no current CUDA device");
+  const uint64_t epoch = g_setup_epoch.load();
+  auto done = [&](uint64_t v) { return (v >> 32) == epoch && (v & 0xffffffffu) >= smem; };
+  if (done(smem_[d].load())) return SFNL_OK;
+  std::lock_guard<std::mutex> lk(g_setup_mu);  // the size only grows, also with several threads
+  if (done(smem_[d].load())) return SFNL_OK;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    cudaGetLastError();
+    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed");
+  }
+  smem_[d].store(epoch << 32 | (uint64_t)smem);
+  return SFNL_OK;
+}
+
+int KernelSetup::resident(const void *kern, int threads, size_t smem) {
+  if (int rc = opt_in(kern, smem)) return rc;
+  int d = 0, n = 0;
+  cudaGetDevice(&d);
+  const uint64_t key = ((uint64_t)(g_setup_epoch.load() & 0xffffu) << 48) | ((uint64_t)(smem / 8) << 32) | ((uint64_t)threads << 16);
+  const uint64_t v = shape_[d].load();
+  if ((v & ~uint64_t(0xffff)) == key && (v & 0xffffu)) return (int)(v & 0xffffu);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return set_error(SFNL_ERR_CUDA, "no resident CTA");
+  }
+  shape_[d].store(key | (uint64_t)n);
+  return n;
+}
+
 int num_sms() {
   DevState *s = dev_state();
   if (!s) return 148;
@@ -561,6 +599,7 @@ int sfnl_last_host_timing(double *s3) {
 }
 
 int sfnl_finalize(void) {
+  KernelSetup::forget_all();
   fast_release_tables();
   large_release_workspaces();
   split_release_tables();

@@ -1469,8 +1469,8 @@ int launch_ek_m(FastArgs &fa, int batch, cudaStream_t st) {
       smem = fast_smem_bytes(EK, NTC, 4 * TfGeo<64>::KS_tot, CS);
     }
   }
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (fast form)");
+  static KernelSetup setup[2];  // of the kernel and of the third-fold kernel
+  if (int rc = setup[kern != fast_kernel<EK, KSC, NTC, ADJ, CS>].opt_in(reinterpret_cast<const void *>(kern), smem)) return rc;
   const int64_t tiles = (fa.np + 7) / 8;
   if (tiles > 0x7fffffff) return set_error(SFNL_ERR_UNSUPPORTED, "np too large");
   dim3 grid((unsigned)tiles, (unsigned)batch);
@@ -1483,11 +1483,9 @@ template <int EK, int KSC, int ADJ>
 int launch_solo(FastArgs &fa, int batch, cudaStream_t st) {
   constexpr size_t smem = solo_smem_bytes(EK, KSC);
   auto kern = solo_kernel<EK, KSC, ADJ>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (fast form)");
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kSoloWarps, smem) != cudaSuccess || per_sm < 1)
-    return set_error(SFNL_ERR_CUDA, "fast form: no resident CTA");
+  static KernelSetup setup;
+  const int per_sm = setup.resident(reinterpret_cast<const void *>(kern), 32 * kSoloWarps, smem);
+  if (per_sm < 0) return per_sm;
   const int64_t ctas = ((fa.np + 7) / 8 + kSoloWarps - 1) / kSoloWarps, cap = (int64_t)num_sms() * per_sm;
   kern<<<dim3((unsigned)(ctas < cap ? ctas : cap), (unsigned)batch), 32 * kSoloWarps, smem, st>>>(fa);
   return check_launch("fast form");
@@ -1638,8 +1636,8 @@ int launch_gauss_general_m(FastArgs &fa, int64_t ng, cudaStream_t st) {
   const int tiles_per_pass = fa.NT < 8 ? fa.NT : 8;
   const int nw = CS ? 2 * tiles_per_pass : (tiles_per_pass < 2 ? 2 : tiles_per_pass);
   auto kern = fast_kernel<EK, KSC, NTC, 0, CS, GK>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (fused Gauss-point product)");
+  static KernelSetup setup;
+  if (int rc = setup.opt_in(reinterpret_cast<const void *>(kern), smem)) return rc;
   const int64_t tiles = (ng + 7) / 8;
   if (tiles > 0x7fffffff) return set_error(SFNL_ERR_UNSUPPORTED, "np too large");
   kern<<<(unsigned)tiles, nw * 32, smem, st>>>(fa);
@@ -1740,8 +1738,8 @@ int launch_gauss_advect_fused(const GaussArgs &ga, bool conservative, double *ou
   const size_t smem = xs > ovl ? xs : ovl;
   auto kern = conservative ? gauss_tf_advect_kernel<M, true> : gauss_tf_advect_kernel<M, false>;
   // opt in whatever the size: the kernel's static shared memory counts against the 48 KB default too
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (fused Gauss-point advection)");
+  static KernelSetup setup[2];
+  if (int rc = setup[conservative].opt_in(reinterpret_cast<const void *>(kern), smem)) return rc;
   const int64_t tiles = (ng + 7) / 8;
   kern<<<(unsigned)tiles, 384, smem, st>>>(fa, ga);
   return check_launch("fused Gauss-point advection");
@@ -1770,8 +1768,8 @@ int launch_gauss_cross_fused(const GaussArgs &ga, int kind, double *out, int64_t
   const size_t smem = fast_smem_bytes(EK_CROSS, g.NT, 4 * g.KS_tot, true);
   auto kern = kind == GK_NS ? gauss_tf_cross_kernel<M, GK_NS> : gauss_tf_cross_kernel<M, GK_LORENTZ>;
   if (kind != GK_NS && kind != GK_LORENTZ) return set_error(SFNL_ERR_ARG, "fused Gauss-point cross product: curl callers only");
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)  // static smem too
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (fused Gauss-point cross product)");
+  static KernelSetup setup[2];  // whatever the size: the kernel's static shared memory counts against 48 KB too
+  if (int rc = setup[kind == GK_NS].opt_in(reinterpret_cast<const void *>(kern), smem)) return rc;
   const int64_t tiles = (ng + 7) / 8;
   kern<<<(unsigned)tiles, 384, smem, st>>>(fa, ga);
   return check_launch("fused Gauss-point cross product");

@@ -237,12 +237,10 @@ int launch_mirror_pw(const ProgArgs &a, const MirrorGeo &g, cudaStream_t st) {
     if ((reinterpret_cast<uintptr_t>(a.in[f]) & 15) || (a.in_ldm[f] & 1) || (a.in_bs[f] & 1)) vec16 = 0;
   const size_t smem = mirror_smem<OP, PW>(g);
   auto kern = mirror_kernel<OP, PW>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (grid form)");
   const int nw = mirror_warps(g.PT / PW * g.NT, 2 * NI * g.KS, g.PT / PW * 2 * ((g.m + 7) / 8), 2 * op_nout(OP) * g.NT);
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nw * 32, smem) != cudaSuccess || per_sm < 1)
-    return set_error(SFNL_ERR_CUDA, "grid form: no resident CTA");
+  static KernelSetup setup;
+  const int per_sm = setup.resident(reinterpret_cast<const void *>(kern), nw * 32, smem);
+  if (per_sm < 0) return per_sm;
   const int64_t tiles = (a.np + 8 * g.PT - 1) / (8 * g.PT), cap = (int64_t)num_sms() * per_sm;
   kern<<<dim3((unsigned)(tiles < cap ? tiles : cap), (unsigned)a.batch), nw * 32, smem, st>>>(a, g, vec16);
   return check_launch("grid form");

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <vector>
@@ -16,6 +17,21 @@ struct ProgArgs;
 int set_error(int code, const char *msg);
 // Checks cudaGetLastError() after a launch; records "<what>: <cuda error>".
 int check_launch(const char *what);
+// One-time set-up of a kernel (a static object beside its launch): the opt-in to dynamic shared memory above 48 KB
+// and the CTAs of a launch shape that an SM holds.  Both are asked of the runtime once per device and size and
+// remembered until sfnl_finalize(): asked again on every launch they were a third of the host's time of a small call
+// (about 1.5 of 4.7 us).
+class KernelSetup {
+ public:
+  int opt_in(const void *kern, size_t smem);                 // SFNL_OK or SFNL_ERR_CUDA
+  int resident(const void *kern, int threads, size_t smem);  // CTAs per SM (>= 1; opted in), or an error (< 0)
+  static void forget_all();
+
+ private:
+  static constexpr int kDevs = 64;
+  std::atomic<uint64_t> smem_[kDevs] = {};  // epoch << 32 | largest size opted in
+  std::atomic<uint64_t> shape_[kDevs] = {};  // epoch (16 bits) | smem / 8 | threads | CTAs
+};
 // Number of SMs of the current device (cached per device).
 int num_sms();
 

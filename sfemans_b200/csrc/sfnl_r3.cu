@@ -639,8 +639,8 @@ int launch_bundle_r3(const ProgArgs &a, cudaStream_t st) {
   if (tma)
     if (int rc = wait_status_word(&ba.status)) return rc;
   auto kern = tma ? fast_bundle_r3_kernel<true> : fast_bundle_r3_kernel<false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kR3Smem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (residue-split bundle)");
+  static KernelSetup setup[2];
+  if (int rc = setup[tma].opt_in(reinterpret_cast<const void *>(kern), kR3Smem)) return rc;
   const int64_t tiles = (a.np + 7) / 8, ctas = (tiles + kR3TilesPerCta - 1) / kR3TilesPerCta;
   if (ctas > 0x7fffffff) return set_error(SFNL_ERR_UNSUPPORTED, "np too large");
   kern<<<(unsigned)ctas, 384, kR3Smem, st>>>(ba);

@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(kThreads, 3) prod_kernel(const ProdArgs a) {
 
 template <int OP>
 int launch_prod(const ProdArgs &pa, int R, cudaStream_t st) {
-  if (cudaFuncSetAttribute(prod_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (residue grids)");
+  static KernelSetup setup;
+  if (int rc = setup.opt_in(reinterpret_cast<const void *>(prod_kernel<OP>), kSmem)) return rc;
   prod_kernel<OP><<<dim3((unsigned)(pa.tiles * pa.nb), (unsigned)R), kThreads, kSmem, st>>>(pa);
   return check_launch("residue grids: program");
 }
@@ -492,8 +492,8 @@ int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st) {
   double *W = nullptr;
   if (int rc = large_workspace(st, (size_t)chunk * (shared_b + kb * entry_b), &W, 2)) return rc;
   const bool adj_out = op_adjoint_out(a.op);
-  if (cudaFuncSetAttribute(base_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (residue grids)");
+  static KernelSetup setup;
+  if (int rc = setup.opt_in(reinterpret_cast<const void *>(base_kernel), kSmem)) return rc;
   for (int64_t c0 = 0; c0 < a.np; c0 += chunk)
     for (int b0 = 0; b0 < a.batch; b0 += (int)kb) {
       const int nb = a.batch - b0 < kb ? a.batch - b0 : (int)kb;

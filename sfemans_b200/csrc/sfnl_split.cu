@@ -864,8 +864,8 @@ int launch_split_pr(SplitArgs &sa, int batch, const ProgArgs &pa, const int *in_
                     cudaStream_t st) {
   constexpr int NI = pr_nin(PR), NO = pr_nout(PR), PTS = pr_pts(PR);
   auto kern = split_kernel<PR, KEB>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sa.g.smem_bytes) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (split form)");
+  static KernelSetup setup;
+  if (int rc = setup.opt_in(reinterpret_cast<const void *>(kern), sa.g.smem_bytes)) return rc;
   const int64_t ntiles = (sa.np + PTS - 1) / PTS;
   // resident CTAs: by TMEM columns, shared memory and the kernel's launch bounds (the occupancy query answers 1 for
   // kernels that allocate TMEM)

@@ -195,12 +195,10 @@ int launch_mirror_synth(const double *v, double *out, double *vmax, int64_t np, 
   while (g.PT < 8 && g.PT * g.NT < 8 && bytes(2 * g.PT) <= 100 * 1024) g.PT *= 2;
   const size_t smem = bytes(g.PT);
   auto kern = mirror_synth_kernel<MODE, NI>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (synthesis)");
   const int nw = mirror_warps(g.PT * g.NT, 1, 0, 0);
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nw * 32, smem) != cudaSuccess || per_sm < 1)
-    return set_error(SFNL_ERR_CUDA, "synthesis: no resident CTA");
+  static KernelSetup setup;
+  const int per_sm = setup.resident(reinterpret_cast<const void *>(kern), nw * 32, smem);
+  if (per_sm < 0) return per_sm;
   const int vec16 = !(np & 1) && !(reinterpret_cast<uintptr_t>(v) & 15);
   const int64_t tiles = (np + 8 * g.PT - 1) / (8 * g.PT), cap = (int64_t)num_sms() * per_sm;
   kern<<<dim3((unsigned)(tiles < cap ? tiles : cap), (unsigned)groups), nw * 32, smem, st>>>(
