@@ -214,7 +214,7 @@ struct FastArgs {
   unsigned adj_in;  // bit f: input field f is a cotangent (synthesise with D)
   int adj_out;      // 1: analyse without D (transpose of the synthesis)
   int accumulate;   // 1: out += result
-  int vec16;        // 1: every input row starts 16-byte aligned (bases aligned, np even): 16-byte copies
+  int vec16;        // rows that start 16-byte aligned (16-byte copies): bit 0 the cosine rows, bit 1 the sine rows
   int allow_tf;     // 1: the third-fold kernel may be used (it allocates its own cached tables)
   const double *syn, *ana;
   GaussArgs ga;     // the Gauss-point staging of fast_kernel<..., GK >= 0>: node-major nodal fields (stride m)
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
     }
   } else {
     const int pc = 2 * (threadIdx.x & 3), rstep = blockDim.x >> 2;
-    const bool v16 = a.vec16 && p0 + 8 <= a.np;
+    const int v16 = p0 + 8 <= a.np ? a.vec16 : 0;
     const bool pv0 = p0 + pc < a.np, pv1 = p0 + pc + 1 < a.np;
     if constexpr (CT) {
       // rows outermost: the row's class, mode and sine offset are decoded once for the NI fields
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
         for (int f = 0; f < NI; ++f) {
           double *dst = dst0 + (size_t)f * KS_tot * 32;
           const double *src = a.in[f] + (int64_t)b * a.in_bs[f] + off + (int64_t)n * a.in_ldm[f];
-          if (live && v16) {
+          if (live && ((v16 >> (c >= 2)) & 1)) {
             cp_async16(dst, src);
           } else {
             if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
           double *dst = xf + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
           const bool live = k < sel4(KE, c) && !(c == 2 && n == 0);  // the sine of mode 0 is ignored
           const double *src = base + (int64_t)n * ldm + (c >= 2 ? a.np : 0);
-          if (live && v16) {
+          if (live && ((v16 >> (c >= 2)) & 1)) {
             cp_async16(dst, src);
           } else {
             if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(32 * kSoloWarps, EKDef<EK>::NI <= 2 ? 4 : 3) s
   __syncwarp();
   auto stage = [&](double *dst0, int64_t tile) {
     const int64_t p = tile * 8 + pc;
-    const bool v16 = a.vec16 && p + 1 < a.np;
+    const int v16 = p + 1 < a.np ? a.vec16 : 0;
 #pragma unroll
     for (int rg = 0; rg < RG; ++rg) {
       if (soff[rg] < 0) continue;
@@ -764,7 +764,7 @@ __global__ void __launch_bounds__(32 * kSoloWarps, EKDef<EK>::NI <= 2 ? 4 : 3) s
 #pragma unroll
       for (int f = 0; f < NI; ++f, dst += KS_tot * 32) {
         const double *src = a.in[f] + (int64_t)b * a.in_bs[f] + p + soff[rg] + (int64_t)mode[rg] * a.in_ldm[f];
-        if (v16) {
+        if ((v16 >> (rg >= KSC)) & 1) {  // the sine classes are the second half of the rows
           cp_async16(dst, src);
         } else {
           if (p < a.np) cp_async8(dst, src); else dst[0] = 0.0;
@@ -896,11 +896,11 @@ struct FieldSet {  // NG scalar fields: cos of mode n, point p at p[f][p + n*ldm
 // CE0, CE2, CO, SE0, SE2, SO) with cp.async and commits one group.  Four consecutive threads copy one
 // row (two points each, one 16-byte copy when the row is 16-byte aligned).  The modes from m on are zero.
 template <int M, int NG>
-__device__ __forceinline__ void tf_stage(double *xs, const FieldSet<NG> &fs, int64_t p0, int64_t np, bool vec16,
+__device__ __forceinline__ void tf_stage(double *xs, const FieldSet<NG> &fs, int64_t p0, int64_t np, int vec16,
                                          int m = M) {
   constexpr int KS_tot = TfGeo<M>::KS_tot, KT = TfGeo<M>::KT;
   const int pc = 2 * (threadIdx.x & 3), rstep = blockDim.x >> 2;
-  const bool v16 = vec16 && p0 + 8 <= np;
+  const int v16 = p0 + 8 <= np ? vec16 : 0;
   const bool pv0 = p0 + pc < np, pv1 = p0 + pc + 1 < np;
   // rows outermost: the row's group, mode and sine offset are decoded once for the NG fields
   for (int r = threadIdx.x >> 2; r < KT; r += rstep) {
@@ -917,7 +917,7 @@ __device__ __forceinline__ void tf_stage(double *xs, const FieldSet<NG> &fs, int
     for (int f = 0; f < NG; ++f) {
       double *dst = dst0 + (size_t)f * KS_tot * 32;
       const double *src = fs.p[f] + off + (int64_t)n * fs.ldm[f];
-      if (live && v16) {
+      if (live && ((v16 >> (gr >= 3)) & 1)) {
         cp_async16(dst, src);
       } else {
         if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
@@ -1392,11 +1392,11 @@ __global__ void __launch_bounds__(384, 2) fast_bundle_tf_kernel(const BundleArgs
     double acc_e[3][2], acc_o[3][2];
     tf_synth<M, 3, 0u>(xs, a.syn, acc_e, acc_o);
     __syncthreads();  // xs is read
-    if (next_first >= 0) tf_stage<M, 3>(xs, fields(next_first), p0, a.np, a.vec16 != 0);
+    if (next_first >= 0) tf_stage<M, 3>(xs, fields(next_first), p0, a.np, a.vec16);
     tf_fold<M, 3>(acc_e, acc_o, xc, v);
   };
   double vu[4][3], vb[4][3], vx[4][3];
-  tf_stage<M, 3>(xs, fields(0), p0, a.np, a.vec16 != 0);  // u
+  tf_stage<M, 3>(xs, fields(0), p0, a.np, a.vec16);  // u
   operand(3, vu);                                        // u; next w
   operand(12, vx);                                       // w; next gradT
   {
@@ -1539,13 +1539,12 @@ int launch_ek(FastArgs &fa, int batch, cudaStream_t st) {
 }  // namespace
 
 namespace {
-// 16-byte copies of whole rows need every row start 16-byte aligned: field bases, the sine offset np,
-// the mode stride and the batch stride all multiples of two doubles.
+// 16-byte copies of whole rows need the row start 16-byte aligned: field bases, mode stride and batch stride multiples
+// of two doubles for the cosine rows, and np too, the offset of the sine rows.
 int rows_aligned16(const FastArgs &fa, int ni) {
-  if (fa.np & 1) return 0;
   for (int i = 0; i < ni; ++i)
     if ((reinterpret_cast<uintptr_t>(fa.in[i]) & 15) || (fa.in_ldm[i] & 1) || (fa.in_bs[i] & 1)) return 0;
-  return 1;
+  return rows16(fa.np);
 }
 }  // namespace
 
@@ -1789,7 +1788,7 @@ int launch_bundle_tf(const ProgArgs &a, cudaStream_t st) {
   constexpr int M = 64;
   BundleArgs ba;
   std::memset(&ba, 0, sizeof(ba));
-  int v16 = (a.np & 1) ? 0 : 1;
+  int v16 = rows16(a.np);
   for (int f = 0; f < 15; ++f) {
     ba.in[f] = a.in[f];
     ba.in_ldm[f] = a.in_ldm[f];

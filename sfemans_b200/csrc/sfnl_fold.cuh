@@ -79,6 +79,9 @@ __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
                "l"(gsrc)
                : "memory");
 }
+// Which rows of aligned arrays start 16-byte aligned: bit 0 the cosine rows, bit 1 the sine rows, np doubles further
+// (with an odd np the 8-byte copies of every row cost a third of the m = 64 cross product's time).
+constexpr int rows16(int64_t np) { return np & 1 ? 1 : 3; }
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }

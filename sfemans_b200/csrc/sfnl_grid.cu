@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256, op_nin(OP) <= 6 ? 2 : 1) mirror_kernel(co
   auto in = [&](int f) { return a.in[f] + (int64_t)b * a.in_bs[f]; };
   auto ldm = [&](int f) { return a.in_ldm[f]; };
   const int64_t tiles = (a.np + 8 * g.PT - 1) / (8 * g.PT);
-  mirror_stage<NI>(xs, g, in, ldm, (int64_t)blockIdx.x * 8 * g.PT, a.np, vec16 != 0);
+  mirror_stage<NI>(xs, g, in, ldm, (int64_t)blockIdx.x * 8 * g.PT, a.np, vec16);
   mirror_table(ctab, stab, g.N);
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t p0 = tile * 8 * g.PT;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256, op_nin(OP) <= 6 ? 2 : 1) mirror_kernel(co
     }
     __syncthreads();
     if (tile + gridDim.x < tiles)
-      mirror_stage<NI>(xs, g, in, ldm, (tile + gridDim.x) * 8 * g.PT, a.np, vec16 != 0);
+      mirror_stage<NI>(xs, g, in, ldm, (tile + gridDim.x) * 8 * g.PT, a.np, vec16);
     for (int it = warp; it < PG * 2 * NU; it += NW) {
       const int u = it % NU, c = (it / NU) & 1, pg = it / (2 * NU);
       constexpr int PC = NO * PW >= 9 ? 1 : 2;  // independent partial sums per output
@@ -232,7 +232,7 @@ size_t mirror_smem(const MirrorGeo &g) {
 template <int OP, int PW>
 int launch_mirror_pw(const ProgArgs &a, const MirrorGeo &g, cudaStream_t st) {
   constexpr int NI = op_nin(OP);
-  int vec16 = (a.np & 1) ? 0 : 1;
+  int vec16 = rows16(a.np);
   for (int f = 0; f < NI; ++f)
     if ((reinterpret_cast<uintptr_t>(a.in[f]) & 15) || (a.in_ldm[f] & 1) || (a.in_bs[f] & 1)) vec16 = 0;
   const size_t smem = mirror_smem<OP, PW>(g);

@@ -58,11 +58,11 @@ __device__ __forceinline__ void mirror_table(double *ctab, double *stab, int N) 
 
 // Copies the NI fields of the 8*PT points from p0 into xs with cp.async (one group, not waited for): field f's
 // cosine of mode n, point p is at in(f)[p + n*ldm(f)], its sine np further.  A thread copies two neighbouring
-// points of one row for every field; rows start 16-byte aligned when v16 (np and the strides even, bases
-// aligned).  The sine of mode 0 is ignored (fft_parallel.F90:241); points past np are zero.
+// points of one row for every field; v16: the rows that start 16-byte aligned (rows16).  The sine of mode 0 is
+// ignored (fft_parallel.F90:241); points past np are zero.
 template <int NI, typename In, typename Ldm>
 __device__ __forceinline__ void mirror_stage(double *xs, const MirrorGeo &g, In in, Ldm ldm, int64_t p0, int64_t np,
-                                             bool v16) {
+                                             int v16) {
   const int pairs = 4 * g.PT, rows = 8 * g.KS;  // rows: (mode, cos/sin)
   for (int i = threadIdx.x; i < pairs * rows; i += blockDim.x) {
     const int pr = i % pairs, row = i / pairs, c = row & 1, n = row >> 1;
@@ -73,7 +73,7 @@ __device__ __forceinline__ void mirror_stage(double *xs, const MirrorGeo &g, In 
 #pragma unroll
     for (int f = 0; f < NI; ++f, dst += (size_t)g.KS * 64) {
       const double *src = in(f) + p + (int64_t)n * ldm(f) + (c ? np : 0);
-      if (l1 && v16) {
+      if (l1 && ((v16 >> c) & 1)) {
         cp_async16(dst, src);
       } else {
         if (l0) cp_async8(dst, src); else dst[0] = 0.0;

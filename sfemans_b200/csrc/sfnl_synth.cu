@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
   auto in = [&](int f) { return v + (int64_t)2 * (f0 + f) * np; };
   auto ldm = [&](int) { return (int64_t)nslot * np; };
   const int64_t tiles = (np + pts - 1) / pts;
-  mirror_stage<NI>(xs, g, in, ldm, (int64_t)blockIdx.x * pts, np, vec16 != 0);
+  mirror_stage<NI>(xs, g, in, ldm, (int64_t)blockIdx.x * pts, np, vec16);
   mirror_table(ctab, stab, N);
   double vm = 0.0;
   int buf = 0;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
     cp_async_wait_0();
     __syncthreads();
     if (tile + gridDim.x < tiles)
-      mirror_stage<NI>(xs + (buf ^ 1) * xsz, g, in, ldm, (tile + gridDim.x) * pts, np, vec16 != 0);
+      mirror_stage<NI>(xs + (buf ^ 1) * xsz, g, in, ldm, (tile + gridDim.x) * pts, np, vec16);
     for (int it = warp; it < g.PT * g.NT; it += NW) {
       const int t = it % g.NT, pt = it / g.NT;
       double acc[1][NI][2][2];
@@ -199,7 +199,7 @@ int launch_mirror_synth(const double *v, double *out, double *vmax, int64_t np, 
   static KernelSetup setup;
   const int per_sm = setup.resident(reinterpret_cast<const void *>(kern), nw * 32, smem);
   if (per_sm < 0) return per_sm;
-  const int vec16 = !(np & 1) && !(reinterpret_cast<uintptr_t>(v) & 15);
+  const int vec16 = (reinterpret_cast<uintptr_t>(v) & 15) || (nslot & 1) ? 0 : rows16(np);
   const int64_t tiles = (np + 8 * g.PT - 1) / (8 * g.PT), cap = (int64_t)num_sms() * per_sm;
   kern<<<dim3((unsigned)(tiles < cap ? tiles : cap), (unsigned)groups), nw * 32, smem, st>>>(
       v, out, reinterpret_cast<unsigned long long *>(vmax), np, nslot, g, vec16);
