@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kSynthThreads) synth_kernel(const double *v, d
 // evaluated.  Measured on a B200 against one warp per point (synth_kernel): grid values of a 3-vector at 28,000
 // points and m = 64 0.48 -> 0.072 ms, the maximum at 56,000 points and m = 32 (with its copy to the host)
 // 0.411 -> 0.089 ms.
-template <int MODE, int NI>
+template <int MODE, int NI, int PW>
 __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, double *out, unsigned long long *vmax,
                                                               int64_t np, int nslot, const MirrorGeo g,
                                                               const int vec16) {
@@ -130,10 +130,13 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
     __syncthreads();
     if (tile + gridDim.x < tiles)
       mirror_stage<NI>(xs + (buf ^ 1) * xsz, g, in, ldm, (tile + gridDim.x) * pts, np, vec16);
-    for (int it = warp; it < g.PT * g.NT; it += NW) {
-      const int t = it % g.NT, pt = it / g.NT;
-      double acc[1][NI][2][2];
-      mirror_synth<NI, 1, 0>(xs + buf * xsz + (size_t)pt * NI * g.KS * 64, ctab, stab, g, t, acc);
+    for (int it = warp; it < g.PT / PW * g.NT; it += NW) {
+      const int t = it % g.NT, pg = it / g.NT;
+      double acc[PW][NI][2][2];
+      mirror_synth<NI, PW, 0>(xs + buf * xsz + (size_t)pg * PW * NI * g.KS * 64, ctab, stab, g, t, acc);
+#pragma unroll
+      for (int w = 0; w < PW; ++w) {
+      const int pt = pg * PW + w;
       double pv = 0.0;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
@@ -142,7 +145,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
         double sp = 0.0, sm = 0.0;
 #pragma unroll
         for (int f = 0; f < NI; ++f) {
-          const double fp = acc[0][f][0][e] + acc[0][f][1][e], fm = acc[0][f][0][e] - acc[0][f][1][e];
+          const double fp = acc[w][f][0][e] + acc[w][f][1][e], fm = acc[w][f][0][e] - acc[w][f][1][e];
           if constexpr (MODE == 0) {
             double *o = os + ((size_t)(8 * pt + gg) * NI + f) * N;
             o[j] = fp;
@@ -157,6 +160,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
       if constexpr (MODE == 2) {
         for (int off = 2; off > 0; off >>= 1) pv = fmax(pv, __shfl_xor_sync(0xffffffffu, pv, off));
         if (q == 0) atomicMax(pm + 8 * pt + gg, (unsigned long long)__double_as_longlong(pv));
+      }
       }
     }
     if constexpr (MODE != 1) {
@@ -183,19 +187,23 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
 }
 
 // SFNL_OK / an error of the launch, or 1 when the tile does not fit in shared memory.
-template <int MODE, int NI>
+template <int MODE, int NI, int PW>
 int launch_mirror_synth(const double *v, double *out, double *vmax, int64_t np, int nslot, int m, int N, int groups,
                         cudaStream_t st) {
-  MirrorGeo g = mirror_geo(m, N, 1);
+  MirrorGeo g = mirror_geo(m, N, PW);
   auto bytes = [&](int pt) {
     const size_t per = 2 * (size_t)NI * g.KS * 64 + (MODE == 0 ? (size_t)8 * NI * N : MODE == 2 ? 8 : 0);
     return sizeof(double) * ((size_t)pt * per + 2 * (size_t)N);
   };
-  if (bytes(1) > 200 * 1024) return 1;
-  while (g.PT < 8 && g.PT * g.NT < 8 && bytes(2 * g.PT) <= 100 * 1024) g.PT *= 2;
+  if constexpr (PW == 2) {
+    // two point tiles share each table entry where two CTAs of such tiles fit on an SM
+    if (bytes(2) > 100 * 1024) return launch_mirror_synth<MODE, NI, 1>(v, out, vmax, np, nslot, m, N, groups, st);
+  }
+  if (bytes(PW) > 200 * 1024) return 1;
+  while (g.PT < 8 && g.PT / PW * g.NT < 8 && bytes(2 * g.PT) <= 100 * 1024) g.PT *= 2;
   const size_t smem = bytes(g.PT);
-  auto kern = mirror_synth_kernel<MODE, NI>;
-  const int nw = mirror_warps(g.PT * g.NT, 1, 0, 0);
+  auto kern = mirror_synth_kernel<MODE, NI, PW>;
+  const int nw = mirror_warps(g.PT / PW * g.NT, 1, 0, 0);
   static KernelSetup setup;
   const int per_sm = setup.resident(reinterpret_cast<const void *>(kern), nw * 32, smem);
   if (per_sm < 0) return per_sm;
@@ -211,11 +219,11 @@ int launch_synth(const double *v, double *out, double *vmax, int64_t np, int nsl
   // the fields that are evaluated, three at a time where they come in threes
   const int nfe = MODE == 0 ? nslot / 2 : nslot == 6 ? 3 : 1;
   if (nfe / 3 <= 65535 && nfe % 3 == 0) {
-    if (const int rc = launch_mirror_synth<MODE, 3>(v, out, vmax, np, nslot, m, N, nfe / 3, st); rc <= 0) return rc;
+    if (const int rc = launch_mirror_synth<MODE, 3, 2>(v, out, vmax, np, nslot, m, N, nfe / 3, st); rc <= 0) return rc;
   }
   if (nfe <= 65535) {
     if (MODE == 0 || nfe == 1)
-      if (const int rc = launch_mirror_synth<MODE, 1>(v, out, vmax, np, nslot, m, N, nfe, st); rc <= 0) return rc;
+      if (const int rc = launch_mirror_synth<MODE, 1, 2>(v, out, vmax, np, nslot, m, N, nfe, st); rc <= 0) return rc;
   }
   const size_t tab_bytes = sizeof(double) * 2 * (size_t)N, per_warp = sizeof(double) * (size_t)nslot * m;
   const size_t budget = 200 * 1024;
