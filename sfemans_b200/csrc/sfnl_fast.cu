@@ -439,12 +439,13 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
         const int k = r - 4 * sel4(KOFF, c), n = class_mode(c, k);
         double *dst0 = xs + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
         const bool live = k < sel4(KE, c) && !(c == 2 && n == 0);  // the sine of mode 0 is ignored
+        const bool wide = live && ((v16 >> (c >= 2)) & 1);
         const int64_t off = p0 + pc + (c >= 2 ? a.np : 0);
 #pragma unroll
         for (int f = 0; f < NI; ++f) {
           double *dst = dst0 + (size_t)f * KS_tot * 32;
           const double *src = a.in[f] + (int64_t)b * a.in_bs[f] + off + (int64_t)n * a.in_ldm[f];
-          if (live && ((v16 >> (c >= 2)) & 1)) {
+          if (wide) {
             cp_async16(dst, src);
           } else {
             if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
@@ -912,12 +913,13 @@ __device__ __forceinline__ void tf_stage(double *xs, const FieldSet<NG> &fs, int
     const int k = r - 4 * kg, n = tf_mode(gr, k);
     double *dst0 = xs + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
     const bool live = k < keg && n < m && !(gr == 3 && k == 0);  // the sine of mode 0 is ignored
+    const bool wide = live && ((v16 >> (gr >= 3)) & 1);
     const int64_t off = p0 + pc + (gr >= 3 ? np : 0);
 #pragma unroll
     for (int f = 0; f < NG; ++f) {
       double *dst = dst0 + (size_t)f * KS_tot * 32;
       const double *src = fs.p[f] + off + (int64_t)n * fs.ldm[f];
-      if (live && ((v16 >> (gr >= 3)) & 1)) {
+      if (wide) {
         cp_async16(dst, src);
       } else {
         if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
