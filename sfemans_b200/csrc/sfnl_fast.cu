@@ -728,7 +728,7 @@ constexpr int solo_max_ks(int ek) { return ek_nout(ek) == 1 ? 4 : 2; }
 constexpr bool solo_ek(int ek) { return ek == EK_CROSS || ek == EK_DOT || ek == EK_PROD || ek == EK_SVECT; }
 constexpr size_t solo_smem_bytes(int ek, int KSC) { return sizeof(double) * (size_t)kSoloWarps * ek_nin(ek) * 4 * KSC * 32; }
 
-template <int EK, int KSC, int ADJ>
+template <int EK, int KSC>
 __global__ void __launch_bounds__(32 * kSoloWarps, EKDef<EK>::NI <= 2 ? 4 : 3) solo_kernel(const FastArgs a) {
   constexpr int NI = EKDef<EK>::NI, NO = EKDef<EK>::NO;
   constexpr int NUC = (KSC + 1) / 2, KS_tot = 4 * KSC, bufd = NI * KS_tot * 32;
@@ -737,7 +737,6 @@ __global__ void __launch_bounds__(32 * kSoloWarps, EKDef<EK>::NI <= 2 ? 4 : 3) s
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, q = lane & 3, b = blockIdx.y;
   const int NT = a.NT;
-  const double invN = 1.0 / (4.0 * 8.0 * NT), twoN = 2.0 * invN;
   double *buf = smem + (size_t)warp * bufd;
 
   // Staging: lane l copies points 2 (l & 3), 2 (l & 3) + 1 of row 8 rg + (l >> 2) of every field (rows as in
@@ -807,9 +806,7 @@ __global__ void __launch_bounds__(32 * kSoloWarps, EKDef<EK>::NI <= 2 ? 4 : 3) s
           const double bv = __ldg(syn_t + (size_t)kt * NT * 32);
 #pragma unroll
           for (int f = 0; f < NI; ++f) {
-            double av = xs[(f * KS_tot + ks) * 32];
-            if ((ADJ == 1 && f < 3) || (ADJ == 2 && f >= 3)) av *= (s == 0 && q == 0 && (c & 1) == 0) ? invN : twoN;
-            dmma(acc[f][c], av, bv);
+            dmma(acc[f][c], xs[(f * KS_tot + ks) * 32], bv);
           }
         }
       if (t == NT - 1 && tile + step < tiles) {  // the coefficients are read: the next tile's may arrive
@@ -873,6 +870,295 @@ __global__ void __launch_bounds__(32 * kSoloWarps, EKDef<EK>::NI <= 2 ? 4 : 3) s
               *dst = r;
           }
         }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// programs of several operands in one launch (m <= 64)
+// ---------------------------------------------------------------------------
+// The transposed cross product, the linearised MHD pair and the MHD bundle share operands between their products.  As
+// sequences of elementary programs each product synthesises both its operands again: 33 transforms of a field for the
+// MHD VJP, 30 for its JVP, 34 for the bundle, 18 for the cross product's VJP.  Here a CTA takes the operands (three
+// fields) one after the other, keeps the quadrant values that later products need in registers (or, u of the MHD
+// programs, in the thread's own part of shared memory), and adds products with a common output before the one
+// analysis: 24, 24, 25 and 15 transforms, every input read and every output written once.  One warp per angle tile
+// with the four classes of three fields (24 accumulator pairs); the next operand is copied while the current one is
+// folded and analysed.  Measured on a B200 against the sequences of launches: cross product's VJP, 175,000 points,
+// m = 32 0.528 -> 0.461 ms; MHD VJP, 30,000 points, 4 cotangents, m = 32 0.740 -> 0.540 ms, m = 16 0.303 -> 0.243 (the
+// launches were the one-warp kernel's); MHD JVP the same, m = 32 0.629 -> 0.531; bundle, 100,000 points, m = 32
+// 0.599 -> 0.446, m = 16 0.261 -> 0.187 ms; MHD pair, 2 tangents, 30,000 points, m = 64 (third-fold launches)
+// 1.03 -> 0.84 ms.
+struct ChainArgs {
+  const double *in[kMaxIn];
+  double *out[kMaxOut];
+  int64_t in_ldm[kMaxIn], out_ldm[kMaxOut], in_bs[kMaxIn], out_bs[kMaxOut];
+  int64_t np;
+  int m, vec16, ke[4];
+  const double *syn, *ana;
+};
+constexpr bool chain_op(int op) { return op == OP_CROSS_VJP || op == OP_MHD_JVP || op == OP_MHD_VJP || op == OP_BUNDLE; }
+constexpr bool chain_keeps_u(int op) { return op == OP_MHD_JVP || op == OP_MHD_VJP; }
+constexpr size_t chain_smem(int op, int KSC, int NTC) {
+  return sizeof(double) * ((size_t)3 * 4 * KSC * 32 + 3 * 4 * NTC * 64 + (chain_keeps_u(op) ? 24 * 32 * NTC : 0));
+}
+constexpr int chain_blocks(int op, int KSC, int NTC) {  // CTAs per SM at 128 registers and by shared memory
+  const int r = 512 / (32 * NTC), s = (int)((size_t)220 * 1024 / (chain_smem(op, KSC, NTC) + 1024));
+  return r < s ? r : s;
+}
+
+template <int OP, int KSC, int NTC>
+__global__ void __launch_bounds__(32 * NTC, chain_blocks(OP, KSC, NTC)) chain_kernel(const ChainArgs a) {
+  constexpr int KS_tot = 4 * KSC, NUC = (KSC + 1) / 2, NU_tot = 4 * NUC;
+  extern __shared__ __align__(16) double smem[];
+  double *xs = smem, *ps = xs + 3 * KS_tot * 32;                      // staged operand, folded products
+  double *us = ps + 3 * 4 * NTC * 64 + threadIdx.x;                   // u's quadrant values of this thread
+  const int lane = threadIdx.x & 31, t = threadIdx.x >> 5, g = lane >> 2, q = lane & 3, b = blockIdx.y;
+  const int64_t p0 = (int64_t)blockIdx.x * 8;
+  const double invN = 1.0 / (32.0 * NTC), twoN = 2.0 * invN;
+
+  auto stage = [&](int f0) {
+    const int pc = 2 * (threadIdx.x & 3);
+    const int v16 = p0 + 8 <= a.np ? a.vec16 : 0;
+    const bool pv0 = p0 + pc < a.np, pv1 = p0 + pc + 1 < a.np;
+    for (int r = threadIdx.x >> 2; r < 4 * KS_tot; r += 8 * NTC) {
+      const int c = r / (4 * KSC), k = r - 4 * KSC * c, n = class_mode(c, k);
+      const bool live = k < sel4(a.ke, c) && !(c == 2 && n == 0);  // the sine of mode 0 is ignored
+      const bool wide = live && ((v16 >> (c >= 2)) & 1);
+      double *dst = xs + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
+      const int64_t off = p0 + pc + (c >= 2 ? a.np : 0);
+#pragma unroll
+      for (int f = 0; f < 3; ++f, dst += KS_tot * 32) {
+        const double *src = a.in[f0 + f] + (int64_t)b * a.in_bs[f0 + f] + off + (int64_t)n * a.in_ldm[f0 + f];
+        if (wide) {
+          cp_async16(dst, src);
+        } else {
+          if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
+          if (live && pv1) cp_async8(dst + 1, src + 1); else dst[1] = 0.0;
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  using Acc = double[3][4][2];
+  using Val = double[2][4][3];  // [parity e][quadrant][component]
+  // Class sums of the staged operand (cot: a cotangent, synthesised with the analysis weights), then the copies of the
+  // operand at field `next` (< 0: none).
+  auto synth = [&](bool cot, int next, Acc &acc) {
+    cp_async_wait_0();
+    __syncthreads();
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[f][c][0] = acc[f][c][1] = 0.0;
+    const double *syn_t = a.syn + (size_t)t * 32 + lane, *xl = xs + a_frag_slot(q, g);
+#pragma unroll
+    for (int s = 0; s < KSC; ++s)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int ks = c * KSC + s;
+        double bv = __ldg(syn_t + (size_t)ks * NTC * 32);
+        double av[3];
+#pragma unroll
+        for (int f = 0; f < 3; ++f) av[f] = xl[(f * KS_tot + ks) * 32];
+        if (cot) {
+          const double wn = (s == 0 && q == 0 && (c & 1) == 0) ? invN : twoN;  // n == 0 only there
+#pragma unroll
+          for (int f = 0; f < 3; ++f) av[f] *= wn;
+        }
+#pragma unroll
+        for (int f = 0; f < 3; ++f) dmma(acc[f][c], av[f], bv);
+      }
+    __syncthreads();
+    if (next >= 0) stage(next);
+  };
+  auto fold = [&](const Acc &acc, int e, double (&v)[4][3]) {
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const double A = acc[f][0][e] + acc[f][1][e], B = acc[f][0][e] - acc[f][1][e];
+      const double C = acc[f][2][e] + acc[f][3][e], D = acc[f][3][e] - acc[f][2][e];
+      v[0][f] = A + C;  // theta
+      v[1][f] = B + D;  // pi - theta
+      v[2][f] = B - D;  // pi + theta
+      v[3][f] = A - C;  // 2 pi - theta
+    }
+  };
+  auto keep = [&](const Acc &acc, Val &h) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) fold(acc, e, h[e]);
+  };
+  // Pre-folded products of parity e into (add: onto) the first NO product slots; a thread reads back only its own.
+  auto put = [&](int e, auto &gq, bool add) {
+    constexpr int NO = sizeof(gq[0]) / sizeof(double);
+#pragma unroll
+    for (int o = 0; o < NO; ++o) {
+      const double s14 = gq[0][o] + gq[3][o], d14 = gq[0][o] - gq[3][o];
+      const double s23 = gq[1][o] + gq[2][o], d32 = gq[2][o] - gq[1][o];
+      double *dst = ps + ((size_t)(o * 4) * NTC + t) * 64 + e * 32 + lane;
+      const double P[4] = {s14 + s23, s14 - s23, d14 + d32, d14 - d32};  // PE, PO, QE, QO
+#pragma unroll
+      for (int c = 0; c < 4; ++c) dst[c * NTC * 64] = add ? dst[c * NTC * 64] + P[c] : P[c];
+    }
+  };
+  // products of the current operand with the kept one: kept x current (sgn +) or current x kept (sgn -)
+  auto cross_put = [&](const Acc &acc, const Val &h, bool kept_first, bool add) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      double v[4][3], gq[4][3];
+      fold(acc, e, v);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        if (kept_first)
+          cross3(h[e][r], v[r], gq[r]);
+        else
+          cross3(v[r], h[e][r], gq[r]);
+      }
+      put(e, gq, add);
+    }
+  };
+  // u's values: to and from the thread's own slots
+  auto save_u = [&](const Acc &acc) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      double v[4][3];
+      fold(acc, e, v);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int f = 0; f < 3; ++f) us[((e * 4 + r) * 3 + f) * 32 * NTC] = v[r][f];
+    }
+  };
+  auto load_u = [&](int e, int r, double (&u)[3]) {
+#pragma unroll
+    for (int f = 0; f < 3; ++f) u[f] = us[((e * 4 + r) * 3 + f) * 32 * NTC];
+  };
+  // outputs o0 .. o0+NO-1 from the product slots
+  auto analyse = [&](auto no_tag, int o0) {
+    constexpr int NO = decltype(no_tag)::value, PC = NO == 1 ? 4 : 2;
+    __syncthreads();
+    const int64_t p = p0 + g;
+    const double *anav = a.ana + (size_t)(op_adjoint_out(OP) ? 1 : 0) * NU_tot * NTC * 64 + lane;
+    for (int cu = t; cu < NU_tot; cu += NTC) {
+      const int c = cu / NUC, u = cu - c * NUC;
+      double yp[PC][NO][2];
+#pragma unroll
+      for (int i = 0; i < PC; ++i)
+#pragma unroll
+        for (int o = 0; o < NO; ++o) yp[i][o][0] = yp[i][o][1] = 0.0;
+      const double *bt = anav + (size_t)cu * NTC * 64, *pa = ps + (size_t)c * NTC * 64 + lane;
+#pragma unroll
+      for (int te = 0; te < 2 * NTC; ++te) {
+        const double bv = __ldg(bt + te * 32);
+#pragma unroll
+        for (int o = 0; o < NO; ++o) dmma(yp[te % PC][o], pa[(o * 4 * NTC * 2 + te) * 32], bv);
+      }
+      if (p >= a.np) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int kk = 8 * u + 2 * q + h;
+        if (kk >= sel4(a.ke, c)) continue;
+        const int n = class_mode(c, kk);
+#pragma unroll
+        for (int o = 0; o < NO; ++o) {
+          double y = yp[0][o][h];
+#pragma unroll
+          for (int i = 1; i < PC; ++i) y += yp[i][o][h];
+          a.out[o0 + o][(int64_t)b * a.out_bs[o0 + o] + p + (int64_t)n * a.out_ldm[o0 + o] + (c >= 2 ? a.np : 0)] =
+              c == 2 && n == 0 ? 0.0 : y;
+        }
+      }
+    }
+  };
+  const std::integral_constant<int, 3> three;
+  Acc acc;
+  Val h;
+  if constexpr (OP == OP_CROSS_VJP) {  // [u 0, w 3, c 6] -> w x c (0), c x u (3)
+    stage(6);
+    synth(true, 0, acc);
+    keep(acc, h);
+    synth(false, 3, acc);
+    cross_put(acc, h, true, false);
+    analyse(three, 3);
+    synth(false, -1, acc);
+    cross_put(acc, h, false, false);
+    analyse(three, 0);
+  } else if constexpr (OP == OP_MHD_JVP) {  // [u 0, w 3, b 6, du 9, dw 12, db 15] -> du x w + u x dw, du x b + u x db
+    stage(0);
+    synth(false, 9, acc);
+    save_u(acc);
+    synth(false, 3, acc);
+    keep(acc, h);  // du
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+      synth(false, 12 + 3 * k, acc);  // w, b
+      cross_put(acc, h, true, false);
+      synth(false, k == 0 ? 6 : -1, acc);  // dw, db
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        double v[4][3], gq[4][3];
+        fold(acc, e, v);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          double u[3];
+          load_u(e, r, u);
+          cross3(u, v[r], gq[r]);
+        }
+        put(e, gq, true);
+      }
+      analyse(three, 3 * k);
+    }
+  } else if constexpr (OP == OP_MHD_VJP) {  // [u 0, w 3, b 6, c1 9, c2 12] -> w x c1 + b x c2 (0), c1 x u (3), c2 x u (6)
+    stage(9);
+    synth(true, 0, acc);
+    keep(acc, h);  // c1
+    synth(false, 3, acc);
+    save_u(acc);
+    cross_put(acc, h, true, false);
+    analyse(three, 3);
+    synth(false, 12, acc);
+    cross_put(acc, h, false, false);  // w x c1 waits in the product slots
+    synth(true, 6, acc);
+    keep(acc, h);  // c2
+    synth(false, -1, acc);
+    cross_put(acc, h, false, true);
+    analyse(three, 0);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      double gq[4][3];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        double u[3];
+        load_u(e, r, u);
+        cross3(h[e][r], u, gq[r]);
+      }
+      put(e, gq, false);
+    }
+    analyse(three, 6);
+  } else {  // [u 0, w 3, b 6, j 9, gradT 12] -> u x w (0), u x b (3), j x b (6), u . gradT (9)
+    static_assert(OP == OP_BUNDLE, "program");
+    stage(0);
+    synth(false, 3, acc);
+    keep(acc, h);  // u
+    synth(false, 12, acc);
+    cross_put(acc, h, true, false);
+    analyse(three, 0);
+    synth(false, 6, acc);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      double v[4][3], gq[4][1];
+      fold(acc, e, v);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) gq[r][0] = h[e][r][0] * v[r][0] + h[e][r][1] * v[r][1] + h[e][r][2] * v[r][2];
+      put(e, gq, false);
+    }
+    analyse(std::integral_constant<int, 1>{}, 9);
+    synth(false, 9, acc);
+    cross_put(acc, h, true, false);
+    keep(acc, h);  // b
+    analyse(three, 3);
+    synth(false, -1, acc);
+    cross_put(acc, h, false, false);
+    analyse(three, 6);
   }
 }
 
@@ -1481,10 +1767,10 @@ int launch_ek_m(FastArgs &fa, int batch, cudaStream_t st) {
 }
 
 // The solo kernel where every class has at most solo_max_ks(EK) k-steps.
-template <int EK, int KSC, int ADJ>
+template <int EK, int KSC>
 int launch_solo(FastArgs &fa, int batch, cudaStream_t st) {
   constexpr size_t smem = solo_smem_bytes(EK, KSC);
-  auto kern = solo_kernel<EK, KSC, ADJ>;
+  auto kern = solo_kernel<EK, KSC>;
   static KernelSetup setup;
   const int per_sm = setup.resident(reinterpret_cast<const void *>(kern), 32 * kSoloWarps, smem);
   if (per_sm < 0) return per_sm;
@@ -1495,16 +1781,21 @@ int launch_solo(FastArgs &fa, int batch, cudaStream_t st) {
 
 template <int EK, int ADJ>
 int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
-  if constexpr (solo_ek(EK)) {
-    if (fa.KS[0] == 1) return launch_solo<EK, 1, ADJ>(fa, batch, st);
-    if (fa.KS[0] == 2) return launch_solo<EK, 2, ADJ>(fa, batch, st);
+  if constexpr (solo_ek(EK) && ADJ == 0) {
+    if (fa.KS[0] == 1) return launch_solo<EK, 1>(fa, batch, st);
+    if (fa.KS[0] == 2) return launch_solo<EK, 2>(fa, batch, st);
     if constexpr (solo_max_ks(EK) == 4) {
-      if (fa.KS[0] == 3) return launch_solo<EK, 3, ADJ>(fa, batch, st);
-      if (fa.KS[0] == 4) return launch_solo<EK, 4, ADJ>(fa, batch, st);
+      if (fa.KS[0] == 3) return launch_solo<EK, 3>(fa, batch, st);
+      if (fa.KS[0] == 4) return launch_solo<EK, 4>(fa, batch, st);
     }
   }
   // every (KS, NT) of make_geo up to m = 64; run-time loops cost the sizes between 16, 32 and 64 a third of their time
   // (cross product, 50,001 points: m = 20 99 -> 62 us, m = 40 207 -> 148, m = 48 337 -> 202, m = 52 384 -> 229)
+  if constexpr (ADJ != 0) {  // transposed products: chain_kernel takes the other sizes up to m = 64
+    if (fa.NT == 6 && fa.KS[0] == 7) return launch_ek_m<EK, 7, 6, ADJ>(fa, batch, st);
+    if (fa.NT == 6 && fa.KS[0] == 8) return launch_ek_m<EK, 8, 6, ADJ>(fa, batch, st);
+    return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);
+  } else {
   switch (10 * fa.KS[0] + fa.NT) {
     case 11: return launch_ek_m<EK, 1, 1, ADJ>(fa, batch, st);
     case 21: return launch_ek_m<EK, 2, 1, ADJ>(fa, batch, st);
@@ -1519,6 +1810,7 @@ int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
     case 76: return launch_ek_m<EK, 7, 6, ADJ>(fa, batch, st);
     case 86: return launch_ek_m<EK, 8, 6, ADJ>(fa, batch, st);
     default: return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);
+  }
   }
 }
 
@@ -1818,6 +2110,62 @@ int launch_bundle_tf(const ProgArgs &a, cudaStream_t st) {
 }
 }  // namespace
 
+namespace {
+// The programs of chain_kernel to m = 64; with six angle tiles the cross product's VJP stays two launches of the
+// third-fold kernel, whose transforms have a quarter fewer DMMAs.
+template <int OP, int KSC, int NTC>
+int launch_chain(const ChainArgs &ca, int batch, cudaStream_t st) {
+  constexpr size_t smem = chain_smem(OP, KSC, NTC);
+  auto kern = chain_kernel<OP, KSC, NTC>;
+  static KernelSetup setup;
+  if (int rc = setup.opt_in(reinterpret_cast<const void *>(kern), smem)) return rc;
+  const int64_t tiles = (ca.np + 7) / 8;
+  if (tiles > 0x7fffffff) return set_error(SFNL_ERR_UNSUPPORTED, "np too large");
+  kern<<<dim3((unsigned)tiles, (unsigned)batch), 32 * NTC, smem, st>>>(ca);
+  return check_launch("fast form");
+}
+bool chain_fits(int op, int m, const Geo &g) {
+  return chain_op(op) && m <= 64 && !(op == OP_CROSS_VJP && g.NT == 6);
+}
+template <int OP>
+int launch_chain_op(const ProgArgs &a, const Geo &g, const Tables &T, cudaStream_t st) {
+  ChainArgs ca;
+  std::memset(&ca, 0, sizeof(ca));
+  ca.np = a.np;
+  ca.m = a.m;
+  ca.vec16 = rows16(a.np);
+  for (int f = 0; f < op_nin(OP); ++f) {
+    ca.in[f] = a.in[f];
+    ca.in_ldm[f] = a.in_ldm[f];
+    ca.in_bs[f] = a.in_bs[f];
+    if ((reinterpret_cast<uintptr_t>(a.in[f]) & 15) || (a.in_ldm[f] & 1) || (a.in_bs[f] & 1)) ca.vec16 = 0;
+  }
+  for (int o = 0; o < op_nout(OP); ++o) {
+    ca.out[o] = a.out[o];
+    ca.out_ldm[o] = a.out_ldm[o];
+    ca.out_bs[o] = a.out_bs[o];
+  }
+  for (int c = 0; c < 4; ++c) ca.ke[c] = g.ke[c];
+  ca.syn = T.syn;
+  ca.ana = T.ana;
+  switch (10 * g.KS[0] + g.NT) {
+    case 11: return launch_chain<OP, 1, 1>(ca, a.batch, st);
+    case 21: return launch_chain<OP, 2, 1>(ca, a.batch, st);
+    case 22: return launch_chain<OP, 2, 2>(ca, a.batch, st);
+    case 32: return launch_chain<OP, 3, 2>(ca, a.batch, st);
+    case 33: return launch_chain<OP, 3, 3>(ca, a.batch, st);
+    case 43: return launch_chain<OP, 4, 3>(ca, a.batch, st);
+    case 54: return launch_chain<OP, 5, 4>(ca, a.batch, st);
+    case 64: return launch_chain<OP, 6, 4>(ca, a.batch, st);
+    case 65: return launch_chain<OP, 6, 5>(ca, a.batch, st);
+    case 75: return launch_chain<OP, 7, 5>(ca, a.batch, st);
+    case 76: return launch_chain<OP, 7, 6>(ca, a.batch, st);
+    case 86: return launch_chain<OP, 8, 6>(ca, a.batch, st);
+  }
+  return set_error(SFNL_ERR_UNSUPPORTED, "FAST form: no such geometry");
+}
+}  // namespace
+
 int launch_fast(const ProgArgs &a, cudaStream_t st) {
   if (a.np == 0) return SFNL_OK;
   const Geo g = make_geo(a.m);
@@ -1828,17 +2176,21 @@ int launch_fast(const ProgArgs &a, cudaStream_t st) {
   int rc = get_tables(g, &T);
   if (rc) return rc;
   if (!fast_fused_fits(a.op, a.m)) return launch_fast_large(a, g, T, st);
+  if (chain_fits(a.op, a.m, g) && a.out_ps == 1) {
+    switch (a.op) {
+      case OP_CROSS_VJP: return launch_chain_op<OP_CROSS_VJP>(a, g, T, st);
+      case OP_MHD_JVP: return launch_chain_op<OP_MHD_JVP>(a, g, T, st);
+      case OP_MHD_VJP: return launch_chain_op<OP_MHD_VJP>(a, g, T, st);
+      default: return launch_chain_op<OP_BUNDLE>(a, g, T, st);
+    }
+  }
   std::vector<Elem> seq;
-  // the linearised cross products as one two-pass program each (the output written once, one analysis):
-  // 1.7x faster than two launches at m = 32 (700k points, one tangent: 3.26 -> 1.92 ms) and 1.25x at
-  // m = 64, where the two launches ran on the third-fold kernel (200k points, 4 tangents: 8.40 -> 6.70 ms);
-  // where their products cannot overlay their coefficients (more than 8 angle tiles, m > 85) the two
-  // launches stay.  The MHD VJP's w x c1 + b x c2 likewise (m = 32, 200k points, 4 tangents: 6.51 -> 5.09 ms)
-  // but at m = 64, where its two launches on the third-fold kernel are a little faster (7.74 against
-  // 7.98 ms); the other transposed products (two cross products into different outputs) gained nothing from
-  // one launch of two passes (m = 32: 2.41 -> 2.69 ms).
+  // the linearised cross product as one two-pass program (the output written once, one analysis): 1.7x faster than
+  // two launches at m = 32 (700k points: 3.26 -> 1.92 ms) and 1.25x at m = 64 (200k points, 4 tangents: 8.40 -> 6.70
+  // ms); where its products cannot overlay its coefficients (more than 8 angle tiles, m > 85) the two launches stay.
+  // The MHD VJP's w x c1 + b x c2 likewise from m = 65 (below, chain_kernel).
   const bool fuse_ok = fast_overlay(EK_CROSS2, g.NT, 4 * g.KS_tot);
-  rc = decompose_program(a.op, seq, fuse_ok ? kFuseJvp | (a.m != 64 ? kFuseVjpSum : 0) : 0);
+  rc = decompose_program(a.op, seq, fuse_ok ? kFuseJvp | kFuseVjpSum : 0);
   if (rc) return rc;
   const bool adj_out = op_adjoint_out(a.op);
   for (const Elem &e : seq) {
