@@ -1,11 +1,11 @@
-// sfnl_res.cu -- the FAST form beyond the fused kernels' reach (m = 97 .. 512) on residue grids of 128 angles, with
-// synthesis, program and analysis of a residue in one kernel.
+// sfnl_res.cu -- the FAST form at m = 65 .. 512 on residue grids of M = 64 or 128 angles, with synthesis, program and
+// analysis of a residue in one kernel.
 //
-// On theta_j = pi(2j+1)/N with N = 128 R >= 3m - 2, the angles j = R i + r are phi_i + d_r, phi_i = pi(2i+1)/128 and
-// d_r = pi(2r + 1 - R)/N.  As in sfnl_large.cu, a field is on residue r the transform of 128 real coefficients to 128
-// angles (mode n = 128 q + k of y_n = z_n e^{i n d_r} is mode k with the sign (-1)^q, and the modes k and 128 - k meet
+// On theta_j = pi(2j+1)/N with N = M R >= 3m - 2, the angles j = R i + r are phi_i + d_r, phi_i = pi(2i+1)/M and
+// d_r = pi(2r + 1 - R)/N.  As in sfnl_large.cu, a field is on residue r the transform of M real coefficients to M
+// angles (mode n = M q + k of y_n = z_n e^{i n d_r} is mode k with the sign (-1)^q, and the modes k and M - k meet
 // in one coefficient), third-folded; a product's sums on the residues add up to its coefficients.  Any m fits with
-// R = ceil((3m - 2)/128) residues (3 to 12); a larger grid than the reference's changes nothing, the product being
+// R = ceil((3m - 2)/M) residues (3 to 12); a larger grid than the reference's changes nothing, the product being
 // alias-free on both (fft_parallel.F90:147-328).
 //
 //   coef_kernel   inputs -> the R residues' coefficients of every field, one pass
@@ -14,8 +14,8 @@
 //   out_kernel    the residues' sums -> outputs, one pass
 //
 // The two-kernel form of sfnl_large.cu wrote every field's grid values and read them back once per three outputs; here
-// only coefficients and sums cross HBM.  Both live in tile blocks, [residue][instance][tile][128 rows][8 points], the
-// coefficients in the order of the A fragments, so that a field's tile is one contiguous copy of 8 KB whatever np is.
+// only coefficients and sums cross HBM.  Both live in tile blocks, [residue][instance][tile][M rows][8 points], the
+// coefficients in the order of the A fragments, so that a field's tile is one contiguous copy whatever np is.
 #include <cuda_runtime.h>
 
 #include "sfnl_fold.cuh"
@@ -26,14 +26,23 @@ namespace sfnl {
 
 namespace {
 
-constexpr int kM = 128, kMH = 64, kNT = 4;  // residue grid, its folded modes, quadrant angle tiles
-constexpr int kKS = tf_koff(kMH, 6);        // 32 k-steps of 4 rows
-constexpr int kTile = kKS * 32;             // doubles of one field's tile
-constexpr int kThreads = 64 * kNT;          // two warps (cosine, sine classes) per angle tile
-static_assert(kKS == 32 && tf_KS(kMH, 0) == 4 && tf_KS(kMH, 1) == 4 && tf_KS(kMH, 2) == 8, "row groups of 64 modes");
-
-// Row of the cosine (group 0-2) of folded mode k in group order CE0, CE2, CO; the sine is 64 rows on.
-__host__ __device__ constexpr int row_of(int k) { return k & 1 ? 32 + (k >> 1) : k & 2 ? 16 + (k >> 2) : k >> 2; }
+// Geometry of a residue grid of M angles (64 or 128).
+template <int M>
+struct Res {
+  static constexpr int MH = M / 2, NT = M / 32;    // folded modes, quadrant angle tiles
+  static constexpr int KSE = MH / 16;              // k-steps of an even group (an odd class has twice as many)
+  static constexpr int KS = tf_koff(MH, 6);        // k-steps of 4 rows
+  static constexpr int TILE = KS * 32;             // doubles of one field's tile
+  static constexpr int THREADS = 64 * NT;          // two warps (cosine, sine classes) per angle tile
+  static constexpr int BLOCKS = 24 / (2 * NT);     // CTAs per SM: 24 warps at 80 registers
+  static constexpr int XC = 2 * NT * 3 * 64, PS = 3 * 4 * NT * 64;
+  static constexpr size_t SMEM = sizeof(double) * (3 * TILE + XC + PS);  // 31 or 60 KB
+  static_assert(KS == 8 * KSE && tf_KS(MH, 0) == KSE && tf_KS(MH, 1) == KSE && tf_KS(MH, 2) == 2 * KSE, "row groups");
+  // Row of the cosine (groups 0-2) of folded mode k in group order CE0, CE2, CO; the sine is MH rows on.
+  __host__ __device__ static constexpr int row_of(int k) {
+    return k & 1 ? MH / 2 + (k >> 1) : k & 2 ? MH / 4 + (k >> 2) : k >> 2;
+  }
+};
 __device__ __forceinline__ int coef_at(int row, int g) { return (row >> 2) * 32 + a_frag_slot(row & 3, g); }
 
 // Fields a program synthesises per batch entry (the others are the base state of a linearised program) and the first.
@@ -56,27 +65,28 @@ struct CoefArgs {
   double invN;
 };
 
-// Thread (point, k): Y_k and Y_{128-k} of each residue from the modes 128 q + k and 128 q + 128 - k (k = 0: Y_0 and
-// Y_64 from 128 q and 128 q + 64); writes alpha_k - i beta_k = Y_k - conj(Y_{128-k}) (k = 0: alpha_0 = Re Y_0 and
-// beta_64 = -Im Y_64 in the sine row of mode 0).  Residues pair as d_{R-1-r} = -d_r: one twiddle serves two.
+// Thread (point, k): Y_k and Y_{M-k} of each residue from the modes M q + k and M q + M - k (k = 0: Y_0 and Y_{M/2}
+// from M q and M q + M/2); writes alpha_k - i beta_k = Y_k - conj(Y_{M-k}) (k = 0: alpha_0 = Re Y_0 and beta_{M/2} =
+// -Im Y_{M/2} in the sine row of mode 0).  Residues pair as d_{R-1-r} = -d_r: one twiddle serves two.
 // The block's twiddles (one k: 2 QM modes of R/2 residues) sit in shared memory and all loads are issued first; with
-// both left to the loop over the modes a pass reached 1 TB/s.
-constexpr int res_qm(int R) { return (R + 2) / 3; }  // 128 q + k < m needs q < QM
-template <int R>
+// both left to the loop over the modes a pass reached 1 TB/s.  k runs fastest over the blocks, so that the 64-byte pieces
+// of a tile are written together (R = 6: 519 -> 338 us for 1.8 GB); the passes run at 5.4 to 6.1 TB/s.
+constexpr int res_qm(int R) { return (R + 2) / 3; }  // M q + k < m needs q < QM
+template <int M, int R>
 __device__ __forceinline__ void load_twiddles(double2 (&tw)[res_qm(R)][2][R / 2], const double *src, int m, int k) {
   constexpr int RP = R / 2, n_tw = res_qm(R) * 2 * RP;
   for (int i = threadIdx.x; i < n_tw; i += blockDim.x) {
     const int r = i % RP, side = (i / RP) & 1, q = i / (2 * RP);
-    const int n = q * kM + (side == 0 ? k : k == 0 ? kMH : kM - k);
+    const int n = q * M + (side == 0 ? k : k == 0 ? M / 2 : M - k);
     tw[q][side][r] = n < m ? reinterpret_cast<const double2 *>(src)[(size_t)r * m + n] : make_double2(0.0, 0.0);
   }
 }
-template <int R>
+template <int M, int R>
 __global__ void __launch_bounds__(128) coef_kernel(const CoefArgs a) {
-  constexpr int RP = R / 2, QM = res_qm(R);
+  constexpr int RP = R / 2, QM = res_qm(R), MH = Res<M>::MH, TILE = Res<M>::TILE;
   __shared__ double2 tw[QM][2][RP];
-  const int64_t nblk = (a.npts + blockDim.x - 1) / blockDim.x, pb = blockIdx.x >> 6;
-  const int inst = (int)(pb / nblk), k = blockIdx.x & (kMH - 1);
+  const int64_t nblk = (a.npts + blockDim.x - 1) / blockDim.x, pb = blockIdx.x / MH;
+  const int inst = (int)(pb / nblk), k = blockIdx.x & (MH - 1);
   const int64_t p = (pb - inst * nblk) * blockDim.x + threadIdx.x;
   int f = 0;
   while (f + 1 < a.nf && inst >= a.inst[f + 1]) ++f;
@@ -88,12 +98,12 @@ __global__ void __launch_bounds__(128) coef_kernel(const CoefArgs a) {
   for (int q = 0; q < QM; ++q)
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
-      const int n = q * kM + (side == 0 ? k : k == 0 ? kMH : kM - k);
+      const int n = q * M + (side == 0 ? k : k == 0 ? MH : M - k);
       const bool live = valid && n < a.m;
       av[q][side] = live ? x[(int64_t)n * ldm] : 0.0;
       bv[q][side] = live && n > 0 ? x[(int64_t)n * ldm + a.np] : 0.0;  // the sine of mode 0 is ignored
     }
-  load_twiddles<R>(tw, a.tw, a.m, k);
+  load_twiddles<M, R>(tw, a.tw, a.m, k);
   __syncthreads();
   if (!valid) return;
   double yr[2][R], yi[2][R];
@@ -123,10 +133,10 @@ __global__ void __launch_bounds__(128) coef_kernel(const CoefArgs a) {
     }
   }
   const int64_t ninst = a.inst[a.nf];
-  double *c = a.C + ((int64_t)inst * a.tiles + (p >> 3)) * kTile;
-  const int row = row_of(k), ic = coef_at(row, (int)(p & 7)), is = coef_at(row + 64, (int)(p & 7));
+  double *c = a.C + ((int64_t)inst * a.tiles + (p >> 3)) * TILE;
+  const int row = Res<M>::row_of(k), ic = coef_at(row, (int)(p & 7)), is = coef_at(row + MH, (int)(p & 7));
 #pragma unroll
-  for (int r = 0; r < R; ++r, c += ninst * a.tiles * kTile) {
+  for (int r = 0; r < R; ++r, c += ninst * a.tiles * TILE) {
     c[ic] = k == 0 ? yr[0][r] : yr[0][r] - yr[1][r];
     c[is] = k == 0 ? -yi[1][r] : -(yi[0][r] + yi[1][r]);
   }
@@ -142,27 +152,27 @@ struct OutArgs {
   const double *tw;
 };
 
-// Thread (point, k): the modes 128 q + k and 128 q + 128 - k (k = 0: 128 q and 128 q + 64) of one output from the R
-// residues' sums, c_n = sum_r e^{-i n d_r} P^r_n with P^r_k = C - i S, P^r_{128-k} = -conj(P^r_k), P^r_64 = -i S_64 and
-// P^r_{128q+k} = (-1)^q P^r_k.
-template <int R>
+// Thread (point, k): the modes M q + k and M q + M - k (k = 0: M q and M q + M/2) of one output from the R residues'
+// sums, c_n = sum_r e^{-i n d_r} P^r_n with P^r_k = C - i S, P^r_{M-k} = -conj(P^r_k), P^r_{M/2} = -i S_{M/2} and
+// P^r_{Mq+k} = (-1)^q P^r_k.
+template <int M, int R>
 __global__ void __launch_bounds__(128) out_kernel(const OutArgs a) {
-  constexpr int RP = R / 2, QM = res_qm(R);
+  constexpr int RP = R / 2, QM = res_qm(R), MH = Res<M>::MH, TILE = Res<M>::TILE;
   __shared__ double2 tw[QM][2][RP];
-  const int64_t nblk = (a.npts + blockDim.x - 1) / blockDim.x, pb = blockIdx.x >> 6;
-  const int inst = (int)(pb / nblk), k = blockIdx.x & (kMH - 1), o = inst / a.nb, b = inst - o * a.nb;
+  const int64_t nblk = (a.npts + blockDim.x - 1) / blockDim.x, pb = blockIdx.x / MH;
+  const int inst = (int)(pb / nblk), k = blockIdx.x & (MH - 1), o = inst / a.nb, b = inst - o * a.nb;
   const int64_t p = (pb - inst * nblk) * blockDim.x + threadIdx.x;
   const bool valid = p < a.npts;
-  const double *s = a.S + ((int64_t)inst * a.tiles + (p >> 3)) * kTile + row_of(k) * 8 + (p & 7);
+  const double *s = a.S + ((int64_t)inst * a.tiles + (p >> 3)) * TILE + Res<M>::row_of(k) * 8 + (p & 7);
   double *op = a.out[o] + (int64_t)(a.b0 + b) * a.bs[o] + p * a.ops;
-  const int64_t ldm = a.ldm[o], rst = (int64_t)a.no * a.nb * a.tiles * kTile;
+  const int64_t ldm = a.ldm[o], rst = (int64_t)a.no * a.nb * a.tiles * TILE;
   double C[R], Sv[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     C[r] = valid ? s[r * rst] : 0.0;
-    Sv[r] = valid ? s[r * rst + 64 * 8] : 0.0;
+    Sv[r] = valid ? s[r * rst + MH * 8] : 0.0;
   }
-  load_twiddles<R>(tw, a.tw, a.m, k);
+  load_twiddles<M, R>(tw, a.tw, a.m, k);
   __syncthreads();
   if (!valid) return;
 #pragma unroll
@@ -170,7 +180,7 @@ __global__ void __launch_bounds__(128) out_kernel(const OutArgs a) {
     const double sg = (q & 1) ? -1.0 : 1.0;
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
-      const int n = q * kM + (side == 0 ? k : k == 0 ? kMH : kM - k);
+      const int n = q * M + (side == 0 ? k : k == 0 ? MH : M - k);
       if (n >= a.m) continue;
       auto px = [&](int r) { return side == 0 ? C[r] : k == 0 ? 0.0 : -C[r]; };
       auto py = [&](int r) { return side == 0 && k == 0 ? 0.0 : -Sv[r]; };
@@ -204,8 +214,10 @@ struct ProdArgs {
 };
 
 // One tile of a residue: copies of the next fields, synthesis and folds of the current ones, analysis of products.
+template <int M>
 struct Tile {
-  double *xs, *xc, *ps;  // staged coefficients [3][32][32], exchange, folded products [3][4][kNT][2][32]
+  static constexpr int kNT = Res<M>::NT, kTile = Res<M>::TILE, kThreads = Res<M>::THREADS, KSE = Res<M>::KSE, MH = Res<M>::MH;
+  double *xs, *xc, *ps;  // staged coefficients [3][KS][32], exchange, folded products [3][4][kNT][2][32]
   const double *syn, *ana;
   int lane, warp, tau, half;
 
@@ -230,18 +242,18 @@ struct Tile {
 #pragma unroll
     for (int f = 0; f < NG; ++f) acc_e[f][0] = acc_e[f][1] = acc_o[f][0] = acc_o[f][1] = 0.0;
     const bool first = tau < kNT / 2;
-    const int ke = 16 * half + (first ? 0 : 4), ko = 16 * half + 8;  // first k-steps: even part, odd class
+    const int ke = 4 * KSE * half + (first ? 0 : KSE), ko = 4 * KSE * half + 2 * KSE;  // first k-steps: even part, odd class
     const double *xl = xs + a_frag_slot(lane & 3, lane >> 2);
     const double *be = syn + ((size_t)ke * kNT + (first ? tau : kNT - 1 - tau)) * 32 + lane;
     const double *bo = syn + ((size_t)ko * kNT + tau) * 32 + lane;
     double bn = __ldg(bo);
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
+    for (int s = 0; s < 2 * KSE; ++s) {
       const double bv = bn;
-      if (s < 7) bn = __ldg(bo + (size_t)(s + 1) * kNT * 32);
+      if (s + 1 < 2 * KSE) bn = __ldg(bo + (size_t)(s + 1) * kNT * 32);
 #pragma unroll
       for (int f = 0; f < NG; ++f) dmma(acc_o[f], xl[f * kTile + (ko + s) * 32], bv);
-      if (s < 4) {
+      if (s < KSE) {
         const double b2 = __ldg(be + (size_t)s * kNT * 32);
 #pragma unroll
         for (int f = 0; f < NG; ++f) dmma(acc_e[f], xl[f * kTile + (ke + s) * 32], b2);
@@ -261,10 +273,13 @@ struct Tile {
     const int q = lane & 3, g = lane >> 2;
 #pragma unroll
     for (int odd = 1; odd >= 0; --odd) {
-      // groups: CO, SO (4 output tiles of 8 modes each) or CE0, CE2, SE0, SE2 (2 each)
-      const int gr = odd ? (warp < 4 ? 2 : 5) : (warp >> 1) + (warp >= 4 ? 1 : 0), u = odd ? warp & 3 : warp & 1;
+      // groups: CO, SO (NUO output tiles of 8 modes each) or CE0, CE2, SE0, SE2 (NUE each)
+      constexpr int NUE = MH / 32, NUO = MH / 16;
+      const int ev = warp / NUE;
+      const int gr = odd ? (warp < NUO ? 2 : 5) : ev + (ev >= 2 ? 1 : 0), u = odd ? warp % NUO : warp % NUE;
       const int c = odd ? (gr == 2 ? 1 : 3) : gr < 3 ? 0 : 2, TE = odd ? 2 * kNT : kNT;
-      const int aof = gr == 0 ? 0 : gr == 1 ? 2 * kNT : gr == 2 ? 4 * kNT : gr == 3 ? 12 * kNT : gr == 4 ? 14 * kNT : 16 * kNT;
+      constexpr int AE = NUE * kNT, AO = 2 * NUO * kNT;  // analysis k-steps of an even group, of an odd class
+      const int aof = gr == 0 ? 0 : gr == 1 ? AE : gr == 2 ? 2 * AE : gr == 3 ? 2 * AE + AO : gr == 4 ? 3 * AE + AO : 4 * AE + AO;
       const double sg = gr == 0 || gr == 4 ? 1.0 : -1.0;  // mirror sign: PE0 +, PE2 -, QE0 -, QE2 +
       const double *bt = ana + (size_t)(aof + u * TE) * 32 + lane;
       const double *pa = ps + (size_t)c * kNT * 64;
@@ -283,7 +298,7 @@ struct Tile {
           dmma(y[te & 1][o], av, bv);
         }
       }
-      const int row0 = (gr == 0 ? 0 : gr == 1 ? 16 : gr == 2 ? 32 : gr == 3 ? 64 : gr == 4 ? 80 : 96) + 8 * u + 2 * q;
+      const int row0 = (gr % 3 == 0 ? 0 : gr % 3 == 1 ? MH / 4 : MH / 2) + (gr >= 3 ? MH : 0) + 8 * u + 2 * q;
 #pragma unroll
       for (int o = 0; o < NO; ++o)
 #pragma unroll
@@ -292,16 +307,19 @@ struct Tile {
   }
 };
 
-__device__ __forceinline__ Tile make_tile(double *smem, const double *syn, const double *ana) {
+template <int M>
+__device__ __forceinline__ Tile<M> make_tile(double *smem, const double *syn, const double *ana) {
   const int warp = threadIdx.x >> 5;
-  return {smem, smem + 3 * kTile, smem + 3 * kTile + 2 * kNT * 3 * 64, syn, ana, (int)threadIdx.x & 31, warp, warp >> 1, warp & 1};
+  double *xc = smem + 3 * Res<M>::TILE;
+  return {smem, xc, xc + Res<M>::XC, syn, ana, (int)threadIdx.x & 31, warp, warp >> 1, warp & 1};
 }
-constexpr size_t kSmem = sizeof(double) * (3 * kTile + 2 * kNT * 3 * 64 + 3 * 4 * kNT * 64);
 
 // Grid values of three shared fields (blockIdx.z) of a tile (blockIdx.x) on residue blockIdx.y.
-__global__ void __launch_bounds__(kThreads, 3) base_kernel(const ProdArgs a) {
+template <int M>
+__global__ void __launch_bounds__(Res<M>::THREADS, Res<M>::BLOCKS) base_kernel(const ProdArgs a) {
+  constexpr int kTile = Res<M>::TILE, kNT = Res<M>::NT;
   extern __shared__ __align__(16) double smem[];
-  const Tile t = make_tile(smem, a.syn, a.ana);
+  const Tile<M> t = make_tile<M>(smem, a.syn, a.ana);
   const int f0 = 3 * blockIdx.z;
   const double *src[3];
 #pragma unroll
@@ -321,11 +339,12 @@ __global__ void __launch_bounds__(kThreads, 3) base_kernel(const ProdArgs a) {
 // Program OP on one tile, batch entry and residue (blockIdx.x = tile * nb + entry, blockIdx.y = residue): the entry's
 // fields are transformed three at a time, the first ones' quadrant values waiting in registers, and the outputs
 // analysed three at a time.  The entries of a tile run next to each other, so that the base state's grid values come
-// from L2 after the first.  60 KB of shared memory and 80 registers: three CTAs of 8 warps per SM.
-template <int OP>
-__global__ void __launch_bounds__(kThreads, 3) prod_kernel(const ProdArgs a) {
+// from L2 after the first.  At 80 registers 24 warps share an SM (three CTAs of 8 at M = 128, six of 4 at M = 64).
+template <int OP, int M>
+__global__ void __launch_bounds__(Res<M>::THREADS, Res<M>::BLOCKS) prod_kernel(const ProdArgs a) {
+  constexpr int kTile = Res<M>::TILE, kNT = Res<M>::NT;
   extern __shared__ __align__(16) double smem[];
-  const Tile t = make_tile(smem, a.syn, a.ana);
+  const Tile<M> t = make_tile<M>(smem, a.syn, a.ana);
   const int64_t tile = blockIdx.x / a.nb;
   const int b = (int)(blockIdx.x - tile * a.nb), r = blockIdx.y;
   auto field = [&](int f) { return a.C + (((int64_t)r * a.ninst + a.inst[f] + b) * a.tiles + tile) * kTile; };
@@ -432,50 +451,69 @@ __global__ void __launch_bounds__(kThreads, 3) prod_kernel(const ProdArgs a) {
   }
 }
 
-template <int OP>
+template <int OP, int M>
 int launch_prod(const ProdArgs &pa, int R, cudaStream_t st) {
   static KernelSetup setup;
-  if (int rc = setup.opt_in(reinterpret_cast<const void *>(prod_kernel<OP>), kSmem)) return rc;
-  prod_kernel<OP><<<dim3((unsigned)(pa.tiles * pa.nb), (unsigned)R), kThreads, kSmem, st>>>(pa);
+  if (int rc = setup.opt_in(reinterpret_cast<const void *>(prod_kernel<OP, M>), Res<M>::SMEM)) return rc;
+  prod_kernel<OP, M><<<dim3((unsigned)(pa.tiles * pa.nb), (unsigned)R), Res<M>::THREADS, Res<M>::SMEM, st>>>(pa);
   return check_launch("residue grids: program");
 }
+template <int M>
+int launch_base(const ProdArgs &pa, int R, cudaStream_t st) {
+  static KernelSetup setup;
+  if (int rc = setup.opt_in(reinterpret_cast<const void *>(base_kernel<M>), Res<M>::SMEM)) return rc;
+  base_kernel<M><<<dim3((unsigned)pa.tiles, (unsigned)R, (unsigned)(pa.nshared / 3)), Res<M>::THREADS, Res<M>::SMEM, st>>>(pa);
+  return check_launch("residue grids: base state");
+}
 
-template <int R>
+template <int M, int R>
 int launch_passes(const CoefArgs *ca, const OutArgs *oa, cudaStream_t st) {
-  if (ca) {
-    const int64_t nblk = (ca->npts + 127) / 128;
-    coef_kernel<R><<<(unsigned)(nblk * ca->inst[ca->nf] * kMH), 128, 0, st>>>(*ca);
-  } else {
-    const int64_t nblk = (oa->npts + 127) / 128;
-    out_kernel<R><<<(unsigned)(nblk * oa->no * oa->nb * kMH), 128, 0, st>>>(*oa);
-  }
+  const int64_t nblk = ((ca ? ca->npts : oa->npts) + 127) / 128 * Res<M>::MH;
+  if (ca)
+    coef_kernel<M, R><<<(unsigned)(nblk * ca->inst[ca->nf]), 128, 0, st>>>(*ca);
+  else
+    out_kernel<M, R><<<(unsigned)(nblk * oa->no * oa->nb), 128, 0, st>>>(*oa);
   return check_launch("residue grids: coefficients and outputs");
 }
+template <int M>
 int launch_passes(int R, const CoefArgs *ca, const OutArgs *oa, cudaStream_t st) {
   switch (R) {
-    case 3: return launch_passes<3>(ca, oa, st);
-    case 4: return launch_passes<4>(ca, oa, st);
-    case 5: return launch_passes<5>(ca, oa, st);
-    case 6: return launch_passes<6>(ca, oa, st);
-    case 7: return launch_passes<7>(ca, oa, st);
-    case 8: return launch_passes<8>(ca, oa, st);
-    case 9: return launch_passes<9>(ca, oa, st);
-    case 10: return launch_passes<10>(ca, oa, st);
-    case 11: return launch_passes<11>(ca, oa, st);
-    default: return launch_passes<12>(ca, oa, st);
+    case 3: return launch_passes<M, 3>(ca, oa, st);
+    case 4: return launch_passes<M, 4>(ca, oa, st);
+    case 5: return launch_passes<M, 5>(ca, oa, st);
+    case 6: return launch_passes<M, 6>(ca, oa, st);
+    case 7: return launch_passes<M, 7>(ca, oa, st);
+    case 8: return launch_passes<M, 8>(ca, oa, st);
+    case 9: return launch_passes<M, 9>(ca, oa, st);
+    case 10: return launch_passes<M, 10>(ca, oa, st);
+    case 11: return launch_passes<M, 11>(ca, oa, st);
+    case 12: return launch_passes<M, 12>(ca, oa, st);
   }
+  return set_error(SFNL_ERR_UNSUPPORTED, "residue grids: no such number of residues");
 }
 
 }  // namespace
 
+// Residue grids of 64 angles while at most this many cover the grid (m <= 256), else of 128: the transforms of 64 angles
+// have half the DMMAs per angle, and the passes' twiddles, twice as many, hide behind HBM.  Against 128 angles: cross
+// product, 35,000 points, m = 128 0.558 -> 0.465 ms, m = 256 1.107 -> 1.012; MHD JVP, 7,000 points, 16 tangents, m = 128
+// 3.47 -> 3.19 ms, m = 256 7.15 -> 7.07.
+constexpr int kRes64Max = 12;
+
+// From m = 65, where the fused kernels run on run-time loops: cross product, 30,000 points, m = 65 0.433 -> 0.274 ms, m =
+// 100 0.769 -> 0.333; MHD VJP, 10,000 points, 4 cotangents, m = 65 1.91 -> 0.83 ms.  The cross product's JVP from m = 73:
+// its two-pass fused program is the faster one before (m = 72 0.370 against 0.393 ms, m = 80 0.573 against 0.395).
 bool res_supported(int op, int m) {
-  if (m <= 85 || m > 512) return false;  // 3 to 12 residues
+  if (m < (op == OP_CROSS_JVP ? 73 : 65) || m > 512) return false;
   return op == OP_CROSS || op == OP_DOT || op == OP_PROD || op == OP_SVECT || linear_op(op);
 }
 
+namespace {
 // Points and batch entries go in chunks whose coefficients, base values and sums fit `cap` bytes of workspace.
-int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st) {
-  const int m = a.m, R = (3 * m - 2 + kM - 1) / kM, N = kM * R;
+template <int M>
+int launch_res_m(const ProgArgs &a, size_t cap, cudaStream_t st) {
+  constexpr int kTile = Res<M>::TILE;
+  const int m = a.m, R = (3 * m - 2 + M - 1) / M, N = M * R;
   const int ni = op_nin(a.op), no = op_nout(a.op);
   const bool lin = linear_op(a.op);
   const int nsh = lin ? first_own(a.op) : 0, own = ni - nsh;
@@ -492,8 +530,6 @@ int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st) {
   double *W = nullptr;
   if (int rc = large_workspace(st, (size_t)chunk * (shared_b + kb * entry_b), &W, 2)) return rc;
   const bool adj_out = op_adjoint_out(a.op);
-  static KernelSetup setup;
-  if (int rc = setup.opt_in(reinterpret_cast<const void *>(base_kernel), kSmem)) return rc;
   for (int64_t c0 = 0; c0 < a.np; c0 += chunk)
     for (int b0 = 0; b0 < a.batch; b0 += (int)kb) {
       const int nb = a.batch - b0 < kb ? a.batch - b0 : (int)kb;
@@ -526,21 +562,19 @@ int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st) {
       for (int f = 0; f < ni; ++f) pa.inst[f] = ca.inst[f];
       pa.nshared = nsh;
       pa.nb = nb;
-      if (int rc = launch_passes(R, &ca, nullptr, st)) return rc;
-      if (lin) {
-        base_kernel<<<dim3((unsigned)ca.tiles, (unsigned)R, (unsigned)(nsh / 3)), kThreads, kSmem, st>>>(pa);
-        if (int rc = check_launch("residue grids: base state")) return rc;
-      }
+      if (int rc = launch_passes<M>(R, &ca, nullptr, st)) return rc;
+      if (lin)
+        if (int rc = launch_base<M>(pa, R, st)) return rc;
       int rc = SFNL_OK;
       switch (a.op) {
-        case OP_CROSS: rc = launch_prod<OP_CROSS>(pa, R, st); break;
-        case OP_DOT: rc = launch_prod<OP_DOT>(pa, R, st); break;
-        case OP_PROD: rc = launch_prod<OP_PROD>(pa, R, st); break;
-        case OP_SVECT: rc = launch_prod<OP_SVECT>(pa, R, st); break;
-        case OP_CROSS_JVP: rc = launch_prod<OP_CROSS_JVP>(pa, R, st); break;
-        case OP_CROSS_VJP: rc = launch_prod<OP_CROSS_VJP>(pa, R, st); break;
-        case OP_MHD_JVP: rc = launch_prod<OP_MHD_JVP>(pa, R, st); break;
-        case OP_MHD_VJP: rc = launch_prod<OP_MHD_VJP>(pa, R, st); break;
+        case OP_CROSS: rc = launch_prod<OP_CROSS, M>(pa, R, st); break;
+        case OP_DOT: rc = launch_prod<OP_DOT, M>(pa, R, st); break;
+        case OP_PROD: rc = launch_prod<OP_PROD, M>(pa, R, st); break;
+        case OP_SVECT: rc = launch_prod<OP_SVECT, M>(pa, R, st); break;
+        case OP_CROSS_JVP: rc = launch_prod<OP_CROSS_JVP, M>(pa, R, st); break;
+        case OP_CROSS_VJP: rc = launch_prod<OP_CROSS_VJP, M>(pa, R, st); break;
+        case OP_MHD_JVP: rc = launch_prod<OP_MHD_JVP, M>(pa, R, st); break;
+        case OP_MHD_VJP: rc = launch_prod<OP_MHD_VJP, M>(pa, R, st); break;
         default: rc = set_error(SFNL_ERR_ARG, "residue grids: unknown program");
       }
       if (rc) return rc;
@@ -562,9 +596,15 @@ int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st) {
         oa.ldm[o] = a.out_ldm[o];
         oa.bs[o] = a.out_bs[o];
       }
-      if (int rc2 = launch_passes(R, nullptr, &oa, st)) return rc2;
+      if (int rc2 = launch_passes<M>(R, nullptr, &oa, st)) return rc2;
     }
   return SFNL_OK;
+}
+}  // namespace
+
+int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st) {
+  if (3 * a.m - 2 <= 64 * kRes64Max) return launch_res_m<64>(a, cap, st);
+  return launch_res_m<128>(a, cap, st);
 }
 
 }  // namespace sfnl

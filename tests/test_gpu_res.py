@@ -1,0 +1,58 @@
+"""The FAST form on residue grids (m = 65 .. 512) at the bounds of its residue counts and grid lengths: 64 angles up to
+m = 256, 128 beyond; each number of residues from both; mode counts that fill the last residue block or leave it nearly
+empty; point counts that are no multiple of the 8-point tiles; and a small workspace, which splits points and batch
+entries into several chunks.  Against pocketfft products; rel-L2 <= 1e-12, the bar of the FP64 forms."""
+import numpy as np
+import pytest
+
+import sfemans_b200 as sf
+from oracle import ref_fft as R
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+SIZES = [65, 72, 73, 86, 87, 107, 108, 128, 129, 150, 171, 192, 200, 214, 235, 256, 257, 299, 300, 384, 385, 470, 512]
+
+
+def _pad(m):
+    return (3 * m + 1) // 2
+
+
+def _field(npts, nslot, m, seed):
+    return R.synthetic_field(npts, nslot, m, 0.05, seed)
+
+
+@pytest.mark.parametrize("m", SIZES)
+@pytest.mark.parametrize("kind", ["cross", "dot", "prod", "svect"])
+def test_products(kind, m):
+    _, n1, n2, _ = sf.KINDS[kind]
+    for npts in (5, 16):
+        V1, V2 = _field(npts, n1, m, 21 + m), _field(npts, n2, m, 22 + m)
+        out = sf.product(sf.KINDS[kind][0], sf.to_device(V1), sf.to_device(V2), m_max_pad=_pad(m), algo=sf.ALGO_FAST)
+        assert R.rel_l2(sf.to_host(out), R.fft_par(kind, V1, V2, _pad(m))) <= TOL
+
+
+@pytest.mark.parametrize("cap", [0, 1 << 20])
+@pytest.mark.parametrize("m", [65, 73, 129, 200, 256, 257, 400])
+def test_linearised_programs(m, cap):
+    npts, k = 21, 3
+    cross = lambda x, y: R.fft_par("cross", np.asfortranarray(x), np.asfortranarray(y), _pad(m))  # noqa: E731
+    u, w, b = (_field(npts, 6, m, 31 + i) for i in range(3))
+    v = np.asfortranarray(np.stack([_field(npts, 18, m, 41 + i) for i in range(k)], -1))
+    c = np.asfortranarray(np.stack([_field(npts, 12, m, 51 + i) for i in range(k)], -1))
+    base = [sf.to_device(x) for x in (u, w, b)]
+    v12, c1 = np.asfortranarray(v[:, :12]), np.asfortranarray(c[:, :6])
+    assert sf.lib().sfnl_test_large_workspace_cap(cap) == 0
+    try:
+        jv, jc = (sf.to_host(f(*base, sf.to_device(x), m_max_pad=_pad(m))) for f, x in ((sf.mhd_jvp, v), (sf.mhd_vjp, c)))
+        jv1 = sf.to_host(sf.cross_jvp(*base[:2], sf.to_device(v12), m_max_pad=_pad(m)))
+        jc1 = sf.to_host(sf.cross_vjp(*base[:2], sf.to_device(c1), m_max_pad=_pad(m)))
+    finally:
+        sf.lib().sfnl_test_large_workspace_cap(0)
+    for t in range(k):
+        du, dw, db = (v[:, 6 * i:6 * i + 6, :, t] for i in range(3))
+        ref1 = cross(du, w) + cross(u, dw)
+        ref = np.concatenate([ref1, cross(du, b) + cross(u, db)], 1)
+        assert R.rel_l2(jv[..., t], ref) <= TOL and R.rel_l2(jv1[..., t], ref1) <= TOL
+        scale = np.linalg.norm(ref) * np.linalg.norm(c[..., t])
+        assert abs(float((ref * c[..., t]).sum() - (v[..., t] * jc[..., t]).sum())) <= TOL * scale
+        assert abs(float((ref1 * c1[..., t]).sum() - (v12[..., t] * jc1[..., t]).sum())) <= TOL * scale
