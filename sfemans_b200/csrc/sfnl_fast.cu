@@ -1791,10 +1791,10 @@ int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
   }
   // every (KS, NT) of make_geo up to m = 64; run-time loops cost the sizes between 16, 32 and 64 a third of their time
   // (cross product, 50,001 points: m = 20 99 -> 62 us, m = 40 207 -> 148, m = 48 337 -> 202, m = 52 384 -> 229)
-  if constexpr (ADJ != 0) {  // transposed products: chain_kernel and the residue grids take the other sizes
+  if constexpr (ADJ != 0) {  // transposed products: chain_kernel takes the other sizes up to m = 64
     if (fa.NT == 6 && fa.KS[0] == 7) return launch_ek_m<EK, 7, 6, ADJ>(fa, batch, st);
     if (fa.NT == 6 && fa.KS[0] == 8) return launch_ek_m<EK, 8, 6, ADJ>(fa, batch, st);
-    return set_error(SFNL_ERR_ARG, "FAST form: unsupported cotangent operands");
+    return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);  // m > 64 without a workspace
   } else {
   switch (10 * fa.KS[0] + fa.NT) {
     case 11: return launch_ek_m<EK, 1, 1, ADJ>(fa, batch, st);
@@ -1838,7 +1838,7 @@ int rows_aligned16(const FastArgs &fa, int ni) {
 }
 }  // namespace
 
-int decompose_program(int op, std::vector<Elem> &seq) {
+int decompose_program(int op, std::vector<Elem> &seq, bool fuse) {
   seq.clear();
   auto add = [&](int ek, std::initializer_list<int> in, std::initializer_list<int> out, unsigned adj, int acc) {
     Elem e{};
@@ -1869,11 +1869,28 @@ int decompose_program(int op, std::vector<Elem> &seq) {
       add(EK_PROD, {6, 7}, {0}, 0, 1);                       // + d c
       break;
     case OP_CROSS_JVP:  // [u, w, du, dw]
-      add(EK_CROSS2, {6, 7, 8, 3, 4, 5, 0, 1, 2, 9, 10, 11}, {0, 1, 2}, 0, 0);  // du x w + u x dw
+      if (fuse) {
+        add(EK_CROSS2, {6, 7, 8, 3, 4, 5, 0, 1, 2, 9, 10, 11}, {0, 1, 2}, 0, 0);  // du x w + u x dw
+        break;
+      }
+      add(EK_CROSS, {6, 7, 8, 3, 4, 5}, {0, 1, 2}, 0, 0);     // du x w
+      add(EK_CROSS, {0, 1, 2, 9, 10, 11}, {0, 1, 2}, 0, 1);   // + u x dw
       break;
     case OP_CROSS_VJP:  // [u, w, c]
       add(EK_CROSS, {3, 4, 5, 6, 7, 8}, {0, 1, 2}, A1, 0);    // w x c
       add(EK_CROSS, {6, 7, 8, 0, 1, 2}, {3, 4, 5}, A0, 0);    // c x u
+      break;
+    case OP_MHD_JVP:  // [u, w, b, du, dw, db]
+      add(EK_CROSS, {9, 10, 11, 3, 4, 5}, {0, 1, 2}, 0, 0);   // du x w
+      add(EK_CROSS, {0, 1, 2, 12, 13, 14}, {0, 1, 2}, 0, 1);  // + u x dw
+      add(EK_CROSS, {9, 10, 11, 6, 7, 8}, {3, 4, 5}, 0, 0);   // du x b
+      add(EK_CROSS, {0, 1, 2, 15, 16, 17}, {3, 4, 5}, 0, 1);  // + u x db
+      break;
+    case OP_MHD_VJP:  // [u, w, b, c1, c2]
+      add(EK_CROSS, {3, 4, 5, 9, 10, 11}, {0, 1, 2}, A1, 0);  // w x c1
+      add(EK_CROSS, {6, 7, 8, 12, 13, 14}, {0, 1, 2}, A1, 1); // + b x c2
+      add(EK_CROSS, {9, 10, 11, 0, 1, 2}, {3, 4, 5}, A0, 0);  // c1 x u
+      add(EK_CROSS, {12, 13, 14, 0, 1, 2}, {6, 7, 8}, A0, 0); // c2 x u
       break;
     default: return set_error(SFNL_ERR_ARG, "unknown program");
   }
@@ -2145,7 +2162,15 @@ int launch_fast(const ProgArgs &a, cudaStream_t st) {
   Tables T;
   int rc = get_tables(g, &T);
   if (rc) return rc;
-  if (!fast_fused_fits(a.op, a.m) || res_supported(a.op, a.m)) return launch_fast_large(a, g, T, st);
+  if (!fast_fused_fits(a.op, a.m)) return launch_fast_large(a, g, T, st);
+  // Where both fit the residue grids are faster, but want a workspace of the stream's own: a call that is being captured
+  // into a graph, where it cannot be allocated, and one for which there is no memory take the fused kernels.
+  if (res_supported(a.op, a.m)) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+    if (cap == cudaStreamCaptureStatusNone)
+      if (const int r = launch_fast_large(a, g, T, st); r != SFNL_ERR_ALLOC) return r;
+  }
   if (chain_fits(a.op, a.m, g) && a.out_ps == 1) {
     switch (a.op) {
       case OP_CROSS_VJP: return launch_chain_op<OP_CROSS_VJP>(a, g, T, st);
@@ -2157,8 +2182,8 @@ int launch_fast(const ProgArgs &a, cudaStream_t st) {
   std::vector<Elem> seq;
   // the linearised cross product as one two-pass program (the output written once, one analysis): 1.7x faster than
   // two launches at m = 32 (700k points: 3.26 -> 1.92 ms) and 1.25x at m = 64 (200k points, 4 tangents: 8.40 -> 6.70
-  // ms); the residue grids take it from m = 73.
-  rc = decompose_program(a.op, seq);
+  // ms); where its products cannot overlay its coefficients (more than 8 angle tiles, m > 85) two launches.
+  rc = decompose_program(a.op, seq, fast_overlay(EK_CROSS2, g.NT, 4 * g.KS_tot));
   if (rc) return rc;
   const bool adj_out = op_adjoint_out(a.op);
   for (const Elem &e : seq) {

@@ -56,3 +56,24 @@ def test_linearised_programs(m, cap):
         scale = np.linalg.norm(ref) * np.linalg.norm(c[..., t])
         assert abs(float((ref * c[..., t]).sum() - (v[..., t] * jc[..., t]).sum())) <= TOL * scale
         assert abs(float((ref1 * c1[..., t]).sum() - (v12[..., t] * jc1[..., t]).sum())) <= TOL * scale
+
+
+@pytest.mark.parametrize("m", [72, 96])
+def test_captured_calls_without_a_workspace(m):
+    # a graph is captured on a stream that has no workspace yet: sizes that the fused kernels hold run on them
+    torch = pytest.importorskip("torch")
+    npts = 19
+    f = [_field(npts, 6, m, 61 + i) for i in range(3)]
+    c = _field(npts, 12, m, 71)
+    u, w, b, cd = (sf.to_device(x) for x in (*f, c))
+    eager = sf.product(sf.OP_CROSS, u, w, m_max_pad=_pad(m)), sf.mhd_vjp(u, w, b, cd, m_max_pad=_pad(m))
+    outs = [torch.zeros_like(x) for x in eager]
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        sf.product(sf.OP_CROSS, u, w, out=outs[0], m_max_pad=_pad(m))
+        sf.mhd_vjp(u, w, b, cd, out=outs[1], m_max_pad=_pad(m))
+    g.replay()
+    torch.cuda.synchronize()
+    for o, e in zip(outs, eager):
+        assert R.rel_l2(sf.to_host(o), sf.to_host(e)) <= TOL
