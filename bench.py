@@ -241,9 +241,9 @@ def main():
 
     forms = {"fp64": dict(algo=sf.ALGO_FAST), "split3": dict(split=sf.SPLIT_BF16X3),
              "split2": dict(split=sf.SPLIT_BF16X2), "grid": dict(algo=sf.ALGO_GRID)}
-    # kernel launches per step: the bundle is one launch in every form except FAST at m != 64 (four
+    # kernel launches per step: the bundle is one launch in every form, FAST beyond m = 64 excepted (four
     # elementary launches); the other workloads are one launch
-    launches = {"fp64": 1 if m == 64 else 4, "split3": 1, "split2": 1, "grid": 1} if args.workload == "mhd_bundle" \
+    launches = {"fp64": 1 if m <= 64 else 4, "split3": 1, "split2": 1, "grid": 1} if args.workload == "mhd_bundle" \
         else {"fp64": 1, "split3": 1, "split2": 1, "grid": 1}
     # every form is timed (the others after the reported one, on fewer steps); the line reports --form,
     # or with --form auto the fastest form that meets its accuracy bar
@@ -319,7 +319,7 @@ def main():
         configs = _extra_configs(args, sf, torch, dev, world, rank, dist, local, stream)
 
     if args.workload == "mhd_bundle":
-        kname = {"fp64": "fast_bundle_r3_kernel" if m == 64 else "fast_kernel<EK_CROSS>",
+        kname = {"fp64": "fast_bundle_r3_kernel" if m == 64 else "chain_kernel<OP_BUNDLE>" if m < 64 else "fast_kernel<EK_CROSS>",
                  "split3": "split_kernel<PR_BUNDLE>", "split2": "split_kernel<PR_BUNDLE>", "grid": "grid_kernel<OP_BUNDLE>"}[best]
     else:
         kname = {"fp64": "fast_kernel<EK_CROSS>", "split3": "split_kernel<PR_CROSS>", "split2": "split_kernel<PR_CROSS>",
@@ -578,7 +578,7 @@ def _extra_configs(args, sf, torch, dev, world, rank, dist, local, stream):
             o = sf.product(sf.OP_CROSS, sets[0][0], sets[0][1], m_max_pad=pad, **kw)
             r["rel_l2_vs_cpu_port"] = R_rel_l2(H(o), ref)
         cfg["forms"][form] = r
-    cfg["roofline"] = roof(nbytes, cfg["forms"]["fp64"]["ms_per_step"], "fast_kernel<EK_CROSS, 16>")
+    cfg["roofline"] = roof(nbytes, cfg["forms"]["fp64"]["ms_per_step"], "solo_kernel<EK_CROSS, 2>")
     res["cross_28k"] = cfg
     del sets
 
@@ -597,7 +597,7 @@ def _extra_configs(args, sf, torch, dev, world, rank, dist, local, stream):
     cfg["jvp"] = {"ms_per_step": ms_j, "value": world * npts * m / (ms_j / 1e3)}
     cfg["vjp"] = {"ms_per_step": ms_t, "value": world * npts * m / (ms_t / 1e3)}
     cfg["roofline"] = {"jvp": roof(nbytes, ms_j, "fast_kernel<EK_CROSS2> (du x w + u x dw in one two-pass launch)"),
-                       "vjp": roof(nbytes, ms_t, "fast_kernel (VJP as two cross products)")}
+                       "vjp": roof(nbytes, ms_t, "chain_kernel<OP_CROSS_VJP> (both cross products in one launch)")}
     sf.cross_jvp(u, w, tan, m_max_pad=pad, out=jv)
     sf.cross_vjp(u, w, cot, m_max_pad=pad, out=jt)
     # full-size checks: central differences of the cross product (h = 1e-6) and <J v, c> = <v, J^T c>
@@ -661,8 +661,8 @@ def _extra_configs(args, sf, torch, dev, world, rank, dist, local, stream):
     except sf.SfnlError as e:
         cfg["split3"] = {"unavailable": str(e)}
     nb = 8.0 * m * npts * (18 + k * (18 + 12))
-    kname5 = ("large_res_coef_kernel<6> + large_syn_tf_kernel + large_prod_tf_kernel + large_res_out_kernel<6> "
-              "(six residue grids, tangents batched per launch)")
+    kname5 = ("coef_kernel<64, 12> + base_kernel<64> + prod_kernel<64> + out_kernel<64, 12> "
+              "(twelve residue grids of 64 angles, tangents batched per launch)")
     cfg["roofline"] = {"jvp": roof(nb, ms_j, kname5), "vjp": roof(nb, ms_t, kname5)}
     if cpu_on:
         n_s, kt = 500, 2

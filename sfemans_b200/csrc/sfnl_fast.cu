@@ -32,9 +32,10 @@
 // mode tiles in the analysis.  Elementary programs are cross (6 -> 3), dot
 // (6 -> 1), product (2 -> 1), scalar x vector (4 -> 3, FFT_SCALAR_VECT_DCL
 // pb = 1), tensor (6 -> 9, FFT_TENSOR_DCL) and the sum of two cross products
-// (12 -> 3, the JVP du x w + u x dw: two synthesis passes, one analysis); the
-// bundle (away from m = 64) and the transposed programs are sequences of
-// elementary launches on one stream.
+// (12 -> 3, the JVP du x w + u x dw: two synthesis passes, one analysis).  The
+// transposed programs, the linearised MHD pair and the bundle away from m = 64
+// run as one launch of chain_kernel up to m = 64; small m takes one warp per tile
+// (solo_kernel) and m > 64 the residue grids (sfnl_res.cu).
 #include <cuda_runtime.h>
 
 #include <cmath>

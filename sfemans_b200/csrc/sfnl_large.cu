@@ -1,5 +1,7 @@
 // sfnl_large.cu -- the FAST form's folded transforms for large m (SFNL_ALGO_FAST,
-// m up to 512), as two kernels that meet at the grid values.
+// m up to 512), as two kernels that meet at the grid values: the bundle, the tensor
+// and the conservative advection beyond the fused kernels (m ~ 100); the products and
+// the linearised programs take the residue grids of sfnl_res.cu from m = 65.
 //
 // Same grid, folds and DFT tables as the fused kernels of sfnl_fast.cu (the
 // exact truncated product of fft_parallel.F90:147-665 evaluated on an
