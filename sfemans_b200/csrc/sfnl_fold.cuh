@@ -253,8 +253,24 @@ struct ResTab {
   const double *tw = nullptr;
 };
 int get_residue_tables(int m, int N, int R, ResTab *out);
-// The library's device workspace of (stream, use), grown to `bytes` (sfnl_large.cu).
-int large_workspace(cudaStream_t st, size_t bytes, double **out, int use = 0);
+// The library's device workspace of (stream, use), held by one call from its construction until the call's last launch
+// is enqueued: another thread's call on the same stream neither enqueues between them nor frees the buffer
+// (sfnl_large.cu).
+class LargeWorkspace {
+ public:
+  struct Entry;
+  LargeWorkspace(cudaStream_t st, int use);
+  ~LargeWorkspace();
+  LargeWorkspace(const LargeWorkspace &) = delete;
+  LargeWorkspace &operator=(const LargeWorkspace &) = delete;
+  int get(size_t bytes, double **out);  // grows it; SFNL_ERR_ALLOC without memory, or while st is being captured
+
+ private:
+  Entry *e_;
+  cudaStream_t st_;
+  unsigned long long id_ = 0;
+  bool capturing_ = false, got_ = false;
+};
 // Residue grids of 128 angles with one program kernel (sfnl_res.cu); cap: bytes of workspace.
 bool res_supported(int op, int m);
 int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st);

@@ -522,32 +522,84 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32) large_prod_kernel(const 
   }
 }
 
-// workspaces, one per (device, stream, use): calls on different streams do not share them.  Use 0: the
-// grid values; 1: the residue coefficients and sums of launch_large_res.
-std::mutex g_lws_mu;
-std::map<std::tuple<int, cudaStream_t, int>, std::pair<double *, size_t>> g_lws;
-
 }  // namespace
 
-int large_workspace(cudaStream_t st, size_t bytes, double **out, int use) {
+// Workspaces, one per (device, stream handle, use): calls on different streams do not share them.  Use 0: the
+// grid values; 1: the residue coefficients and sums of launch_large_res; 2: launch_res.  They stay until
+// sfnl_finalize; a call holds its entry's lock while it enqueues (LargeWorkspace).
+struct LargeWorkspace::Entry {
+  std::mutex mu;
+  double *p = nullptr;
+  size_t bytes = 0;
+  cudaEvent_t done = nullptr;     // the last call's work
+  bool used = false;              // done is recorded
+  unsigned long long stream = 0;  // id of the stream it is recorded on
+};
+
+namespace {
+std::mutex g_lws_mu;  // the map; its entries are never erased
+std::map<std::tuple<int, cudaStream_t, int>, LargeWorkspace::Entry> g_lws;
+}  // namespace
+
+LargeWorkspace::LargeWorkspace(cudaStream_t st, int use) : st_(st) {
   int dev = 0;
   cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lk(g_lws_mu);
-  auto &w = g_lws[{dev, st, use}];
-  if (w.second < bytes) {
-    if (w.first) {
-      cudaStreamSynchronize(st);  // the previous call on this stream may still read it
-      cudaFree(w.first);
-    }
-    w.first = nullptr;
-    w.second = 0;
-    if (cudaMalloc(&w.first, bytes) != cudaSuccess) {
+  {
+    std::lock_guard<std::mutex> lk(g_lws_mu);
+    e_ = &g_lws[{dev, st, use}];
+  }
+  e_->mu.lock();
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  capturing_ = cap != cudaStreamCaptureStatusNone;
+  if (cudaStreamGetId(st, &id_) != cudaSuccess) cudaGetLastError();
+}
+
+LargeWorkspace::~LargeWorkspace() {
+  if (got_ && !capturing_) {
+    e_->used = cudaEventRecord(e_->done, st_) == cudaSuccess;
+    if (!e_->used) {  // nothing later could wait for this call's work
       cudaGetLastError();
+      cudaStreamSynchronize(st_);
+    }
+    e_->stream = id_;
+  }
+  e_->mu.unlock();
+}
+
+int LargeWorkspace::get(size_t bytes, double **out) {
+  Entry &e = *e_;
+  if (e.bytes < bytes) {
+    if (capturing_)
+      return set_error(SFNL_ERR_ALLOC, "the large-m workspace cannot be allocated while the stream is being captured");
+    if (e.p) {
+      cudaStreamSynchronize(st_);  // the previous call on this stream may still read it
+      if (e.used) cudaEventSynchronize(e.done);
+      cudaFree(e.p);
+    }
+    e.p = nullptr;
+    e.bytes = 0;
+    if (!e.done && cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      e.done = nullptr;
+      return set_error(SFNL_ERR_CUDA, "cudaEventCreate for the large-m workspace failed");
+    }
+    if (cudaMalloc(&e.p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      e.p = nullptr;
       return set_error(SFNL_ERR_ALLOC, "cudaMalloc of the large-m workspace failed");
     }
-    w.second = bytes;
+    e.bytes = bytes;
+    e.used = false;
   }
-  *out = w.first;
+  // One handle can name several streams: cudaStreamPerThread one of each thread, and a destroyed stream's handle a
+  // later one.  Work of another stream is waited for on the device.
+  if (!capturing_ && e.used && e.stream != id_ && cudaStreamWaitEvent(st_, e.done, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return set_error(SFNL_ERR_CUDA, "cudaStreamWaitEvent for the large-m workspace failed");
+  }
+  got_ = true;
+  *out = e.p;
   return SFNL_OK;
 }
 
@@ -654,15 +706,23 @@ constexpr int64_t kLargeMinChunk = 4096;
 void large_res_release_tables();
 
 void large_release_workspaces() {
-  std::lock_guard<std::mutex> lk(g_lws_mu);
+  std::vector<std::pair<int, LargeWorkspace::Entry *>> all;
+  {  // a call holds its entry while it looks up another one, so the map's lock is not held over the entries'
+    std::lock_guard<std::mutex> lk(g_lws_mu);
+    for (auto &kv : g_lws) all.push_back({std::get<0>(kv.first), &kv.second});
+  }
   int prev = 0;
   cudaGetDevice(&prev);
-  for (auto &kv : g_lws)
-    if (kv.second.first) {
-      cudaSetDevice(std::get<0>(kv.first));
-      cudaFree(kv.second.first);  // waits for the work still reading it
-    }
-  g_lws.clear();
+  for (auto &[dev, e] : all) {
+    std::lock_guard<std::mutex> lk(e->mu);
+    cudaSetDevice(dev);
+    if (e->p) cudaFree(e->p);  // waits for the work still reading it
+    if (e->done) cudaEventDestroy(e->done);
+    e->p = nullptr;
+    e->bytes = 0;
+    e->done = nullptr;
+    e->used = false;
+  }
   cudaSetDevice(prev);
   large_res_release_tables();
 }
@@ -719,7 +779,8 @@ int run_large(const ProgArgs &a, const Geo &g, const Tables &T, const LargePlan 
   if (chunk < 32) chunk = 32;
   if (chunk > a.np) chunk = ((a.np + 7) / 8) * 8;
   double *G = nullptr;
-  if (int rc = large_workspace(st, per_point * (size_t)chunk, &G)) return rc;
+  LargeWorkspace ws(st, 0);
+  if (int rc = ws.get(per_point * (size_t)chunk, &G)) return rc;
   // the third fold needs mirror pairs of angle tiles
   const int NT = rp ? rp->NT : g.NT, mt = rp ? rp->mt : g.m;
   const bool tf = NT % 2 == 0;
@@ -1072,7 +1133,8 @@ int launch_large_res(const ProgArgs &a, const Geo &g, int R, cudaStream_t st) {
   if (chunk < 32) chunk = 32;
   if (chunk > a.np) chunk = ((a.np + 7) / 8) * 8;
   double *W = nullptr;
-  if (int rc = large_workspace(st, per_point * (size_t)chunk, &W, 1)) return rc;
+  LargeWorkspace ws(st, 1);
+  if (int rc = ws.get(per_point * (size_t)chunk, &W)) return rc;
   const bool adj_out = op_adjoint_out(a.op);
   const double invN = 1.0 / N, w = adj_out ? 1.0 : 2.0 * invN, w0 = adj_out ? 1.0 : invN;
   constexpr int kThreads = 256;

@@ -528,7 +528,8 @@ int launch_res_m(const ProgArgs &a, size_t cap, cudaStream_t st) {
   const int64_t chunks = (a.np + chunk - 1) / chunk;  // of equal length
   chunk = ((a.np + chunks - 1) / chunks + 7) / 8 * 8;
   double *W = nullptr;
-  if (int rc = large_workspace(st, (size_t)chunk * (shared_b + kb * entry_b), &W, 2)) return rc;
+  LargeWorkspace ws(st, 2);
+  if (int rc = ws.get((size_t)chunk * (shared_b + kb * entry_b), &W)) return rc;
   const bool adj_out = op_adjoint_out(a.op);
   for (int64_t c0 = 0; c0 < a.np; c0 += chunk)
     for (int b0 = 0; b0 < a.batch; b0 += (int)kb) {
