@@ -539,6 +539,14 @@ struct LargeWorkspace::Entry {
 namespace {
 std::mutex g_lws_mu;  // the map; its entries are never erased
 std::map<std::tuple<int, cudaStream_t, int>, LargeWorkspace::Entry> g_lws;
+
+// Allocating and freeing are refused, and end the capture, while another thread captures a graph in the default mode,
+// unless this thread's mode is relaxed; neither touches that capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 }  // namespace
 
 LargeWorkspace::LargeWorkspace(cudaStream_t st, int use) : st_(st) {
@@ -572,6 +580,7 @@ int LargeWorkspace::get(size_t bytes, double **out) {
   if (e.bytes < bytes) {
     if (capturing_)
       return set_error(SFNL_ERR_ALLOC, "the large-m workspace cannot be allocated while the stream is being captured");
+    RelaxedCapture relaxed;
     if (e.p) {
       cudaStreamSynchronize(st_);  // the previous call on this stream may still read it
       if (e.used) cudaEventSynchronize(e.done);

@@ -62,3 +62,34 @@ def test_two_threads(stream, first, second):
     assert not errors
     for _, want, outs in problems:
         assert all(torch.equal(out, want) for out in outs)
+
+
+@pytest.mark.parametrize("m", [72, 200])
+def test_a_capture_in_another_thread_goes_on(m):
+    # a first and a growing call allocate their workspace while another thread captures a graph on its own stream
+    torch = pytest.importorskip("torch")
+    pad, sizes = (3 * m + 1) // 2, (150, 900)
+    f = [[sf.to_device(R.synthetic_field(n, 6, m, 0.05, 7 + i)) for i in range(2)] for n in sizes]
+    wants = [sf.product(sf.OP_CROSS, *ab, m_max_pad=pad, stream=0) for ab in f]
+    outs, side, errors = [torch.empty_like(w) for w in wants], torch.cuda.Stream(), []
+    x = torch.ones(64, device="cuda")
+    torch.cuda.synchronize()
+
+    def work():
+        try:
+            for (a, b), out in zip(f, outs):
+                sf.product(sf.OP_CROSS, a, b, out=out, m_max_pad=pad, stream=side)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x.mul_(2.0)
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+        x.add_(1.0)
+    g.replay()
+    torch.cuda.synchronize()
+    assert not errors and bool((x == 3.0).all())
+    assert all(torch.equal(o, w) for o, w in zip(outs, wants))
