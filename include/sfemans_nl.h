@@ -38,8 +38,19 @@
  *
  * Threading: entry points are thread-safe; work is enqueued on the stream
  * passed in (NULL = the legacy default stream) and the device-pointer entry
- * points return without synchronising.  The *_host entry points take host
+ * points return without synchronising, but for a call that grows a workspace
+ * (below), which waits for its stream.  The *_host entry points take host
  * arrays, copy them in and out, and return after the result is on the host.
+ *
+ * Workspaces: from m = 65 the FAST form of the cross, dot and scalar products,
+ * of scalar x vector and of the linearised programs (the cross JVP from m = 73)
+ * works through a device buffer of its stream, up to 2 GiB and at most a
+ * quarter of the free memory, kept until sfnl_finalize.  Up to m = 107 a call
+ * that is being captured into a graph, or needs more than that share, runs
+ * without it.  Beyond, shorter runs of points go through a smaller buffer, and a
+ * capture needs a call of the same size on its stream before it.  The bundle and
+ * the advection beyond m = 107 and the tensor beyond m = 86 have buffers of their
+ * own, from 1 GiB up to a quarter of the free memory.
  */
 #ifndef SFEMANS_NL_H
 #define SFEMANS_NL_H
@@ -243,11 +254,9 @@ int sfnl_gauss_operands_f64(int kind, const double *v, const double *v2, const d
  *   VJP  cot (np, 6, m, k) -> out (np, 12, m, k) = J^T cot, the transpose for the
  *        plain Euclidean inner product of the coefficient arrays, so that
  *        <J v, c> = <v, J^T c> exactly in exact arithmetic.
- * u, w: (np, 6, m) shared by all k_batch tangents.  From m = 65 (the residue
- * grids; the cross JVP from m = 73) the base state is synthesised once per point
- * chunk and the tangents in one launch per chunk, through a workspace of up to
- * 2 GiB per stream (kept until sfnl_finalize).  Up to m about 100 a call that is
- * being captured, or finds no memory for it, runs without the workspace.
+ * u, w: (np, 6, m) shared by all k_batch tangents.  From m = 65 (the cross JVP
+ * from m = 73) the base state is synthesised once per point chunk and the
+ * tangents in one launch per chunk, through the stream's workspace.
  * ------------------------------------------------------------------------- */
 int sfnl_cross_jvp_f64(const double *u, const double *w, const double *tan, double *out, int64_t np, int m_max,
                        int m_max_pad, int k_batch, sfnl_stream_t stream);

@@ -263,6 +263,7 @@ class LargeWorkspace {
   ~LargeWorkspace();
   LargeWorkspace(const LargeWorkspace &) = delete;
   LargeWorkspace &operator=(const LargeWorkspace &) = delete;
+  size_t share(size_t bytes) const;     // bytes if it holds them, else what it may grow to: a quarter of the free memory
   int get(size_t bytes, double **out);  // grows it; SFNL_ERR_ALLOC without memory, or while st is being captured
 
  private:

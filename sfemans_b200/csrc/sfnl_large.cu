@@ -575,6 +575,19 @@ LargeWorkspace::~LargeWorkspace() {
   e_->mu.unlock();
 }
 
+// The memory is also the caller's (an allocator of its own beside this library): a workspace takes at most a quarter of
+// what is free, its own bytes counted in.
+size_t LargeWorkspace::share(size_t bytes) const {
+  if (e_->bytes >= bytes) return bytes;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return bytes;
+  }
+  const size_t quarter = (free_b + e_->bytes) / 4;
+  return quarter > e_->bytes ? quarter : e_->bytes;
+}
+
 int LargeWorkspace::get(size_t bytes, double **out) {
   Entry &e = *e_;
   if (e.bytes < bytes) {

@@ -509,6 +509,7 @@ bool res_supported(int op, int m) {
 }
 
 namespace {
+constexpr size_t kResMinBytes = size_t(32) << 20;
 // Points and batch entries go in chunks whose coefficients, base values and sums fit `cap` bytes of workspace.
 template <int M>
 int launch_res_m(const ProgArgs &a, size_t cap, cudaStream_t st) {
@@ -521,15 +522,33 @@ int launch_res_m(const ProgArgs &a, size_t cap, cudaStream_t st) {
   if (int rc = get_residue_tables(m, N, R, &T)) return rc;
   // doubles per point: N for a field's coefficients, grid values or an output's sums
   const size_t shared_b = sizeof(double) * (size_t)N * 2 * nsh, entry_b = sizeof(double) * (size_t)N * (own + no);
-  int64_t kb = (int64_t)((cap / 64 - shared_b) / entry_b);  // at least 64 points at a time where the cap allows
-  kb = cap / 64 <= shared_b || kb < 1 ? 1 : kb > a.batch ? a.batch : kb;
-  int64_t chunk = (int64_t)(cap / (shared_b + kb * entry_b)) / 8 * 8;
-  chunk = chunk < 8 ? 8 : chunk;
-  const int64_t chunks = (a.np + chunk - 1) / chunk;  // of equal length
-  chunk = ((a.np + chunks - 1) / chunks + 7) / 8 * 8;
-  double *W = nullptr;
+  int64_t kb = 0, chunk = 0;
+  size_t bytes = 0;
+  auto plan = [&](size_t room) {
+    kb = (int64_t)((room / 64 - shared_b) / entry_b);  // at least 64 points at a time where the room allows
+    kb = room / 64 <= shared_b || kb < 1 ? 1 : kb > a.batch ? a.batch : kb;
+    chunk = (int64_t)(room / (shared_b + kb * entry_b)) / 8 * 8;
+    chunk = chunk < 8 ? 8 : chunk;
+    const int64_t chunks = (a.np + chunk - 1) / chunk;  // of equal length
+    chunk = ((a.np + chunks - 1) / chunks + 7) / 8 * 8;
+    bytes = (size_t)chunk * (shared_b + kb * entry_b);
+  };
+  plan(cap);
   LargeWorkspace ws(st, 2);
-  if (int rc = ws.get((size_t)chunk * (shared_b + kb * entry_b), &W)) return rc;
+  // Where the fused kernels fit, a call that needs more than the share of the free memory leaves it to them; beyond, the
+  // points go in shorter chunks, down to kResMinBytes, while there is no memory for longer ones.
+  const bool fused = fast_fused_fits(a.op, a.m);
+  if (const size_t share = ws.share(bytes); share < bytes) {
+    if (fused) return set_error(SFNL_ERR_ALLOC, "residue grids: little free memory");
+    plan(share > kResMinBytes ? share : kResMinBytes);
+  }
+  double *W = nullptr;
+  int rc = ws.get(bytes, &W);
+  while (rc == SFNL_ERR_ALLOC && !fused && bytes > kResMinBytes) {
+    plan(bytes / 2);
+    rc = ws.get(bytes, &W);
+  }
+  if (rc) return rc;
   const bool adj_out = op_adjoint_out(a.op);
   for (int64_t c0 = 0; c0 < a.np; c0 += chunk)
     for (int b0 = 0; b0 < a.batch; b0 += (int)kb) {
@@ -563,10 +582,9 @@ int launch_res_m(const ProgArgs &a, size_t cap, cudaStream_t st) {
       for (int f = 0; f < ni; ++f) pa.inst[f] = ca.inst[f];
       pa.nshared = nsh;
       pa.nb = nb;
-      if (int rc = launch_passes<M>(R, &ca, nullptr, st)) return rc;
+      if (rc = launch_passes<M>(R, &ca, nullptr, st)) return rc;
       if (lin)
-        if (int rc = launch_base<M>(pa, R, st)) return rc;
-      int rc = SFNL_OK;
+        if (rc = launch_base<M>(pa, R, st)) return rc;
       switch (a.op) {
         case OP_CROSS: rc = launch_prod<OP_CROSS, M>(pa, R, st); break;
         case OP_DOT: rc = launch_prod<OP_DOT, M>(pa, R, st); break;
@@ -597,7 +615,7 @@ int launch_res_m(const ProgArgs &a, size_t cap, cudaStream_t st) {
         oa.ldm[o] = a.out_ldm[o];
         oa.bs[o] = a.out_bs[o];
       }
-      if (int rc2 = launch_passes<M>(R, nullptr, &oa, st)) return rc2;
+      if (rc = launch_passes<M>(R, nullptr, &oa, st)) return rc;
     }
   return SFNL_OK;
 }

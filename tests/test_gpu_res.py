@@ -77,3 +77,31 @@ def test_captured_calls_without_a_workspace(m):
     torch.cuda.synchronize()
     for o, e in zip(outs, eager):
         assert R.rel_l2(sf.to_host(o), sf.to_host(e)) <= TOL
+
+
+def test_a_workspace_leaves_memory_to_the_caller():
+    # with 4 GiB free the buffer may take a quarter: at m = 72 the fused kernels run instead, at m = 200 shorter chunks
+    torch = pytest.importorskip("torch")
+    G = 1 << 30
+    u, w, b = (sf.to_device(_field(7000, 6, 72, 81 + i)) for i in range(3))
+    cot = sf.to_device(np.stack([_field(7000, 12, 72, 85 + i) for i in range(4)], -1))
+    x, y = (sf.to_device(_field(30_000, 6, 200, 91 + i)) for i in range(2))
+    calls = [lambda out: sf.mhd_vjp(u, w, b, cot, m_max_pad=_pad(72), out=out),
+             lambda out: sf.product(sf.OP_CROSS, x, y, m_max_pad=_pad(200), out=out)]
+    outs = [sf.fortran_empty(7000, 18, 72, 4), sf.fortran_empty(30_000, 6, 200)]
+    wants = [f(torch.empty_like(o)) for f, o in zip(calls, outs)]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    sf.lib().sfnl_finalize()
+    for f, o in zip(calls, outs):  # tables and kernels are loaded; small calls, small buffers
+        f(o)
+    torch.cuda.synchronize()
+    sf.lib().sfnl_finalize()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - 4 * G, dtype=torch.uint8, device="cuda")
+    for f, o, w_, most in zip(calls, outs, wants, (G // 8, G + G // 8)):  # tables of a few MB beside the buffer
+        before = torch.cuda.mem_get_info()[0]
+        f(o.zero_())
+        torch.cuda.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] <= most
+        assert float((o - w_).norm() / w_.norm()) <= TOL
+    del filler
