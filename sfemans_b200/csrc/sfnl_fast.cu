@@ -1793,8 +1793,10 @@ int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
   // every (KS, NT) of make_geo up to m = 64; run-time loops cost the sizes between 16, 32 and 64 a third of their time
   // (cross product, 50,001 points: m = 20 99 -> 62 us, m = 40 207 -> 148, m = 48 337 -> 202, m = 52 384 -> 229)
   if constexpr (ADJ != 0) {  // transposed products: chain_kernel takes the other sizes up to m = 64
-    if (fa.NT == 6 && fa.KS[0] == 7) return launch_ek_m<EK, 7, 6, ADJ>(fa, batch, st);
-    if (fa.NT == 6 && fa.KS[0] == 8) return launch_ek_m<EK, 8, 6, ADJ>(fa, batch, st);
+    if constexpr (ek_passes(EK) == 1) {
+      if (fa.NT == 6 && fa.KS[0] == 7) return launch_ek_m<EK, 7, 6, ADJ>(fa, batch, st);
+      if (fa.NT == 6 && fa.KS[0] == 8) return launch_ek_m<EK, 8, 6, ADJ>(fa, batch, st);
+    }
     return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);  // m > 64 without a workspace
   } else {
   switch (10 * fa.KS[0] + fa.NT) {
@@ -1817,7 +1819,11 @@ int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
 
 template <int EK>
 int launch_ek(FastArgs &fa, int batch, cudaStream_t st) {
-  if constexpr (EK == EK_CROSS) {
+  if constexpr (ek_passes(EK) == 2) {  // the cotangents' fields among the 12 staged ones (pass 0: 0-5, pass 1: 6-11)
+    if (fa.adj_in == 0u) return launch_ek_adj<EK, 0>(fa, batch, st);
+    if (fa.adj_in == 0xE38u) return launch_ek_adj<EK, 2>(fa, batch, st);  // second operand of both passes
+    return set_error(SFNL_ERR_ARG, "FAST form: unsupported cotangent operands");
+  } else if constexpr (EK == EK_CROSS) {
     if (fa.adj_in == 0x07u) return launch_ek_adj<EK, 1>(fa, batch, st);
     if (fa.adj_in == 0x38u) return launch_ek_adj<EK, 2>(fa, batch, st);
     if (fa.adj_in != 0u) return set_error(SFNL_ERR_ARG, "FAST form: unsupported cotangent operand");
@@ -1882,14 +1888,23 @@ int decompose_program(int op, std::vector<Elem> &seq, bool fuse) {
       add(EK_CROSS, {6, 7, 8, 0, 1, 2}, {3, 4, 5}, A0, 0);    // c x u
       break;
     case OP_MHD_JVP:  // [u, w, b, du, dw, db]
+      if (fuse) {
+        add(EK_CROSS2, {9, 10, 11, 3, 4, 5, 0, 1, 2, 12, 13, 14}, {0, 1, 2}, 0, 0);  // du x w + u x dw
+        add(EK_CROSS2, {9, 10, 11, 6, 7, 8, 0, 1, 2, 15, 16, 17}, {3, 4, 5}, 0, 0);  // du x b + u x db
+        break;
+      }
       add(EK_CROSS, {9, 10, 11, 3, 4, 5}, {0, 1, 2}, 0, 0);   // du x w
       add(EK_CROSS, {0, 1, 2, 12, 13, 14}, {0, 1, 2}, 0, 1);  // + u x dw
       add(EK_CROSS, {9, 10, 11, 6, 7, 8}, {3, 4, 5}, 0, 0);   // du x b
       add(EK_CROSS, {0, 1, 2, 15, 16, 17}, {3, 4, 5}, 0, 1);  // + u x db
       break;
     case OP_MHD_VJP:  // [u, w, b, c1, c2]
-      add(EK_CROSS, {3, 4, 5, 9, 10, 11}, {0, 1, 2}, A1, 0);  // w x c1
-      add(EK_CROSS, {6, 7, 8, 12, 13, 14}, {0, 1, 2}, A1, 1); // + b x c2
+      if (fuse) {  // both passes' second operands are cotangents
+        add(EK_CROSS2, {3, 4, 5, 9, 10, 11, 6, 7, 8, 12, 13, 14}, {0, 1, 2}, A1 | A1 << 6, 0);  // w x c1 + b x c2
+      } else {
+        add(EK_CROSS, {3, 4, 5, 9, 10, 11}, {0, 1, 2}, A1, 0);  // w x c1
+        add(EK_CROSS, {6, 7, 8, 12, 13, 14}, {0, 1, 2}, A1, 1); // + b x c2
+      }
       add(EK_CROSS, {9, 10, 11, 0, 1, 2}, {3, 4, 5}, A0, 0);  // c1 x u
       add(EK_CROSS, {12, 13, 14, 0, 1, 2}, {6, 7, 8}, A0, 0); // c2 x u
       break;
@@ -2181,9 +2196,11 @@ int launch_fast(const ProgArgs &a, cudaStream_t st) {
     }
   }
   std::vector<Elem> seq;
-  // the linearised cross product as one two-pass program (the output written once, one analysis): 1.7x faster than
-  // two launches at m = 32 (700k points: 3.26 -> 1.92 ms) and 1.25x at m = 64 (200k points, 4 tangents: 8.40 -> 6.70
-  // ms); where its products cannot overlay its coefficients (more than 8 angle tiles, m > 85) two launches.
+  // the sums of two cross products in the linearised programs as one two-pass program each (the output written once,
+  // one analysis): cross product's JVP 1.7x faster than two launches at m = 32 (700k points: 3.26 -> 1.92 ms) and 1.25x
+  // at m = 64 (200k points, 4 tangents: 8.40 -> 6.70 ms); the MHD pair, 6,000 points, m = 72, JVP 0.471 -> 0.257 ms,
+  // VJP 0.476 -> 0.353.  Where the products cannot overlay the coefficients (more than 8 angle tiles, m > 86) launches
+  // of one product each.
   rc = decompose_program(a.op, seq, fast_overlay(EK_CROSS2, g.NT, 4 * g.KS_tot));
   if (rc) return rc;
   const bool adj_out = op_adjoint_out(a.op);

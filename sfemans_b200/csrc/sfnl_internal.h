@@ -108,7 +108,7 @@ struct Elem {
   unsigned adj;  // bit f: operand f is a cotangent (synthesised with the analysis weights)
   int acc;       // 1: add to the output instead of overwriting it
 };
-// fuse: the cross product's JVP as one EK_CROSS2 program instead of two launches.
+// fuse: the sums of two cross products of the linearised programs as one EK_CROSS2 program instead of two launches.
 int decompose_program(int op, std::vector<Elem> &seq, bool fuse);  // sfnl_fast.cu
 bool split_supported(int op, int m);                    // sfnl_split.cu
 

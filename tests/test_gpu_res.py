@@ -105,3 +105,27 @@ def test_a_workspace_leaves_memory_to_the_caller():
         assert before - torch.cuda.mem_get_info()[0] <= most
         assert float((o - w_).norm() / w_.norm()) <= TOL
     del filler
+
+
+@pytest.mark.parametrize("kind,nbase,nin,nout,launches", [("cross_jvp", 2, 12, 6, (1, 2)), ("cross_vjp", 2, 6, 12, (2, 2)),
+                                                          ("mhd_jvp", 3, 18, 12, (2, 4)), ("mhd_vjp", 3, 12, 18, (3, 4))])
+@pytest.mark.parametrize("m", [73, 86, 87, 107])
+def test_captured_linearised_programs(m, kind, nbase, nin, nout, launches):
+    # to m = 86 a sum of two cross products is one launch of a captured call, beyond two
+    torch = pytest.importorskip("torch")
+    cudart = pytest.importorskip("cuda.bindings.runtime")
+    npts, k = 13, 2
+    f = [sf.to_device(_field(npts, 6, m, 61 + i)) for i in range(nbase)]
+    x = sf.to_device(np.stack([_field(npts, nin, m, 71 + i) for i in range(k)], -1))
+    call = lambda out: getattr(sf, kind)(*f, x, m_max_pad=_pad(m), out=out)  # noqa: E731
+    want, out = call(sf.fortran_empty(npts, nout, m, k)), sf.fortran_empty(npts, nout, m, k)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        call(out)
+    err, _, count = cudart.cudaGraphGetNodes(g.raw_cuda_graph(), 0)
+    assert int(err) == 0 and count == launches[m > 86]
+    g.instantiate()
+    g.replay()
+    torch.cuda.synchronize()
+    assert R.rel_l2(sf.to_host(out), sf.to_host(want)) <= TOL
