@@ -455,25 +455,36 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
         }
       }
     } else {  // run-time geometry: fields outermost (measured faster there)
+      // The rows' alignment is a constant of the loops: tested in each row it cost 2 to 6 % of the tile's time (cross
+      // product's JVP, 14,000 points, m = 80 0.395 -> 0.411 ms).
+      auto rows = [&](auto wide_tag) {
+        constexpr int WIDE = decltype(wide_tag)::value;
 #pragma unroll
-      for (int f = 0; f < NI; ++f) {
-        const double *base = a.in[f] + (int64_t)b * a.in_bs[f] + p0 + pc;
-        const int64_t ldm = a.in_ldm[f];
-        double *xf = xs + (size_t)f * KS_tot * 32;
-        for (int r = threadIdx.x >> 2; r < KT; r += rstep) {
-          const int c = (r >= 4 * KOFF[1]) + (r >= 4 * KOFF[2]) + (r >= 4 * KOFF[3]);
-          const int k = r - 4 * sel4(KOFF, c), n = class_mode(c, k);
-          double *dst = xf + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
-          const bool live = k < sel4(KE, c) && !(c == 2 && n == 0);  // the sine of mode 0 is ignored
-          const double *src = base + (int64_t)n * ldm + (c >= 2 ? a.np : 0);
-          if (live && ((v16 >> (c >= 2)) & 1)) {
-            cp_async16(dst, src);
-          } else {
-            if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
-            if (live && pv1) cp_async8(dst + 1, src + 1); else dst[1] = 0.0;
+        for (int f = 0; f < NI; ++f) {
+          const double *base = a.in[f] + (int64_t)b * a.in_bs[f] + p0 + pc;
+          const int64_t ldm = a.in_ldm[f];
+          double *xf = xs + (size_t)f * KS_tot * 32;
+          for (int r = threadIdx.x >> 2; r < KT; r += rstep) {
+            const int c = (r >= 4 * KOFF[1]) + (r >= 4 * KOFF[2]) + (r >= 4 * KOFF[3]);
+            const int k = r - 4 * sel4(KOFF, c), n = class_mode(c, k);
+            double *dst = xf + (size_t)(r >> 2) * 32 + a_frag_slot(r & 3, pc);
+            const bool live = k < sel4(KE, c) && !(c == 2 && n == 0);  // the sine of mode 0 is ignored
+            const double *src = base + (int64_t)n * ldm + (c >= 2 ? a.np : 0);
+            if (live && (WIDE == 3 || (WIDE == 1 && c < 2))) {
+              cp_async16(dst, src);
+            } else {
+              if (live && pv0) cp_async8(dst, src); else dst[0] = 0.0;
+              if (live && pv1) cp_async8(dst + 1, src + 1); else dst[1] = 0.0;
+            }
           }
         }
-      }
+      };
+      if (v16 == 3)
+        rows(std::integral_constant<int, 3>{});
+      else if (v16 == 1)
+        rows(std::integral_constant<int, 1>{});
+      else
+        rows(std::integral_constant<int, 0>{});
     }
   }
   cp_async_wait_all();
