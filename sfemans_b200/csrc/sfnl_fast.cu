@@ -726,17 +726,20 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
 // folded products of an angle tile go from the registers of the lane that formed them straight into the analysis
 // as A fragments and no warp waits for another.
 // The two-warp CTAs of fast_kernel ran copy, synthesis, products and analysis one after the other with barriers
-// between (DMMA pipe 31 % busy at m = 16).  Programs with one output fit up to m = 32.  Every class takes KSC k-steps
+// between (DMMA pipe 31 % busy at m = 16).  Programs with one output fit up to m = 32.
+// Every class takes KSC k-steps
 // and NUC output tiles, also where the odd one needs fewer (zero coefficients; results not stored), so that no
 // branch keeps the loads of the table fragments from running ahead (with the branches the cross product at m = 16 took
 // 33 us).  One buffer and three CTAs of four warps per SM beat two buffers and two CTAs (22.2 against 23.7 us per call
 // with the host's share): the next tile's copies start when the last angle tile's coefficients are read.  Measured on
 // a B200 against fast_kernel: cross product, 28,000 points, m = 16 26.6 -> 24.6 us; 50,001 points, m = 10 50 -> 30 us;
-// product of scalars, 100,000 points, m = 8 32 -> 19 us; dot product, 50,001 points, m = 24 114 -> 69 us.  Three
-// outputs at m = 17..32 need 255 registers (two CTAs) and were slower than fast_kernel (m = 32: 192 against 160 us).
+// product of scalars, 100,000 points, m = 8 32 -> 19 us; dot product, 60,000 points, m = 24 66 -> 61 us.  Three
+// outputs at m = 17..32 need 255 registers (two CTAs) and were slower than fast_kernel (m = 32: 192 against 160 us), and
+// so was the dot product at m = 25..32, whose tile is the longest (m = 32, 3,000 points 9.7 against 12.5 us, 14,000
+// points 22.8 against 26.9, 100,000 points 134.8 against 136.4).
 constexpr int kSoloWarps = 4;
 // Largest k-steps per class (KSC; the analysis has NUC = (KSC + 1) / 2 output tiles of 8 per class).
-constexpr int solo_max_ks(int ek) { return ek_nout(ek) == 1 ? 4 : 2; }
+constexpr int solo_max_ks(int ek) { return ek == EK_PROD ? 4 : ek == EK_DOT ? 3 : 2; }
 constexpr bool solo_ek(int ek) { return ek == EK_CROSS || ek == EK_DOT || ek == EK_PROD || ek == EK_SVECT; }
 constexpr size_t solo_smem_bytes(int ek, int KSC) { return sizeof(double) * (size_t)kSoloWarps * ek_nin(ek) * 4 * KSC * 32; }
 
@@ -1796,10 +1799,10 @@ int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
   if constexpr (solo_ek(EK) && ADJ == 0) {
     if (fa.KS[0] == 1) return launch_solo<EK, 1>(fa, batch, st);
     if (fa.KS[0] == 2) return launch_solo<EK, 2>(fa, batch, st);
-    if constexpr (solo_max_ks(EK) == 4) {
+    if constexpr (solo_max_ks(EK) >= 3)
       if (fa.KS[0] == 3) return launch_solo<EK, 3>(fa, batch, st);
+    if constexpr (solo_max_ks(EK) >= 4)
       if (fa.KS[0] == 4) return launch_solo<EK, 4>(fa, batch, st);
-    }
   }
   // every (KS, NT) of make_geo up to m = 64; run-time loops cost the sizes between 16, 32 and 64 a third of their time
   // (cross product, 50,001 points: m = 20 99 -> 62 us, m = 40 207 -> 148, m = 48 337 -> 202, m = 52 384 -> 229)
