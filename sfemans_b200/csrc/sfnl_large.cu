@@ -531,9 +531,10 @@ struct LargeWorkspace::Entry {
   std::mutex mu;
   double *p = nullptr;
   size_t bytes = 0;
-  cudaEvent_t done = nullptr;     // the last call's work
+  unsigned long long stream = 0;  // id of the last call's stream
+  cudaEvent_t done = nullptr;     // cudaStreamPerThread: the last call's work
   bool used = false;              // done is recorded
-  unsigned long long stream = 0;  // id of the stream it is recorded on
+  std::vector<double *> retired;  // freed with the others
 };
 
 namespace {
@@ -564,13 +565,12 @@ LargeWorkspace::LargeWorkspace(cudaStream_t st, int use) : st_(st) {
 }
 
 LargeWorkspace::~LargeWorkspace() {
-  if (got_ && !capturing_) {
+  if (got_ && !capturing_ && st_ == cudaStreamPerThread) {
     e_->used = cudaEventRecord(e_->done, st_) == cudaSuccess;
     if (!e_->used) {  // nothing later could wait for this call's work
       cudaGetLastError();
       cudaStreamSynchronize(st_);
     }
-    e_->stream = id_;
   }
   e_->mu.unlock();
 }
@@ -590,6 +590,19 @@ size_t LargeWorkspace::share(size_t bytes) const {
 
 int LargeWorkspace::get(size_t bytes, double **out) {
   Entry &e = *e_;
+  // One handle can name several streams: cudaStreamPerThread one of each thread, where the last call's work is waited for
+  // on the device, and a destroyed stream's handle a later one, whose first call waits for all work (an event of every
+  // call would cost 1 us of a small one's 13) or, during a capture elsewhere, leaves the old buffer be.
+  const bool other = e.p && !capturing_ && e.stream != id_, per_thread = st_ == cudaStreamPerThread;
+  if (other && !per_thread) {
+    RelaxedCapture relaxed;
+    if (cudaDeviceSynchronize() != cudaSuccess) {
+      cudaGetLastError();
+      e.retired.push_back(e.p);
+      e.p = nullptr;
+      e.bytes = 0;
+    }
+  }
   if (e.bytes < bytes) {
     if (capturing_)
       return set_error(SFNL_ERR_ALLOC, "the large-m workspace cannot be allocated while the stream is being captured");
@@ -601,7 +614,8 @@ int LargeWorkspace::get(size_t bytes, double **out) {
     }
     e.p = nullptr;
     e.bytes = 0;
-    if (!e.done && cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming) != cudaSuccess) {
+    e.used = false;
+    if (per_thread && !e.done && cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
       e.done = nullptr;
       return set_error(SFNL_ERR_CUDA, "cudaEventCreate for the large-m workspace failed");
@@ -612,14 +626,11 @@ int LargeWorkspace::get(size_t bytes, double **out) {
       return set_error(SFNL_ERR_ALLOC, "cudaMalloc of the large-m workspace failed");
     }
     e.bytes = bytes;
-    e.used = false;
-  }
-  // One handle can name several streams: cudaStreamPerThread one of each thread, and a destroyed stream's handle a
-  // later one.  Work of another stream is waited for on the device.
-  if (!capturing_ && e.used && e.stream != id_ && cudaStreamWaitEvent(st_, e.done, 0) != cudaSuccess) {
+  } else if (other && e.used && cudaStreamWaitEvent(st_, e.done, 0) != cudaSuccess) {
     cudaGetLastError();
     return set_error(SFNL_ERR_CUDA, "cudaStreamWaitEvent for the large-m workspace failed");
   }
+  if (!capturing_) e.stream = id_;
   got_ = true;
   *out = e.p;
   return SFNL_OK;
@@ -739,6 +750,8 @@ void large_release_workspaces() {
     std::lock_guard<std::mutex> lk(e->mu);
     cudaSetDevice(dev);
     if (e->p) cudaFree(e->p);  // waits for the work still reading it
+    for (double *p : e->retired) cudaFree(p);
+    e->retired.clear();
     if (e->done) cudaEventDestroy(e->done);
     e->p = nullptr;
     e->bytes = 0;

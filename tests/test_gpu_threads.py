@@ -93,3 +93,22 @@ def test_a_capture_in_another_thread_goes_on(m):
     torch.cuda.synchronize()
     assert not errors and bool((x == 3.0).all())
     assert all(torch.equal(o, w) for o, w in zip(outs, wants))
+
+
+def test_a_new_stream_with_an_old_handle():
+    # streams made and destroyed one after the other, their work still pending, mostly share one handle
+    torch = pytest.importorskip("torch")
+    cudart = pytest.importorskip("cuda.bindings.runtime")
+    (a, b), (c, d) = ([sf.to_device(R.synthetic_field(n, 6, 72, 0.05, n + i)) for i in range(2)] for n in (4000, 700))
+    wants = [sf.product(sf.OP_CROSS, x, y, m_max_pad=108, stream=0) for x, y in ((a, b), (c, d))]
+    outs = [[torch.empty_like(w) for _ in range(20)] for w in wants]
+    torch.cuda.synchronize()
+    for pair in zip(*outs):
+        for (x, y), out in zip(((a, b), (c, d)), pair):
+            err, st = cudart.cudaStreamCreateWithFlags(1)  # not blocking
+            assert int(err) == 0
+            sf.product(sf.OP_CROSS, x, y, out=out, m_max_pad=108, stream=int(st))
+            assert int(cudart.cudaStreamDestroy(st)[0]) == 0
+    torch.cuda.synchronize()
+    for want, group in zip(wants, outs):
+        assert all(torch.equal(out, want) for out in group)
