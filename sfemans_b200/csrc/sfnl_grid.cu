@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(256, op_nin(OP) <= 6 ? 2 : 1) mirror_kernel(co
                                                                               const int vec16) {
   constexpr int NI = op_nin(OP), NO = op_nout(OP);
   constexpr unsigned ADJ = OP == OP_CROSS_VJP ? 0x1C0u : OP == OP_MHD_VJP ? 0x7E00u : 0u;
+  constexpr int PAD = OP == OP_DIV || OP == OP_SVDIV || OP == OP_TENSION;
   extern __shared__ __align__(16) double smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
   const int gg = lane >> 2, q = lane & 3, b = blockIdx.y;
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(256, op_nin(OP) <= 6 ? 2 : 1) mirror_kernel(co
   auto in = [&](int f) { return a.in[f] + (int64_t)b * a.in_bs[f]; };
   auto ldm = [&](int f) { return a.in_ldm[f]; };
   const int64_t tiles = (a.np + 8 * g.PT - 1) / (8 * g.PT);
-  mirror_stage<NI>(xs, g, in, ldm, (int64_t)blockIdx.x * 8 * g.PT, a.np, vec16);
+  mirror_stage<NI, PAD>(xs, g, in, ldm, (int64_t)blockIdx.x * 8 * g.PT, a.np, vec16);
   mirror_table(ctab, stab, g.N);
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int64_t p0 = tile * 8 * g.PT;
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(256, op_nin(OP) <= 6 ? 2 : 1) mirror_kernel(co
     }
     __syncthreads();
     if (tile + gridDim.x < tiles)
-      mirror_stage<NI>(xs, g, in, ldm, (tile + gridDim.x) * 8 * g.PT, a.np, vec16);
+      mirror_stage<NI, PAD>(xs, g, in, ldm, (tile + gridDim.x) * 8 * g.PT, a.np, vec16);
     for (int it = warp; it < PG * 2 * NU; it += NW) {
       const int u = it % NU, c = (it / NU) & 1, pg = it / (2 * NU);
       constexpr int PC = NO * PW >= 9 ? 1 : 2;  // independent partial sums per output

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
   auto in = [&](int f) { return v + (int64_t)2 * (f0 + f) * np; };
   auto ldm = [&](int) { return (int64_t)nslot * np; };
   const int64_t tiles = (np + pts - 1) / pts;
-  mirror_stage<NI>(xs, g, in, ldm, (int64_t)blockIdx.x * pts, np, vec16);
+  mirror_stage<NI, 0>(xs, g, in, ldm, (int64_t)blockIdx.x * pts, np, vec16);
   mirror_table(ctab, stab, N);
   double vm = 0.0;
   int buf = 0;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
     cp_async_wait_0();
     __syncthreads();
     if (tile + gridDim.x < tiles)
-      mirror_stage<NI>(xs + (buf ^ 1) * xsz, g, in, ldm, (tile + gridDim.x) * pts, np, vec16);
+      mirror_stage<NI, 0>(xs + (buf ^ 1) * xsz, g, in, ldm, (tile + gridDim.x) * pts, np, vec16);
     for (int it = warp; it < g.PT / PW * g.NT; it += NW) {
       const int t = it % g.NT, pg = it / g.NT;
       double acc[PW][NI][2][2];
