@@ -154,12 +154,12 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
           sp = fma(fp, fp, sp);
           sm = fma(fm, fm, sm);
         }
-        if constexpr (MODE != 0) pv = fmax(pv, fmax(sqrt(sp), sqrt(sm)));
+        if constexpr (MODE != 0) pv = fmax(pv, fmax(sp, sm));  // the root of the maximum is the maximum of the roots
       }
       if constexpr (MODE == 1) vm = fmax(vm, pv);
       if constexpr (MODE == 2) {
         for (int off = 2; off > 0; off >>= 1) pv = fmax(pv, __shfl_xor_sync(0xffffffffu, pv, off));
-        if (q == 0) atomicMax(pm + 8 * pt + gg, (unsigned long long)__double_as_longlong(pv));
+        if (q == 0) atomicMax(pm + 8 * pt + gg, (unsigned long long)__double_as_longlong(sqrt(pv)));
       }
       }
     }
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
   }
   if constexpr (MODE == 1) {
     for (int off = 16; off > 0; off >>= 1) vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, off));
-    if (lane == 0) atomicMax(vmax, (unsigned long long)__double_as_longlong(vm));
+    if (lane == 0) atomicMax(vmax, (unsigned long long)__double_as_longlong(sqrt(vm)));
   }
 }
 
