@@ -1492,7 +1492,9 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_cross_kernel(const FastArgs a
   for (int it = threadIdx.x >> 5; it < KS_tot / 2; it += blockDim.x >> 5) {
     const int gc = it < tf_koff(M, 1) ? 0 : it < tf_koff(M, 2) ? 1 : 2;
     const int s = it - (gc == 0 ? 0 : gc == 1 ? tf_koff(M, 1) : tf_koff(M, 2));
-    const int g = threadIdx.x & 7, kq = (threadIdx.x & 31) >> 3, i = tf_mode(gc, 4 * s + kq);
+    int g = threadIdx.x & 7;
+    asm volatile("" : "+r"(g));  // keeps the loads of the point's weights in the loop (before it they spill: 134 -> 164 us)
+    const int kq = (threadIdx.x & 31) >> 3, i = tf_mode(gc, 4 * s + kq);
     double rot[6], w[6];
     gauss_curl_gathered<KIND, M, NW>(ga, s_node[g], s_wt[g], s_g1[g], s_g2[g], s_ray[g], i, rot, w);
     // rows of mode i: cosine group CE0 (i = 0 mod 4), CE2 (i = 2 mod 4) or CO (odd), sine group 3 further
@@ -1572,7 +1574,9 @@ __global__ void __launch_bounds__(384, 2) gauss_tf_advect_kernel(const FastArgs 
   for (int it = threadIdx.x >> 5; it < KS_tot / 2; it += blockDim.x >> 5) {
     const int gc = it < tf_koff(M, 1) ? 0 : it < tf_koff(M, 2) ? 1 : 2;
     const int s = it - (gc == 0 ? 0 : gc == 1 ? tf_koff(M, 1) : tf_koff(M, 2));
-    const int g = threadIdx.x & 7, kq = (threadIdx.x & 31) >> 3, i = tf_mode(gc, 4 * s + kq);
+    int g = threadIdx.x & 7;
+    asm volatile("" : "+r"(g));  // keeps the loads of the point's weights in the loop (before it they spill: 117 -> 141 us)
+    const int kq = (threadIdx.x & 31) >> 3, i = tf_mode(gc, 4 * s + kq);
     double wv[6] = {0, 0, 0, 0, 0, 0}, d1[6] = {0, 0, 0, 0, 0, 0}, d2[6] = {0, 0, 0, 0, 0, 0};
     double cw[2] = {0, 0}, c1[2] = {0, 0}, c2[2] = {0, 0};
 #pragma unroll
