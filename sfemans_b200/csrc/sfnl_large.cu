@@ -1,7 +1,8 @@
 // sfnl_large.cu -- the FAST form's folded transforms for large m (SFNL_ALGO_FAST,
-// m up to 512), as two kernels that meet at the grid values: the bundle, the tensor
-// and the conservative advection beyond the fused kernels (m ~ 100); the products and
-// the linearised programs take the residue grids of sfnl_res.cu from m = 65.
+// m up to 512), as two kernels that meet at the grid values: the bundle and the
+// conservative advection from m = 108, the tensor from m = 87, where one CTA of the fused
+// kernels holds no tile of them; the products and the linearised programs take the
+// residue grids of sfnl_res.cu from m = 65.
 //
 // Same grid, folds and DFT tables as the fused kernels of sfnl_fast.cu (the
 // exact truncated product of fft_parallel.F90:147-665 evaluated on an
@@ -24,7 +25,7 @@ namespace {
 // ---------------------------------------------------------------------------
 // large m: the same folded transforms in two kernels, program by program
 // ---------------------------------------------------------------------------
-// Beyond m ~ 100 one CTA cannot hold an 8-point tile's coefficients of six fields and its folded
+// Beyond m = 107 (tensor 86) one CTA cannot hold an 8-point tile's coefficients of six fields and its folded
 // products at once (at m = 256: 196 KB and 147 KB), so the transforms are split at the grid values:
 //   large_syn_kernel  one CTA per (four 8-point tiles, field): stages the field's 2m coefficient rows,
 //                     runs the four class contractions on every angle tile (each B fragment of the
@@ -35,8 +36,6 @@ namespace {
 //                     evaluates the whole program (sfnl_ops.cuh) and the analysis pre-fold of the group's
 //                     outputs into shared memory, and every warp adds the chunk's k-steps to the
 //                     accumulators of its output tiles; the outputs are written at the end.
-// The whole program is evaluated on the grid, so a linearised product du x w + u x dw is analysed once,
-// and the fields shared by all tangents of a batch (the base state) are transformed once per point chunk.
 // With an even number of quadrant angle tiles (every m > 96: the quadrant is a multiple of 16 angles)
 // large_syn_tf_kernel and large_prod_tf_kernel do the same with the third fold (mirror tile pairs),
 // a quarter fewer DMMAs.
@@ -48,19 +47,14 @@ constexpr size_t kLargeSynSmem = 200 * 1024;  // staged coefficients of one synt
 struct LargeArgs {
   const double *in[kMaxIn];
   double *out[kMaxOut];
-  int64_t in_ldm[kMaxIn], out_ldm[kMaxOut], in_bs[kMaxIn], out_bs[kMaxOut];
-  int64_t gslot[kMaxIn];  // G offset of each field (units of tiles * NT * 256 doubles)
-  int syn_f[kMaxIn];      // large_syn_kernel: the fields this launch synthesises (blockIdx.y indexes it)
+  int64_t in_ldm[kMaxIn], out_ldm[kMaxOut];
   int64_t npts;     // points of this chunk (fields are offset to its first point)
   int64_t in_sin;   // sine offset of the inputs (the arrays' np)
   int64_t out_sin;  // sine offset of the outputs (np * point stride)
   int64_t out_ps;   // point stride of the outputs
   int NT, NU_tot, KS_tot;
   int ks_off[4], KS[4], nu_off[4], ke[4];
-  unsigned adj_in;  // bit f: field f is a cotangent
-  int adj_out, vec16, batch_entry;  // batch entry of blockIdx.z == 0 (synthesis) / blockIdx.y == 0 (program)
-  int nown;                          // workspace slots per batch entry (the batched fields)
-  int nbl;                           // batch entries per launch (gridDim.z of the synthesis, gridDim.y of the program)
+  int adj_out, vec16;  // adj_out: no analysis weights
   const double *syn, *ana;
   double *G;
   int64_t tiles;
@@ -77,13 +71,10 @@ template <int PT>
 __global__ void __launch_bounds__(kLargeSynMaxWarps * 32) large_syn_kernel(const LargeArgs a) {
   extern __shared__ double xs[];  // [PT][KS_tot][4][8] of one field, points swizzled (a_frag_slot)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int f = a.syn_f[blockIdx.y];
+  const int f = blockIdx.y;
   const int64_t tile0 = (int64_t)blockIdx.x * PT, p0 = tile0 * 8;
   const int NT = a.NT, KT = 4 * a.KS_tot;
   const size_t pts = (size_t)a.KS_tot * 32;  // point-tile stride in xs
-  const int bz = blockIdx.z;  // entries a.batch_entry + bz (batched fields only; 0 for the shared ones)
-  const double *in_f = a.in[f] + (int64_t)(a.batch_entry + bz) * a.in_bs[f];
-  const int64_t gslot_f = a.gslot[f] + (a.in_bs[f] ? (int64_t)bz * a.nown : 0);
   const int64_t ldm = a.in_ldm[f];
   int KS[4], KOFF[4], KE[4];
 #pragma unroll
@@ -97,7 +88,7 @@ __global__ void __launch_bounds__(kLargeSynMaxWarps * 32) large_syn_kernel(const
     const int pc = 2 * (threadIdx.x % tpr), rstep = blockDim.x / tpr;
     const bool v16 = a.vec16 && p0 + pc + 2 <= a.npts;
     const bool pv0 = p0 + pc < a.npts, pv1 = p0 + pc + 1 < a.npts;
-    const double *base = in_f + p0 + pc;
+    const double *base = a.in[f] + p0 + pc;
     double *dst0 = xs + (size_t)(pc >> 3) * pts;
     for (int r = threadIdx.x / tpr; r < KT; r += rstep) {
       const int c = (r >= 4 * KOFF[1]) + (r >= 4 * KOFF[2]) + (r >= 4 * KOFF[3]);
@@ -115,15 +106,6 @@ __global__ void __launch_bounds__(kLargeSynMaxWarps * 32) large_syn_kernel(const
   }
   cp_async_wait_all();
   __syncthreads();
-  if ((a.adj_in >> f) & 1u) {  // a cotangent: synthesised with the analysis weights 1/N (n = 0), 2/N
-    const double invN = 1.0 / (4.0 * 8.0 * NT), twoN = 2.0 * invN;
-    for (size_t i = threadIdx.x; i < PT * pts; i += blockDim.x) {
-      const int ks = (int)((i % pts) >> 5);
-      const bool n0 = (ks == KOFF[0] || ks == KOFF[2]) && ((i >> 3) & 3) == 0;  // k = 0 of an even class
-      xs[i] *= n0 ? invN : twoN;
-    }
-    __syncthreads();
-  }
   const double *xs_l = xs + a_frag_slot(lane & 3, lane >> 2);
   int ks_max = KS[0];
 #pragma unroll
@@ -159,7 +141,7 @@ __global__ void __launch_bounds__(kLargeSynMaxWarps * 32) large_syn_kernel(const
     for (int pt = 0; pt < PT; ++pt) {
       const int64_t tile = tile0 + pt;
       if (tile >= a.tiles) break;
-      double *gp0 = a.G + ((gslot_f * a.tiles + tile) * NT + t) * 256 + lane;
+      double *gp0 = a.G + ((f * a.tiles + tile) * NT + t) * 256 + lane;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const double A = acc[pt][0][e] + acc[pt][1][e], B = acc[pt][0][e] - acc[pt][1][e];
@@ -184,20 +166,17 @@ template <int PT>
 __global__ void __launch_bounds__(kLargeSynMaxWarps * 32, 1) large_syn_tf_kernel(const LargeArgs a) {
   extern __shared__ double xs[];  // [PT][KS_tot][4][8], points swizzled (a_frag_slot)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int f = a.syn_f[blockIdx.y];
+  const int f = blockIdx.y;
   const int64_t tile0 = (int64_t)blockIdx.x * PT, p0 = tile0 * 8;
   const int NT = a.NT, NH = NT >> 1, KS_tot = a.tkoff[6], KT = 4 * KS_tot;
   const size_t pts = (size_t)KS_tot * 32;
-  const int bz = blockIdx.z;  // entries a.batch_entry + bz (batched fields only; 0 for the shared ones)
-  const double *in_f = a.in[f] + (int64_t)(a.batch_entry + bz) * a.in_bs[f];
-  const int64_t gslot_f = a.gslot[f] + (a.in_bs[f] ? (int64_t)bz * a.nown : 0);
   const int64_t ldm = a.in_ldm[f];
   {  // stage: 4*PT threads per row, two points each
     constexpr int tpr = 4 * PT;
     const int pc = 2 * (threadIdx.x % tpr), rstep = blockDim.x / tpr;
     const bool v16 = a.vec16 && p0 + pc + 2 <= a.npts;
     const bool pv0 = p0 + pc < a.npts, pv1 = p0 + pc + 1 < a.npts;
-    const double *base = in_f + p0 + pc;
+    const double *base = a.in[f] + p0 + pc;
     double *dst0 = xs + (size_t)(pc >> 3) * pts;
     for (int r = threadIdx.x / tpr; r < KT; r += rstep) {
       const int ks = r >> 2;
@@ -219,15 +198,6 @@ __global__ void __launch_bounds__(kLargeSynMaxWarps * 32, 1) large_syn_tf_kernel
   }
   cp_async_wait_all();
   __syncthreads();
-  if ((a.adj_in >> f) & 1u) {  // a cotangent: synthesised with the analysis weights 1/N (n = 0), 2/N
-    const double invN = 1.0 / (4.0 * 8.0 * NT), twoN = 2.0 * invN;
-    for (size_t i = threadIdx.x; i < PT * pts; i += blockDim.x) {
-      const int ks = (int)((i % pts) >> 5);
-      const bool n0 = (ks == 0 || ks == a.tkoff[3]) && ((i >> 3) & 3) == 0;  // k = 0 of CE0 / SE0
-      xs[i] *= n0 ? invN : twoN;
-    }
-    __syncthreads();
-  }
   const double *xs_l = xs + a_frag_slot(lane & 3, lane >> 2);
   const size_t bstride = (size_t)NT * 32;
   const int ks0 = a.tks[0], ks1 = a.tks[1], ks2 = a.tks[2];
@@ -292,7 +262,7 @@ __global__ void __launch_bounds__(kLargeSynMaxWarps * 32, 1) large_syn_tf_kernel
       for (int pt = 0; pt < PT; ++pt) {
         const int64_t tile = tile0 + pt;
         if (tile >= a.tiles) break;
-        double *gp0 = a.G + ((gslot_f * a.tiles + tile) * NT + t) * 256 + lane;
+        double *gp0 = a.G + ((f * a.tiles + tile) * NT + t) * 256 + lane;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const double CE = ce[side][pt][e], SE = se[side][pt][e], CO = od[0][pt][e], SO = od[1][pt][e];
@@ -321,7 +291,6 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32, CPW <= 2 ? 2 : 1) large_
   constexpr int KP = kLargeTfPairs, LT = 2 * KP;  // pairs per chunk, local tiles
   extern __shared__ double pc_s[];  // [NOG][4 classes][LT local tiles][2][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3;
-  const int by = blockIdx.y, b = a.batch_entry + by;  // batch entry of this CTA
   const int64_t tile = blockIdx.x, p = tile * 8 + (lane >> 2);
   const int NT = a.NT, NH = NT >> 1;
   double y[CPW][NOG][2];
@@ -347,7 +316,7 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32, CPW <= 2 ? 2 : 1) large_
         double x[NI], yy[NO];
 #pragma unroll
         for (int f = 0; f < NI; ++f)
-          x[f] = Gl[(a.gslot[f] + (a.in_bs[f] ? (int64_t)by * a.nown : 0)) * fstride + (size_t)t * 256 + r * 64 + e * 32];
+          x[f] = Gl[f * fstride + (size_t)t * 256 + r * 64 + e * 32];
         apply_op<OP>(x, yy);
 #pragma unroll
         for (int o = 0; o < NOG; ++o) gq[r][o] = yy[O0 + o];
@@ -427,7 +396,7 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32, CPW <= 2 ? 2 : 1) large_
 #pragma unroll
       for (int o = 0; o < NOG; ++o) {
         const int og = O0 + o;
-        double *dst = a.out[og] + (int64_t)b * a.out_bs[og] + p * a.out_ps + (int64_t)n * a.out_ldm[og] +
+        double *dst = a.out[og] + p * a.out_ps + (int64_t)n * a.out_ldm[og] +
                       (gr >= 3 ? a.out_sin : 0);
         *dst = (gr >= 3 && n == 0 && !a.nyq) ? 0.0 : y[j][o][h];
       }
@@ -435,15 +404,14 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32, CPW <= 2 ? 2 : 1) large_
   }
 }
 
-// Outputs O0 .. O0+NOG-1 of program OP for batch entry a.batch_entry (the output group is a template
-// parameter so that the program's values stay in registers).
+// Outputs O0 .. O0+NOG-1 of program OP (the output group is a template parameter so that the program's
+// values stay in registers) over an odd number of angle tiles: the tensor at m = 87 to 96.
 template <int OP, int O0, int CPW>
 __global__ void __launch_bounds__(kLargeProdWarps * 32) large_prod_kernel(const LargeArgs a) {
   constexpr int NI = op_nin(OP), NO = op_nout(OP);
   constexpr int NOG = NO - O0 < kLargeGroup ? NO - O0 : kLargeGroup;
   extern __shared__ double pc_s[];  // [NOG][4][LCT][2][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3;
-  const int by = blockIdx.y, b = a.batch_entry + by;  // batch entry of this CTA
   const int64_t tile = blockIdx.x, p = tile * 8 + (lane >> 2);
   const int NT = a.NT;
   double y[CPW][NOG][2];
@@ -453,7 +421,7 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32) large_prod_kernel(const 
     for (int o = 0; o < NOG; ++o) y[j][o][0] = y[j][o][1] = 0.0;
   const int64_t fstride = a.tiles * NT * 256;
   const double *Gl = a.G + tile * NT * 256 + lane;
-  const double *anav = a.ana + (size_t)(a.adj_out ? 1 : 0) * a.NU_tot * NT * 2 * 32 + lane;
+  const double *anav = a.ana + lane;
   const size_t cst = (size_t)kLCT * 2 * 32;  // class stride in pc_s
   for (int t0 = 0; t0 < NT; t0 += kLCT) {
     const int ct = NT - t0 < kLCT ? NT - t0 : kLCT;
@@ -466,7 +434,7 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32) large_prod_kernel(const 
         double x[NI], yy[NO];
 #pragma unroll
         for (int f = 0; f < NI; ++f)
-          x[f] = Gl[(a.gslot[f] + (a.in_bs[f] ? (int64_t)by * a.nown : 0)) * fstride + (size_t)t * 256 + r * 64 + e * 32];
+          x[f] = Gl[f * fstride + (size_t)t * 256 + r * 64 + e * 32];
         apply_op<OP>(x, yy);
 #pragma unroll
         for (int o = 0; o < NOG; ++o) gq[r][o] = yy[O0 + o];
@@ -514,7 +482,7 @@ __global__ void __launch_bounds__(kLargeProdWarps * 32) large_prod_kernel(const 
 #pragma unroll
       for (int o = 0; o < NOG; ++o) {
         const int og = O0 + o;
-        double *dst = a.out[og] + (int64_t)b * a.out_bs[og] + p * a.out_ps + (int64_t)n * a.out_ldm[og] +
+        double *dst = a.out[og] + p * a.out_ps + (int64_t)n * a.out_ldm[og] +
                       (c >= 2 ? a.out_sin : 0);
         *dst = (c == 2 && n == 0) ? 0.0 : y[j][o][h];
       }
@@ -642,10 +610,14 @@ template <int OP, int O0, int CPW>
 int launch_large_prod(const LargeArgs &la, bool tf, cudaStream_t st) {
   constexpr int NO = op_nout(OP), NOG = NO - O0 < kLargeGroup ? NO - O0 : kLargeGroup;
   const size_t smem = sizeof(double) * (size_t)NOG * 4 * (tf ? 2 * kLargeTfPairs : kLCT) * 2 * 32;
-  auto kern = tf ? large_prod_tf_kernel<OP, O0, CPW> : large_prod_kernel<OP, O0, CPW>;
+  auto kern = large_prod_tf_kernel<OP, O0, CPW>;
+  if constexpr (OP == OP_TENSOR && CPW == 2)
+    if (!tf) kern = large_prod_kernel<OP, O0, CPW>;
+  if (!tf && kern == large_prod_tf_kernel<OP, O0, CPW>)
+    return set_error(SFNL_ERR_UNSUPPORTED, "large-m FAST form: odd number of angle tiles");
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (large-m program and analysis)");
-  kern<<<dim3((unsigned)la.tiles, (unsigned)la.nbl), kLargeProdWarps * 32, smem, st>>>(la);
+  kern<<<(unsigned)la.tiles, kLargeProdWarps * 32, smem, st>>>(la);
   return check_launch("large-m program and analysis");
 }
 
@@ -682,24 +654,14 @@ int launch_large_prod_all(const LargeArgs &la, bool tf, cudaStream_t st) {
 
 int launch_large_prod_op(int op, const LargeArgs &la, bool tf, cudaStream_t st) {
   switch (op) {
-    case OP_CROSS: return launch_large_prod_all<OP_CROSS>(la, tf, st);
-    case OP_DOT: return launch_large_prod_all<OP_DOT>(la, tf, st);
-    case OP_PROD: return launch_large_prod_all<OP_PROD>(la, tf, st);
     case OP_BUNDLE: return launch_large_prod_all<OP_BUNDLE>(la, tf, st);
-    case OP_CROSS_JVP: return launch_large_prod_all<OP_CROSS_JVP>(la, tf, st);
-    case OP_CROSS_VJP: return launch_large_prod_all<OP_CROSS_VJP>(la, tf, st);
-    case OP_MHD_JVP: return launch_large_prod_all<OP_MHD_JVP>(la, tf, st);
-    case OP_MHD_VJP: return launch_large_prod_all<OP_MHD_VJP>(la, tf, st);
-    case OP_SVECT: return launch_large_prod_all<OP_SVECT>(la, tf, st);
     case OP_TENSOR: return launch_large_prod_all<OP_TENSOR>(la, tf, st);
     case OP_ADVECT: return launch_large_prod_all<OP_ADVECT>(la, tf, st);
   }
-  return set_error(SFNL_ERR_ARG, "large-m FAST form: program not bilinear");
+  return set_error(SFNL_ERR_ARG, "large-m FAST form: a program of the residue grids");
 }
 
-// nbz: batch entries (blockIdx.z) of the launch, 1 for the batch-invariant fields.
-int launch_large_syn(const LargeArgs &la, int nfields, int nbz, bool tf, cudaStream_t st) {
-  if (nfields == 0) return SFNL_OK;
+int launch_large_syn(const LargeArgs &la, int nfields, bool tf, cudaStream_t st) {
   // angle tiles (pairs of mirror tiles with the third fold) spread evenly over at most kLargeSynMaxWarps warps
   const int units = tf ? la.NT / 2 : la.NT;
   const int rounds = (units + kLargeSynMaxWarps - 1) / kLargeSynMaxWarps, nw = (units + rounds - 1) / rounds;
@@ -709,7 +671,7 @@ int launch_large_syn(const LargeArgs &la, int nfields, int nbz, bool tf, cudaStr
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return set_error(SFNL_ERR_CUDA, "cudaFuncSetAttribute failed (large-m synthesis)");
     const int64_t blocks = (la.tiles + pt - 1) / pt;
-    kern<<<dim3((unsigned)blocks, (unsigned)nfields, (unsigned)nbz), nw * 32, smem, st>>>(la);
+    kern<<<dim3((unsigned)blocks, (unsigned)nfields), nw * 32, smem, st>>>(la);
     return check_launch("large-m synthesis");
   };
   if (tf) {
@@ -729,10 +691,6 @@ constexpr size_t kLargeWorkspaceBytes = size_t(1) << 30;  // grid values of one 
 // Tests only (sfnl_test_large_workspace_cap): a bound on both workspaces far below the production ones, so
 // that small calls run many point chunks and batch groups; 0: none.
 std::atomic<size_t> g_test_cap{0};
-// Batched programs (tangents): the workspace may grow to this, or to a quarter of the free device memory,
-// so that one launch serves every batch entry of a point chunk of at least kLargeMinChunk points.
-constexpr size_t kLargeBatchWorkspaceBytes = size_t(8) << 30;
-constexpr int64_t kLargeMinChunk = 4096;
 
 }  // namespace
 
@@ -770,45 +728,15 @@ struct LargePlan {
   double *syn, *ana;         // its tables
 };
 
-// The two-kernel form: per point chunk, the batch-invariant fields (base state) once, then the batch
-// entries in groups of kb: one synthesis launch for the group's own fields (blockIdx.z = entry) and one
-// launch per group of three outputs (blockIdx.y = entry).  The grid-value workspace holds the shared
-// fields and kb entries' own fields of one point chunk: kb = the whole batch when a chunk of at least
-// kLargeMinChunk points fits the batched workspace bound, else as many entries as such a chunk allows.
+// The two-kernel form: per point chunk, one synthesis launch for the fields and one launch per group of three
+// outputs; the workspace holds the grid values of a chunk.
 // rp: a residue pass (launch_large_res): the residue grid's geometry and tables, the Nyquist mode in the
-// sine row of mode 0, no analysis weights and no cotangent weights (both applied outside).
+// sine row of mode 0, no analysis weights (applied outside).
 int run_large(const ProgArgs &a, const Geo &g, const Tables &T, const LargePlan *rp, cudaStream_t st) {
   const int ni = op_nin(a.op), no = op_nout(a.op);
-  int nshared = 0, nown = 0;  // batch-invariant fields take the first G slots, the batched ones the next
-  int64_t gslot[kMaxIn];
-  for (int f = 0; f < ni; ++f) gslot[f] = a.in_bs[f] == 0 ? nshared++ : -1;
-  for (int f = 0; f < ni; ++f)
-    if (gslot[f] < 0) gslot[f] = nshared + nown++;
-  const size_t field_bytes = sizeof(double) * (size_t)(rp ? rp->N : g.N);  // one field's grid values per point
+  const size_t per_point = sizeof(double) * (size_t)(rp ? rp->N : g.N) * ni;  // the fields' grid values
   size_t cap = kLargeWorkspaceBytes;
-  int kb = 1;
-  if (a.batch > 1 && nown > 0) {
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-      cudaGetLastError();
-      free_b = 0;
-    }
-    size_t bcap = kLargeBatchWorkspaceBytes < free_b / 4 ? kLargeBatchWorkspaceBytes : free_b / 4;
-    if (bcap < cap) bcap = cap;
-    const size_t per_entry = field_bytes * nown * (size_t)kLargeMinChunk;
-    const size_t shared_b = field_bytes * nshared * (size_t)kLargeMinChunk;
-    const int64_t fit = bcap > shared_b ? (int64_t)((bcap - shared_b) / per_entry) : 0;
-    kb = (int)(fit < 1 ? 1 : fit > a.batch ? a.batch : fit);
-    cap = bcap;
-  }
-  if (const size_t tc = g_test_cap.load()) {
-    cap = tc;
-    if (a.batch > 1 && nown > 0) {
-      const int64_t fit = (int64_t)(tc / (field_bytes * (size_t)(nshared + nown) * 32));
-      kb = (int)(fit < 1 ? 1 : fit > a.batch ? a.batch : fit);
-    }
-  }
-  const size_t per_point = field_bytes * (size_t)(nshared + (int64_t)kb * nown);
+  if (const size_t tc = g_test_cap.load()) cap = tc;
   int64_t chunk = (int64_t)(cap / per_point);
   chunk = (chunk / 32) * 32;
   if (chunk < 32) chunk = 32;
@@ -826,10 +754,6 @@ int run_large(const ProgArgs &a, const Geo &g, const Tables &T, const LargePlan 
   } else if (tf) {
     if (int rc = get_tf_tables(g, &TT)) return rc;
   }
-  const bool adj_out = rp ? true : op_adjoint_out(a.op);
-  unsigned adj = 0;
-  for (int f = 0; f < ni && !rp; ++f)
-    if (op_adjoint_in(a.op, f)) adj |= 1u << f;
   for (int64_t c0 = 0; c0 < a.np; c0 += chunk) {
     LargeArgs la;
     std::memset(&la, 0, sizeof(la));
@@ -838,19 +762,15 @@ int run_large(const ProgArgs &a, const Geo &g, const Tables &T, const LargePlan 
     la.in_sin = a.np;
     la.out_ps = a.out_ps;
     la.out_sin = a.np * a.out_ps;
-    la.nown = nown;
     int v16 = (a.np & 1) ? 0 : 1;
     for (int f = 0; f < ni; ++f) {
       la.in[f] = a.in[f] + c0;
       la.in_ldm[f] = a.in_ldm[f];
-      la.in_bs[f] = a.in_bs[f];
-      la.gslot[f] = gslot[f];
-      if ((reinterpret_cast<uintptr_t>(la.in[f]) & 15) || (la.in_ldm[f] & 1) || (la.in_bs[f] & 1)) v16 = 0;
+      if ((reinterpret_cast<uintptr_t>(la.in[f]) & 15) || (la.in_ldm[f] & 1)) v16 = 0;
     }
     for (int o = 0; o < no; ++o) {
       la.out[o] = a.out[o] + c0 * a.out_ps;
       la.out_ldm[o] = a.out_ldm[o];
-      la.out_bs[o] = a.out_bs[o];
     }
     la.NT = NT;
     la.NU_tot = g.NU_tot;
@@ -861,8 +781,7 @@ int run_large(const ProgArgs &a, const Geo &g, const Tables &T, const LargePlan 
       la.nu_off[c] = g.nu_off[c];
       la.ke[c] = g.ke[c];
     }
-    la.adj_in = adj;
-    la.adj_out = adj_out ? 1 : 0;
+    la.adj_out = rp ? 1 : 0;
     la.vec16 = v16;
     la.syn = TT.syn;
     la.ana = TT.ana;
@@ -881,22 +800,8 @@ int run_large(const ProgArgs &a, const Geo &g, const Tables &T, const LargePlan 
     for (int gr = 0; gr < 3; ++gr) la.tke[gr] = tf_ke(mt, gr);
     la.asteps = la.taoff[6];
     la.nyq = rp ? 1 : 0;
-    // the batch-invariant fields, once per chunk
-    int k = 0;
-    for (int f = 0; f < ni; ++f)
-      if (a.in_bs[f] == 0) la.syn_f[k++] = f;
-    la.batch_entry = 0;
-    la.nbl = 1;
-    if (int rc = launch_large_syn(la, k, 1, tf, st)) return rc;
-    for (int b0 = 0; b0 < a.batch; b0 += kb) {
-      la.batch_entry = b0;
-      la.nbl = a.batch - b0 < kb ? a.batch - b0 : kb;
-      k = 0;
-      for (int f = 0; f < ni; ++f)
-        if (a.in_bs[f] != 0) la.syn_f[k++] = f;
-      if (int rc = launch_large_syn(la, k, la.nbl, tf, st)) return rc;
-      if (int rc = launch_large_prod_op(a.op, la, tf, st)) return rc;
-    }
+    if (int rc = launch_large_syn(la, ni, tf, st)) return rc;
+    if (int rc = launch_large_prod_op(a.op, la, tf, st)) return rc;
   }
   return SFNL_OK;
 }
@@ -921,7 +826,7 @@ int run_large(const ProgArgs &a, const Geo &g, const Tables &T, const LargePlan 
 // mode).  At m = 128 the passes over the coefficients and sums cost more than the DMMAs saved (cross
 // product at 100k points 2.65 -> 2.93 ms with R = 3); from m = 256 on the residues win.
 constexpr int kMaxResidues = 12;
-std::atomic<int> g_test_residues{0};  // tests: force R (0: the choice below)
+std::atomic<int> g_test_residues{0};  // tests: force R in the two-kernel form (0: the choice below)
 
 bool residues_fit(int m, int N, int R) {
   if (N != 3 * m || R < 3 || R > kMaxResidues || N % R) return false;
@@ -1017,21 +922,21 @@ int get_residue_tables(int m, int N, int R, ResTab *out) {
 
 namespace {
 
-// The R residues of one input field (batch entry blockIdx.z) at the chunk's points: thread (point, k),
+// The R residues of one input field at the chunk's points: thread (point, k),
 // k < M/2, gathers Y_k and Y_{M-k} of each residue from the modes qM + k and qM + M - k (k = 0: Y_0 and
 // Y_{M/2} from qM and qM + M/2) and writes alpha_k, beta_k (k = 0: alpha_0 and beta_{M/2}) into
 // y + r * ystride, each (npc, 2, M/2): cosine k at 2k npc, sine k at (2k + 1) npc, the sine row 0 holding
-// beta_{M/2}.  Cotangents (adj) take the analysis weights 1/N (n = 0), 2/N first.  The residues pair as
+// beta_{M/2}.  The residues pair as
 // d_{R-1-r} = -d_r (and d = 0 for the middle one of an odd R), so one twiddle serves two residues.
 template <int R>
-__global__ void large_res_coef_kernel(const double *x, int64_t ldm, int64_t xsin, int64_t xbs, double *y,
-                                      int64_t ystride, int64_t npc, int m, int adj, double invN, const double *tw) {
+__global__ void large_res_coef_kernel(const double *x, int64_t ldm, int64_t xsin, double *y, int64_t ystride,
+                                      int64_t npc, int m, const double *tw) {
   constexpr int RP = R / 2;  // residue pairs
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npc) return;
   const int k = blockIdx.y, M = 3 * m / R, mh = M >> 1;
-  const double *xp = x + (int64_t)blockIdx.z * xbs + p;
-  double *yp = y + (int64_t)blockIdx.z * M * npc + p;
+  const double *xp = x + p;
+  double *yp = y + p;
   double yr[2][R], yi[2][R];  // Y_k (side 0) and Y_{M-k} (side 1; k = 0: Y_{M/2}) of each residue
 #pragma unroll
   for (int side = 0; side < 2; ++side)
@@ -1040,11 +945,10 @@ __global__ void large_res_coef_kernel(const double *x, int64_t ldm, int64_t xsin
   const int khi = k == 0 ? mh : M - k;
 #pragma unroll
   for (int q = 0; q < R / 3; ++q) {  // m = (R/3) M: every qM + k and qM + M - k is a mode
-    const double sg = (q & 1) ? -1.0 : 1.0;
+    const double wn = (q & 1) ? -1.0 : 1.0;
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
       const int n = q * M + (side ? khi : k);
-      const double wn = (adj ? (n == 0 ? invN : 2.0 * invN) : 1.0) * sg;
       const double a = xp[(int64_t)n * ldm] * wn, b = xp[(int64_t)n * ldm + xsin] * wn;
       // y_n = (a - i b)(c +- i s): residue r (+s) and R-1-r (-s)
 #pragma unroll
@@ -1076,20 +980,20 @@ __global__ void large_res_coef_kernel(const double *x, int64_t ldm, int64_t xsin
   }
 }
 
-// One output (batch entry blockIdx.z) from the R residues' sums S + r * rstride, each (npc, 2, M/2) with
+// One output from the R residues' sums S + r * rstride, each (npc, 2, M/2) with
 // the sine row 0 holding S_{M/2}: thread (point, k), k < M/2, writes the modes qM + k and qM + M - k
-// (k = 0: qM and qM + M/2) below m.  w = 2/N (or 1 without analysis weights), w0 = 1/N (or 1).  Paired
+// (k = 0: qM and qM + M/2) below m.  w = 2/N, w0 = 1/N.  Paired
 // residues share their twiddle as in large_res_coef_kernel.
 template <int R>
 __global__ void large_res_out_kernel(const double *S, int64_t rstride, double *out, int64_t ldm, int64_t osin,
-                                     int64_t ops, int64_t obs, int64_t npc, int m, double w, double w0,
+                                     int64_t ops, int64_t npc, int m, double w, double w0,
                                      const double *tw) {
   constexpr int RP = R / 2;
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= npc) return;
   const int k = blockIdx.y, M = 3 * m / R, mh = M >> 1;
-  const double *sp = S + (int64_t)blockIdx.z * M * npc + p;
-  double *op = out + (int64_t)blockIdx.z * obs + p * ops;
+  const double *sp = S + p;
+  double *op = out + p * ops;
   const int64_t ic = (int64_t)(2 * k) * npc, is = (int64_t)(2 * k + 1) * npc;
   // P^r_k = C - i S; the mirror P^r_{M-k} = -conj(P^r_k) = -C - i S; k = 0: P^r_0 = C, P^r_{M/2} = -i S
   double C[R], Sv[R];
@@ -1129,31 +1033,15 @@ __global__ void large_res_out_kernel(const double *S, int64_t rstride, double *o
   }
 }
 
-template <int R>
-void launch_res_coef(dim3 grid, int threads, cudaStream_t st, const double *x, int64_t ldm, int64_t xsin,
-                     int64_t xbs, double *y, int64_t ystride, int64_t npc, int m, int adj, double invN,
-                     const double *tw) {
-  large_res_coef_kernel<R><<<grid, threads, 0, st>>>(x, ldm, xsin, xbs, y, ystride, npc, m, adj, invN, tw);
-}
-template <int R>
-void launch_res_out(dim3 grid, int threads, cudaStream_t st, const double *S, int64_t rstride, double *out, int64_t ldm,
-                    int64_t osin, int64_t ops, int64_t obs, int64_t npc, int m, double w, double w0, const double *tw) {
-  large_res_out_kernel<R><<<grid, threads, 0, st>>>(S, rstride, out, ldm, osin, ops, obs, npc, m, w, w0, tw);
-}
-
 // The two-kernel form on the residue grids: per point chunk, the R residues' coefficients of every input
-// field in one pass (N/R doubles per point, field instance and residue), the residue passes of the program
-// (run_large; sums into N/R doubles per point, output instance and residue), and the outputs from the R
-// residues' sums in one pass.
+// field in one pass (N/R doubles per point, field and residue), the residue passes of the program (run_large;
+// sums into N/R doubles per point, output and residue), and the outputs from the R residues' sums in one pass.
 int launch_large_res(const ProgArgs &a, const Geo &g, int R, cudaStream_t st) {
   const int m = a.m, N = g.N, M = N / R, mh = M / 2, ni = op_nin(a.op), no = op_nout(a.op);
   ResTab T;
   if (int rc = get_residue_tables(m, N, R, &T)) return rc;
   const LargePlan rp{M, M / 32, mh, T.syn, T.ana};
-  int64_t inst_in = 0;
-  for (int f = 0; f < ni; ++f) inst_in += a.in_bs[f] ? a.batch : 1;
-  const int64_t inst_out = (int64_t)no * a.batch;
-  const size_t per_point = sizeof(double) * (size_t)N * (size_t)(inst_in + inst_out);
+  const size_t per_point = sizeof(double) * (size_t)N * (size_t)(ni + no);
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     cudaGetLastError();
@@ -1170,36 +1058,27 @@ int launch_large_res(const ProgArgs &a, const Geo &g, int R, cudaStream_t st) {
   double *W = nullptr;
   LargeWorkspace ws(st, 1);
   if (int rc = ws.get(per_point * (size_t)chunk, &W)) return rc;
-  const bool adj_out = op_adjoint_out(a.op);
-  const double invN = 1.0 / N, w = adj_out ? 1.0 : 2.0 * invN, w0 = adj_out ? 1.0 : invN;
   constexpr int kThreads = 256;
-  auto coef = R == 3 ? launch_res_coef<3> : R == 6 ? launch_res_coef<6> : launch_res_coef<12>;
-  auto outk = R == 3 ? launch_res_out<3> : R == 6 ? launch_res_out<6> : launch_res_out<12>;
+  auto coef = R == 3 ? large_res_coef_kernel<3> : R == 6 ? large_res_coef_kernel<6> : large_res_coef_kernel<12>;
+  auto outk = R == 3 ? large_res_out_kernel<3> : R == 6 ? large_res_out_kernel<6> : large_res_out_kernel<12>;
   for (int64_t c0 = 0; c0 < a.np; c0 += chunk) {
     const int64_t npc = a.np - c0 < chunk ? a.np - c0 : chunk;
-    const unsigned bx = (unsigned)((npc + kThreads - 1) / kThreads);
+    const dim3 grid((unsigned)((npc + kThreads - 1) / kThreads), (unsigned)mh);
     // residue r's arrays: inputs at W + r * rin, outputs at W + R rin + r * rout
-    const int64_t rin = inst_in * M * npc, rout = inst_out * M * npc;
+    const int64_t rin = (int64_t)ni * M * npc, rout = (int64_t)no * M * npc;
     ProgArgs ar = a;
     ar.np = npc;
     ar.out_ps = 1;
-    int64_t off = 0;
     for (int f = 0; f < ni; ++f) {
-      const int nb = a.in_bs[f] ? a.batch : 1;
-      coef(dim3(bx, (unsigned)mh, (unsigned)nb), kThreads, st, a.in[f] + c0, a.in_ldm[f], a.np, a.in_bs[f], W + off, rin,
-           npc, m, op_adjoint_in(a.op, f) ? 1 : 0, invN, T.tw);
-      ar.in[f] = W + off;
+      double *y = W + (int64_t)f * M * npc;
+      coef<<<grid, kThreads, 0, st>>>(a.in[f] + c0, a.in_ldm[f], a.np, y, rin, npc, m, T.tw);
+      ar.in[f] = y;
       ar.in_ldm[f] = 2 * npc;
-      ar.in_bs[f] = a.in_bs[f] ? (int64_t)M * npc : 0;
-      off += (int64_t)nb * M * npc;
     }
     if (int rc = check_launch("large-m residue coefficients")) return rc;
-    off = R * rin;
     for (int o = 0; o < no; ++o) {
-      ar.out[o] = W + off;
+      ar.out[o] = W + R * rin + (int64_t)o * M * npc;
       ar.out_ldm[o] = 2 * npc;
-      ar.out_bs[o] = (int64_t)M * npc;
-      off += (int64_t)a.batch * M * npc;
     }
     for (int r = 0; r < R; ++r) {
       ProgArgs rr = ar;
@@ -1208,8 +1087,8 @@ int launch_large_res(const ProgArgs &a, const Geo &g, int R, cudaStream_t st) {
       if (int rc = run_large(rr, g, Tables{}, &rp, st)) return rc;
     }
     for (int o = 0; o < no; ++o)
-      outk(dim3(bx, (unsigned)mh, (unsigned)a.batch), kThreads, st, ar.out[o], rout, a.out[o] + c0 * a.out_ps,
-           a.out_ldm[o], a.np * a.out_ps, a.out_ps, a.out_bs[o], npc, m, w, w0, T.tw);
+      outk<<<grid, kThreads, 0, st>>>(ar.out[o], rout, a.out[o] + c0 * a.out_ps, a.out_ldm[o], a.np * a.out_ps, a.out_ps,
+                                      npc, m, 2.0 / N, 1.0 / N, T.tw);
     if (int rc = check_launch("large-m residue outputs")) return rc;
   }
   return SFNL_OK;
@@ -1233,10 +1112,11 @@ void large_res_release_tables() {
   cudaSetDevice(prev);
 }
 
-// The two-kernel form: on the grid's residue classes when the grid is 3m angles and m >= 256 (R of them:
-// 3/R of the DMMAs of the whole grid, launch_large_res), else on the whole grid.
+// The products and linearised programs on residue grids (launch_res).  The others in the two-kernel form: on the grid's
+// residue classes when the grid is 3m angles and m >= 256 (R of them: 3/R of the DMMAs of the whole grid,
+// launch_large_res), else on the whole grid.
 int launch_fast_large(const ProgArgs &a, const Geo &g, const Tables &T, cudaStream_t st) {
-  if (!g_test_residues.load() && res_supported(a.op, a.m)) {
+  if (res_supported(a.op, a.m)) {
     const size_t tc = g_test_cap.load();
     return launch_res(a, tc ? tc : kResWorkspaceBytes, st);
   }
