@@ -949,7 +949,8 @@ __global__ void large_res_coef_kernel(const double *x, int64_t ldm, int64_t xsin
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
       const int n = q * M + (side ? khi : k);
-      const double a = xp[(int64_t)n * ldm] * wn, b = xp[(int64_t)n * ldm + xsin] * wn;
+      const double a = xp[(int64_t)n * ldm] * wn;
+      const double b = n > 0 ? xp[(int64_t)n * ldm + xsin] * wn : 0.0;  // the sine of mode 0 is ignored
       // y_n = (a - i b)(c +- i s): residue r (+s) and R-1-r (-s)
 #pragma unroll
       for (int r = 0; r < RP; ++r) {

@@ -87,6 +87,16 @@ def test_non_finite_points_stay_alone(kind, m, algo):
     assert all(hit)
 
 
+@pytest.mark.parametrize("kind,m,algo", CASES + [("bundle", 128, None), ("bundle", 256, None), ("tensor", 256, None)])
+def test_the_sine_of_mode_0_is_not_read(kind, m, algo):
+    f = _inputs(kind, 21, m)
+    algo = sf.ALGO_FAST if kind == "tensor" else algo
+    want = _run(kind, f, algo)
+    for x in f:
+        x[:, 1::2, 0] = float("nan")
+    assert all(np.array_equal(g, w) for g, w in zip(_run(kind, f, algo), want))
+
+
 @pytest.mark.parametrize("npts", [29, 40])
 @pytest.mark.parametrize("nslot,m", [(2, 20), (6, 33), (4, 9)])
 def test_synthesis(nslot, m, npts):
