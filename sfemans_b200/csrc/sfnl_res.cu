@@ -5,7 +5,7 @@
 // d_r = pi(2r + 1 - R)/N.  As in sfnl_large.cu, a field is on residue r the transform of M real coefficients to M
 // angles (mode n = M q + k of y_n = z_n e^{i n d_r} is mode k with the sign (-1)^q, and the modes k and M - k meet
 // in one coefficient), third-folded; a product's sums on the residues add up to its coefficients.  Any m fits with
-// R = ceil((3m - 2)/M) residues (3 to 12); a larger grid than the reference's changes nothing, the product being
+// R = ceil((3m - 2)/M) residues (4 to 12); a larger grid than the reference's changes nothing, the product being
 // alias-free on both (fft_parallel.F90:147-328).
 //
 //   coef_kernel   inputs -> the R residues' coefficients of every field, one pass
@@ -477,11 +477,12 @@ int launch_passes(const CoefArgs *ca, const OutArgs *oa, cudaStream_t st) {
 }
 template <int M>
 int launch_passes(int R, const CoefArgs *ca, const OutArgs *oa, cudaStream_t st) {
+  if constexpr (M == 64) switch (R) {  // 128 angles begin beyond 12 residues of 64
+      case 4: return launch_passes<M, 4>(ca, oa, st);
+      case 5: return launch_passes<M, 5>(ca, oa, st);
+      case 6: return launch_passes<M, 6>(ca, oa, st);
+    }
   switch (R) {
-    case 3: return launch_passes<M, 3>(ca, oa, st);
-    case 4: return launch_passes<M, 4>(ca, oa, st);
-    case 5: return launch_passes<M, 5>(ca, oa, st);
-    case 6: return launch_passes<M, 6>(ca, oa, st);
     case 7: return launch_passes<M, 7>(ca, oa, st);
     case 8: return launch_passes<M, 8>(ca, oa, st);
     case 9: return launch_passes<M, 9>(ca, oa, st);
