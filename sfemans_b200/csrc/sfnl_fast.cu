@@ -734,12 +734,19 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
 // with the host's share): the next tile's copies start when the last angle tile's coefficients are read.  Measured on
 // a B200 against fast_kernel: cross product, 28,000 points, m = 16 26.6 -> 24.6 us; 50,001 points, m = 10 50 -> 30 us;
 // product of scalars, 100,000 points, m = 8 32 -> 19 us; dot product, 60,000 points, m = 24 66 -> 61 us.  Three
-// outputs at m = 17..32 need 255 registers (two CTAs) and were slower than fast_kernel (m = 32: 192 against 160 us), and
-// so was the dot product at m = 25..32, whose tile is the longest (m = 32, 3,000 points 9.7 against 12.5 us, 14,000
-// points 22.8 against 26.9, 100,000 points 134.8 against 136.4).
+// outputs at m = 17..32 need 255 registers (two CTAs) and were slower than fast_kernel (m = 32: 192 against 160 us).
 constexpr int kSoloWarps = 4;
 // Largest k-steps per class (KSC; the analysis has NUC = (KSC + 1) / 2 output tiles of 8 per class).
-constexpr int solo_max_ks(int ek) { return ek == EK_PROD ? 4 : ek == EK_DOT ? 3 : 2; }
+constexpr int solo_max_ks(int ek) { return ek_nout(ek) == 1 ? 4 : 2; }
+// The dot product's tiles at m = 25..32 are the longest of these, so that a wave of them that is not full costs most:
+// fast_kernel is the faster one below 1 2/3 waves of 12 warps per SM (m = 28, 14,200 points 22.9 against 26.9 us, 20,000
+// points 31.2 against 35.2) and from m = 29, where its own loops are full, everywhere (m = 32, 40,000 points 60.4
+// against 64.4, 114,000 points 152.4 against 150.2) but where two waves are (28,000 points 43.6 against 39.6); with more
+// waves at m = 25..28 solo_kernel (85,000 points 118.6 against 109.1).
+inline bool solo_takes_dot(int m, int64_t np) {
+  const int64_t wave = (int64_t)12 * num_sms(), tiles = (np + 7) / 8;
+  return m <= 28 ? 3 * tiles >= 5 * wave : tiles <= 2 * wave && 4 * tiles >= 7 * wave;
+}
 constexpr bool solo_ek(int ek) { return ek == EK_CROSS || ek == EK_DOT || ek == EK_PROD || ek == EK_SVECT; }
 constexpr size_t solo_smem_bytes(int ek, int KSC) { return sizeof(double) * (size_t)kSoloWarps * ek_nin(ek) * 4 * KSC * 32; }
 
@@ -1803,10 +1810,10 @@ int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
   if constexpr (solo_ek(EK) && ADJ == 0) {
     if (fa.KS[0] == 1) return launch_solo<EK, 1>(fa, batch, st);
     if (fa.KS[0] == 2) return launch_solo<EK, 2>(fa, batch, st);
-    if constexpr (solo_max_ks(EK) >= 3)
+    if constexpr (solo_max_ks(EK) == 4) {
       if (fa.KS[0] == 3) return launch_solo<EK, 3>(fa, batch, st);
-    if constexpr (solo_max_ks(EK) >= 4)
-      if (fa.KS[0] == 4) return launch_solo<EK, 4>(fa, batch, st);
+      if (fa.KS[0] == 4 && (EK != EK_DOT || solo_takes_dot(fa.m, fa.np * batch))) return launch_solo<EK, 4>(fa, batch, st);
+    }
   }
   // every (KS, NT) of make_geo up to m = 64; run-time loops cost the sizes between 16, 32 and 64 a third of their time
   // (cross product, 50,001 points: m = 20 99 -> 62 us, m = 40 207 -> 148, m = 48 337 -> 202, m = 52 384 -> 229)
@@ -1817,21 +1824,22 @@ int launch_ek_adj(FastArgs &fa, int batch, cudaStream_t st) {
     }
     return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);  // m > 64 without a workspace
   } else {
+  constexpr int S = !solo_ek(EK) ? 0 : EK == EK_DOT ? 3 : solo_max_ks(EK);  // solo_kernel has taken these
   switch (10 * fa.KS[0] + fa.NT) {
-    case 11: return launch_ek_m<EK, 1, 1, ADJ>(fa, batch, st);
-    case 21: return launch_ek_m<EK, 2, 1, ADJ>(fa, batch, st);
-    case 22: return launch_ek_m<EK, 2, 2, ADJ>(fa, batch, st);
-    case 32: return launch_ek_m<EK, 3, 2, ADJ>(fa, batch, st);
-    case 33: return launch_ek_m<EK, 3, 3, ADJ>(fa, batch, st);
-    case 43: return launch_ek_m<EK, 4, 3, ADJ>(fa, batch, st);
+    case 11: if constexpr (S < 1) return launch_ek_m<EK, 1, 1, ADJ>(fa, batch, st); else break;
+    case 21: if constexpr (S < 2) return launch_ek_m<EK, 2, 1, ADJ>(fa, batch, st); else break;
+    case 22: if constexpr (S < 2) return launch_ek_m<EK, 2, 2, ADJ>(fa, batch, st); else break;
+    case 32: if constexpr (S < 3) return launch_ek_m<EK, 3, 2, ADJ>(fa, batch, st); else break;
+    case 33: if constexpr (S < 3) return launch_ek_m<EK, 3, 3, ADJ>(fa, batch, st); else break;
+    case 43: if constexpr (S < 4) return launch_ek_m<EK, 4, 3, ADJ>(fa, batch, st); else break;
     case 54: return launch_ek_m<EK, 5, 4, ADJ>(fa, batch, st);
     case 64: return launch_ek_m<EK, 6, 4, ADJ>(fa, batch, st);
     case 65: return launch_ek_m<EK, 6, 5, ADJ>(fa, batch, st);
     case 75: return launch_ek_m<EK, 7, 5, ADJ>(fa, batch, st);
     case 76: return launch_ek_m<EK, 7, 6, ADJ>(fa, batch, st);
     case 86: return launch_ek_m<EK, 8, 6, ADJ>(fa, batch, st);
-    default: return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);
   }
+  return launch_ek_m<EK, 0, 0, ADJ>(fa, batch, st);
   }
 }
 

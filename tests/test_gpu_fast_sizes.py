@@ -57,3 +57,13 @@ def test_adjoint_identity_at_geometry_bounds(m):
         lhs, rhs = float((jv[..., t] * c[..., t]).sum()), float((v[..., t] * jc[..., t]).sum())
         scale = np.linalg.norm(jv[..., t]) * np.linalg.norm(c[..., t])
         assert abs(lhs - rhs) <= TOL * scale
+
+
+@pytest.mark.parametrize("waves", [1.6, 1.7, 1.74, 1.8, 2.0, 2.1])
+@pytest.mark.parametrize("m", [25, 28, 29, 32])
+def test_dot_products_around_the_waves_of_the_one_warp_kernel(m, waves):
+    torch = pytest.importorskip("torch")
+    npts = int(8 * 12 * torch.cuda.get_device_properties(0).multi_processor_count * waves) - 3
+    V1, V2 = R.synthetic_field(npts, 6, m, 0.2, 7), R.synthetic_field(npts, 6, m, 0.2, 8)
+    out = sf.product(sf.OP_DOT, sf.to_device(V1), sf.to_device(V2), m_max_pad=_pad(m), algo=sf.ALGO_FAST)
+    assert R.rel_l2(sf.to_host(out), R.fft_par("dot", V1, V2, _pad(m))) <= TOL
