@@ -7,7 +7,7 @@
 // half-complex pack of :88-112, :1497-1511, whose sine of mode 0 is ignored) on the N = 2*m_max_pad-1
 // angles of the reference grid.  The mirror symmetry of that grid, theta_{N-j} = 2 pi - theta_j, is
 // folded out: with C_j the cosine part and S_j the sine part at angle j, f_j = C_j + S_j and
-// f_{N-j} = C_j - S_j, so each warp evaluates (N+1)/2 angles.
+// f_{N-j} = C_j - S_j, so N/2 + 1 angles are evaluated.
 //
 // Two kernels.  mirror_synth_kernel takes every size whose tile fits in shared memory: 8-point tiles on the FP64
 // tensor cores (sfnl_mirror.cuh).  synth_kernel (one warp per point, lanes owning angles) is the fallback beyond.
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kSynthThreads) synth_kernel(const double *v, d
   }
   __syncthreads();
   if (warp >= warps_per_cta) return;
-  const int nh = (N + 1) / 2;  // angles 0..nh-1 and their mirrors N-j
+  const int nh = N / 2 + 1;  // angles 0..nh-1 and their mirrors N-j (0, and N/2 of an even grid, are their own)
   double vm = 0.0;
   for (int64_t p = (int64_t)blockIdx.x * warps_per_cta + warp; p < np; p += (int64_t)gridDim.x * warps_per_cta) {
     for (int idx = lane; idx < nslot * m; idx += 32) {
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kSynthThreads) synth_kernel(const double *v, d
         } else {
           double *o = out + (size_t)N * (f + (int64_t)nf * p);
           o[j] = C + S;
-          if (j > 0) o[N - j] = C - S;
+          if (j > 0 && 2 * j != N) o[N - j] = C - S;
         }
       }
       if constexpr (MAXV) {

@@ -87,3 +87,15 @@ def test_host_entry_points_in_chunks():
     g = R.synth_grid(V, 95, workers=8)
     ref = float(np.sqrt((g ** 2).sum(axis=1)).max())
     assert abs(sf.FFT_MAX_VEL_DCL(None, V, 1, npts, 48) - ref) <= MAX_TOL * ref
+
+
+@pytest.mark.parametrize("nslot,m,N", [(10, 489, 1441), (10, 489, 1442), (2, 2000, 4000), (6, 558, 1428)])
+def test_synthesis_beyond_a_tile(nslot, m, N):
+    # grids whose tile exceeds shared memory; an even one has a second angle that is its own mirror
+    npts = 3
+    v = R.synthetic_field(npts, nslot, m, 0.01, 5)
+    th = 2.0 * np.pi * (np.outer(np.arange(m), np.arange(N)) % N) / N
+    want = np.einsum("pfm,mn->nfp", v[:, 0::2], np.cos(th)) + np.einsum("pfm,mn->nfp", v[:, 1::2], np.sin(th))
+    got = host(sf.synthesis(dev(v), n_theta=N))
+    assert R.rel_l2(got, want) <= 1e-12
+    assert np.allclose(got, want, rtol=0, atol=1e-12 * np.abs(want).max() * np.sqrt(m))
