@@ -997,7 +997,7 @@ int sfnl_fft_max_vel_dcl(const double *V1_in, double *V_out, int np, int nb_fiel
   if (rc) return rc;
   double best = 0.0;
   for (double x : pmax)
-    if (!(x <= best)) best = x;  // a NaN propagates, as in the device entry
+    if (x > best || x != x) best = x;  // a NaN propagates, as in the device entry
   *V_out = best;
   return SFNL_OK;
 }

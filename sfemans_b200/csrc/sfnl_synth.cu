@@ -26,6 +26,9 @@ namespace {
 
 constexpr int kSynthThreads = 128;
 
+// The larger one, or a NaN that either is (fmax would drop it).
+__device__ __forceinline__ double max_nan(double a, double b) { return b > a || b != b ? b : a; }
+
 // MODE 0: grid values to out (N, nslot/2, np); 1: maximum of |v| into *vmax (atomic); 2: maximum of
 // |v| of each point to out[p].
 template <int MODE>
@@ -80,19 +83,19 @@ __global__ void __launch_bounds__(kSynthThreads) synth_kernel(const double *v, d
       if constexpr (MAXV) {
         const double a = sqrt(fp[0] * fp[0] + fp[1] * fp[1] + fp[2] * fp[2]);
         const double bm = sqrt(fm[0] * fm[0] + fm[1] * fm[1] + fm[2] * fm[2]);
-        vm = fmax(vm, a);
-        if (j > 0) vm = fmax(vm, bm);
+        vm = max_nan(vm, a);
+        if (j > 0) vm = max_nan(vm, bm);
       }
     }
     if constexpr (MODE == 2) {
-      for (int off = 16; off > 0; off >>= 1) vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, off));
+      for (int off = 16; off > 0; off >>= 1) vm = max_nan(vm, __shfl_xor_sync(0xffffffffu, vm, off));
       if (lane == 0) out[p] = vm;
       vm = 0.0;
     }
     __syncwarp();
   }
   if constexpr (MODE == 1) {
-    for (int off = 16; off > 0; off >>= 1) vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, off));
+    for (int off = 16; off > 0; off >>= 1) vm = max_nan(vm, __shfl_xor_sync(0xffffffffu, vm, off));
     if (lane == 0) atomicMax(vmax, (unsigned long long)__double_as_longlong(vm));
   }
 }
@@ -154,11 +157,11 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
           sp = fma(fp, fp, sp);
           sm = fma(fm, fm, sm);
         }
-        if constexpr (MODE != 0) pv = fmax(pv, fmax(sp, sm));  // the root of the maximum is the maximum of the roots
+        if constexpr (MODE != 0) pv = max_nan(pv, max_nan(sp, sm));  // the root of the maximum is the maximum of the roots
       }
-      if constexpr (MODE == 1) vm = fmax(vm, pv);
+      if constexpr (MODE == 1) vm = max_nan(vm, pv);
       if constexpr (MODE == 2) {
-        for (int off = 2; off > 0; off >>= 1) pv = fmax(pv, __shfl_xor_sync(0xffffffffu, pv, off));
+        for (int off = 2; off > 0; off >>= 1) pv = max_nan(pv, __shfl_xor_sync(0xffffffffu, pv, off));
         if (q == 0) atomicMax(pm + 8 * pt + gg, (unsigned long long)__double_as_longlong(sqrt(pv)));
       }
       }
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, d
     }
   }
   if constexpr (MODE == 1) {
-    for (int off = 16; off > 0; off >>= 1) vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, off));
+    for (int off = 16; off > 0; off >>= 1) vm = max_nan(vm, __shfl_xor_sync(0xffffffffu, vm, off));
     if (lane == 0) atomicMax(vmax, (unsigned long long)__double_as_longlong(sqrt(vm)));
   }
 }

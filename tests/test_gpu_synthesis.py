@@ -99,3 +99,18 @@ def test_synthesis_beyond_a_tile(nslot, m, N):
     got = host(sf.synthesis(dev(v), n_theta=N))
     assert R.rel_l2(got, want) <= 1e-12
     assert np.allclose(got, want, rtol=0, atol=1e-12 * np.abs(want).max() * np.sqrt(m))
+
+
+@pytest.mark.parametrize("nslot,m,npts", [(6, 5, 1), (6, 16, 61), (2, 33, 9), (4, 64, 300), (6, 700, 2)])
+def test_a_nan_propagates_to_the_maximum(nslot, m, npts):
+    # in one point of many, first, middle or last; device and host entries
+    import ctypes
+
+    pad = 3 * m // 2
+    for p in {0, npts // 2, npts - 1}:
+        v = R.synthetic_field(npts, nslot, m, 0.2, 3)
+        v[p, 0, 1] = np.nan
+        assert np.isnan(sf.max_vel(dev(v), pad))
+        out = ctypes.c_double()
+        assert sf.lib().sfnl_fft_max_vel_dcl(ctypes.c_void_p(v.ctypes.data), ctypes.byref(out), npts, nslot, m, 1, npts, pad) == 0
+        assert np.isnan(out.value)
