@@ -35,7 +35,9 @@
 // (12 -> 3, the JVP du x w + u x dw: two synthesis passes, one analysis).  The
 // transposed programs, the linearised MHD pair and the bundle away from m = 64
 // run as one launch of chain_kernel up to m = 64; small m takes one warp per tile
-// (solo_kernel) and m > 64 the residue grids (sfnl_res.cu).
+// (solo_kernel).  From m = 65 the products and the linearised programs take the
+// residue grids (sfnl_res.cu), but for captured calls to m = 107; the bundle and the
+// advection stay here to m = 107, the tensor to m = 86 (then sfnl_large.cu).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -392,7 +394,7 @@ __global__ void __launch_bounds__(fast_max_threads(NTC, CS),
     // A warp takes one k-step of a parity, 4 modes of the 8 points: its lanes fill whole A-fragment blocks (a warp on
     // 32 modes of one point stored to two banks, 8 lanes each), and the points, most of them of one element, read
     // the same nodal values.  Navier-Stokes caller, 101,150 Gauss points of P2 triangles: m = 32 0.311 -> 0.284 ms, m = 20
-    // 0.204 -> 0.185 ms (the third-fold kernels at m = 64 0.750 -> 0.701 ms); one more warp for the analysis' eight output
+    // 0.204 -> 0.185 ms (the third-fold kernels at m = 64, 60,000 points, 0.461 -> 0.419 ms); one more warp for the analysis' eight output
     // tiles changed nothing at m = 32 and cost a quarter at m = 20.
     const int m = a.m;
     for (int it = warp; it < KS[0] + KS[1]; it += NW) {

@@ -272,7 +272,7 @@ class LargeWorkspace {
   unsigned long long id_ = 0;
   bool capturing_ = false, got_ = false;
 };
-// Residue grids of 128 angles with one program kernel (sfnl_res.cu); cap: bytes of workspace.
+// Residue grids of 64 or 128 angles with one program kernel (sfnl_res.cu); cap: bytes of workspace.
 bool res_supported(int op, int m);
 int launch_res(const ProgArgs &a, size_t cap, cudaStream_t st);
 

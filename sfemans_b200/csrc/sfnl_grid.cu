@@ -10,8 +10,8 @@
 // for every N, odd or even, dealiasing or not: with a pad too short to
 // dealias it reproduces the reference's aliased result.
 //
-// Two kernels.  mirror_kernel takes every size whose tile fits in shared memory (m up to about 100 for six
-// fields): the mirror j -> N-j of the grid is folded out and the remaining contractions run on the FP64 tensor
+// Two kernels.  mirror_kernel takes every size whose tile fits in shared memory (with the reference's grid to m = 144
+// for the cross product, 200 for the dot product, 176 for v / s, 80 for the tensors): the mirror j -> N-j of the grid is folded out and the remaining contractions run on the FP64 tensor
 // cores, 8-point tiles staged with cp.async (sfnl_mirror.cuh).  grid_kernel (one warp per point, the coefficients
 // broadcast from shared memory, lanes owning angles and then modes) is the fallback beyond.  This form is the
 // parity anchor, and the only form of the programs that depend on the grid (the quotients and the tension

@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kLargeSynMaxWarps * 32, 1) large_syn_tf_kernel
 // Program and analysis with the third fold: chunks of two angle-tile pairs (t, t+1 and their mirrors); the
 // odd output groups contract all four tiles, the even ones P(t) +- P(mirror) over the first-half tiles
 // (signs PE0 +, PE2 -, QE0 -, QE2 +).  With up to two output tiles per warp (m <= 256 on the grid's residue
-// classes, m <= 192 without them) the kernel is held to 64 registers, two CTAs per SM: a spill of about
-// 136 bytes buys twice the resident warps, 4-11 % faster on a B200 from m = 128 to 256; with more tiles per
+// classes, m <= 192 without them) the kernel is held to 64 registers, two CTAs per SM: at most 64 bytes of
+// spills buy twice the resident warps, 4-11 % faster on a B200 from m = 128 to 256; with more tiles per
 // warp the accumulators spill too much and one CTA per SM was as fast or faster (m = 384, 512).
 template <int OP, int O0, int CPW>
 __global__ void __launch_bounds__(kLargeProdWarps * 32, CPW <= 2 ? 2 : 1) large_prod_tf_kernel(const LargeArgs a) {
@@ -675,7 +675,7 @@ int launch_large_syn(const LargeArgs &la, int nfields, bool tf, cudaStream_t st)
     return check_launch("large-m synthesis");
   };
   if (tf) {
-    // two point tiles per CTA: at 118 registers and 2 x 16-32 KB of staged rows, four CTAs share an SM; four
+    // two point tiles per CTA: at 122 registers and 2 x 16-32 KB of staged rows, four CTAs share an SM; four
     // tiles per CTA (each B fragment feeding four DMMAs) left three 4-warp CTAs per SM (168 registers) and
     // were 10-30 % slower (m = 128 to 512)
     if (2 * tile_bytes <= kLargeSynSmem) return go(large_syn_tf_kernel<2>, 2);
@@ -835,10 +835,9 @@ bool residues_fit(int m, int N, int R) {
 }
 
 // Residue classes of the two-kernel form for m modes on the N-angle grid; 0: the whole grid.  Six where
-// they fit, else three: on a B200, R = 6 against 3 took the cross product at m = 256 (350k points) from
-// 18.7 to 16.9 ms, at m = 384 (100k points) from 11.4 to 7.9 ms and at m = 512 (60k points) from 10.1 to
-// 6.8 ms, the 16-tangent MHD JVP at m = 256 (50k points) from 87.0 to 80.3 ms; residue grids of 64 angles
-// (R = 12 at m = 256) were slower than both.
+// they fit, else three: on a B200, R = 6 against 3 takes the bundle at m = 256 (100k points) from 15.5 to
+// 14.0 ms, at m = 384 (50k points) from 16.7 to 11.9 ms and at m = 512 (30k points) from 14.5 to 9.8 ms, the
+// tensor at m = 256 from 12.0 to 10.2 ms; twelve classes are slower than six (bundle at m = 256 20.5 ms).
 int large_residues(int m, int N) {
   if (const int R = g_test_residues.load()) return residues_fit(m, N, R) ? R : 0;
   if (m < 256 || m > 512) return 0;

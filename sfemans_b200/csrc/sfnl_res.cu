@@ -70,7 +70,8 @@ struct CoefArgs {
 // -Im Y_{M/2} in the sine row of mode 0).  Residues pair as d_{R-1-r} = -d_r: one twiddle serves two.
 // The block's twiddles (one k: 2 QM modes of R/2 residues) sit in shared memory and all loads are issued first; with
 // both left to the loop over the modes a pass reached 1 TB/s.  k runs fastest over the blocks, so that the 64-byte pieces
-// of a tile are written together (R = 6: 519 -> 338 us for 1.8 GB); the passes run at 5.4 to 6.1 TB/s.
+// of a tile are written together (six residues of 128 angles: 519 -> 338 us for 1.8 GB).  The passes run at 5.9 and 6.1
+// TB/s with six residues of 64 angles (m = 128), at 4.4 and 5.5 with twelve (m = 256).
 constexpr int res_qm(int R) { return (R + 2) / 3; }  // M q + k < m needs q < QM
 template <int M, int R>
 __device__ __forceinline__ void load_twiddles(double2 (&tw)[res_qm(R)][2][R / 2], const double *src, int m, int k) {
@@ -503,7 +504,10 @@ constexpr int kRes64Max = 12;
 
 // From m = 65, where the fused kernels run on run-time loops: cross product, 30,000 points, m = 65 0.433 -> 0.274 ms, m =
 // 100 0.769 -> 0.333; MHD VJP, 10,000 points, 4 cotangents, m = 65 1.91 -> 0.83 ms.  The cross product's JVP from m = 73:
-// its two-pass fused program is the faster one before (m = 72 0.370 against 0.393 ms, m = 80 0.573 against 0.395).
+// its two-pass fused program is the faster one before (m = 72 0.370 against 0.393 ms, m = 80 0.573 against 0.395).  Few
+// points do not move the line, although three or four launches with small grids replace one (1,000 points, m = 65: cross
+// product 18.7 against 18.7 us, dot product 16.6 against 17.4, MHD VJP 85.5 against 45.8; m = 85 cross product 22.8
+// against 18.7), but by 1 us of 14 for the scalar product to m = 80.
 bool res_supported(int op, int m) {
   if (m < (op == OP_CROSS_JVP ? 73 : 65) || m > 512) return false;
   return op == OP_CROSS || op == OP_DOT || op == OP_PROD || op == OP_SVECT || linear_op(op);

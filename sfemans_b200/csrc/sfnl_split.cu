@@ -38,11 +38,11 @@
 // two fields (a constant term table per program), evaluated by one thread per
 // (output, point, group of 2 or 4 angles).  The folded products, sliced, are the A operand
 // of the analysis, whose rows are (output, point) pairs; each 16-angle chunk is
-// analysed into a fresh accumulator and added in FP64 to the output, which the
-// same thread updates chunk after chunk (the lines stay in L2).
+// analysed into a fresh accumulator and added in FP64 to the sums of the chunks before
+// it, which the same thread keeps in registers (m <= 32) or in the output (L2).
 //
 // CTAs of 16 warps, persistent over tiles; four threads per row, one per class (slicing, output) or
-// quarter of a chunk (recombination).  Thread 0
+// quarter of a chunk (recombination).  One thread of the last warp
 // issues the MMAs; completion is signalled through an mbarrier whose waits
 // are bounded (a timeout sets a status word and abandons the tile instead of
 // spinning forever).

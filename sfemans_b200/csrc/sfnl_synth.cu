@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kSynthThreads) synth_kernel(const double *v, d
 // A CTA walks over its tiles; the coefficients of the next one are copied (second buffer) while the current one is
 // evaluated.  Measured on a B200 against one warp per point (synth_kernel): grid values of a 3-vector at 28,000
 // points and m = 64 0.48 -> 0.072 ms, the maximum at 56,000 points and m = 32 (with its copy to the host)
-// 0.411 -> 0.089 ms.
+// 0.411 -> 0.072 ms.
 template <int MODE, int NI, int PW>
 __global__ void __launch_bounds__(256, 2) mirror_synth_kernel(const double *v, double *out, unsigned long long *vmax,
                                                               int64_t np, int nslot, const MirrorGeo g,
