@@ -529,7 +529,10 @@ LargeWorkspace::LargeWorkspace(cudaStream_t st, int use) : st_(st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
   capturing_ = cap != cudaStreamCaptureStatusNone;
-  if (cudaStreamGetId(st, &id_) != cudaSuccess) cudaGetLastError();
+  if (cudaStreamGetId(st, &id_) != cudaSuccess) {
+    cudaGetLastError();
+    id_ = e_->stream;  // taken for the last call's
+  }
 }
 
 LargeWorkspace::~LargeWorkspace() {
