@@ -50,7 +50,9 @@
  * without it.  Beyond, shorter runs of points go through a smaller buffer, and a
  * capture needs a call of the same size on its stream before it.  The bundle and
  * the advection beyond m = 107 and the tensor beyond m = 86 have buffers of their
- * own, from 1 GiB up to a quarter of the free memory.
+ * own, from 1 GiB up to a quarter of the free memory.  A buffer that a graph was
+ * captured with stays until sfnl_finalize, also when a later call grows the
+ * stream's.
  */
 #ifndef SFEMANS_NL_H
 #define SFEMANS_NL_H

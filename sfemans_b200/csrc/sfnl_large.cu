@@ -502,7 +502,8 @@ struct LargeWorkspace::Entry {
   unsigned long long stream = 0;  // id of the last call's stream
   cudaEvent_t done = nullptr;     // cudaStreamPerThread: the last call's work
   bool used = false;              // done is recorded
-  std::vector<double *> retired;  // freed with the others
+  bool captured = false;          // a graph may hold the buffer
+  std::vector<double *> retired;  // buffers that may still be in use, freed with the others
 };
 
 namespace {
@@ -529,7 +530,7 @@ LargeWorkspace::LargeWorkspace(cudaStream_t st, int use) : st_(st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
   capturing_ = cap != cudaStreamCaptureStatusNone;
-  if (cudaStreamGetId(st, &id_) != cudaSuccess) {
+  if (!capturing_ && cudaStreamGetId(st, &id_) != cudaSuccess) {  // asking for it would end a capture
     cudaGetLastError();
     id_ = e_->stream;  // taken for the last call's
   }
@@ -578,14 +579,16 @@ int LargeWorkspace::get(size_t bytes, double **out) {
     if (capturing_)
       return set_error(SFNL_ERR_ALLOC, "the large-m workspace cannot be allocated while the stream is being captured");
     RelaxedCapture relaxed;
-    if (e.p) {
+    if (e.p && e.captured) {
+      e.retired.push_back(e.p);
+    } else if (e.p) {
       cudaStreamSynchronize(st_);  // the previous call on this stream may still read it
       if (e.used) cudaEventSynchronize(e.done);
       cudaFree(e.p);
     }
     e.p = nullptr;
     e.bytes = 0;
-    e.used = false;
+    e.used = e.captured = false;
     if (per_thread && !e.done && cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
       e.done = nullptr;
@@ -601,7 +604,10 @@ int LargeWorkspace::get(size_t bytes, double **out) {
     cudaGetLastError();
     return set_error(SFNL_ERR_CUDA, "cudaStreamWaitEvent for the large-m workspace failed");
   }
-  if (!capturing_) e.stream = id_;
+  if (capturing_)
+    e.captured = true;
+  else
+    e.stream = id_;
   got_ = true;
   *out = e.p;
   return SFNL_OK;
@@ -713,6 +719,7 @@ void large_release_workspaces() {
     if (e->p) cudaFree(e->p);  // waits for the work still reading it
     for (double *p : e->retired) cudaFree(p);
     e->retired.clear();
+    e->captured = false;
     if (e->done) cudaEventDestroy(e->done);
     e->p = nullptr;
     e->bytes = 0;

@@ -129,3 +129,40 @@ def test_captured_linearised_programs(m, kind, nbase, nin, nout, launches):
     g.replay()
     torch.cuda.synchronize()
     assert R.rel_l2(sf.to_host(out), sf.to_host(want)) <= TOL
+
+
+@pytest.mark.parametrize("kind", ["cross", "bundle"])
+def test_a_graph_keeps_its_buffer(kind):
+    # captured after a call of its size; a larger call on the same stream grows the stream's buffer before the replay
+    torch = pytest.importorskip("torch")
+    m, st = 128, torch.cuda.Stream()
+
+    def problem(npts):
+        f = [sf.to_device(_field(npts, 6, m, 31 + i)) for i in range(2 if kind == "cross" else 5)]
+        outs = [sf.fortran_empty(npts, s, m) for s in ((6,) if kind == "cross" else (6, 6, 6, 2))]
+        if kind == "cross":
+            return lambda: sf.product(sf.OP_CROSS, *f, out=outs[0], m_max_pad=_pad(m)), outs
+        return lambda: sf.bundle_mhd(*f, m_max_pad=_pad(m), outs=tuple(outs)), outs
+
+    (small, outs), (large, _) = problem(40), problem(5000)
+    torch.cuda.synchronize()
+    sf.lib().sfnl_finalize()
+    with torch.cuda.stream(st):
+        small()
+    torch.cuda.synchronize()
+    wants = [o.clone() for o in outs]
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        small()
+    with torch.cuda.stream(st):
+        large()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for o in outs:
+            o.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            g.replay()
+            large()
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, w) for o, w in zip(outs, wants))
