@@ -64,14 +64,15 @@ def test_two_threads(stream, first, second):
         assert all(torch.equal(out, want) for out in outs)
 
 
+@pytest.mark.parametrize("legacy", [False, True])
 @pytest.mark.parametrize("m", [72, 200])
-def test_a_capture_in_another_thread_goes_on(m):
+def test_a_capture_in_another_thread_goes_on(m, legacy):
     # a first and a growing call allocate their workspace while another thread captures a graph on its own stream
     torch = pytest.importorskip("torch")
     pad, sizes = (3 * m + 1) // 2, (150, 900)
     f = [[sf.to_device(R.synthetic_field(n, 6, m, 0.05, 7 + i)) for i in range(2)] for n in sizes]
     wants = [sf.product(sf.OP_CROSS, *ab, m_max_pad=pad, stream=0) for ab in f]
-    outs, side, errors = [torch.empty_like(w) for w in wants], torch.cuda.Stream(), []
+    outs, side, errors = [torch.empty_like(w) for w in wants], 0 if legacy else torch.cuda.Stream(), []
     x = torch.ones(64, device="cuda")
     torch.cuda.synchronize()
 
